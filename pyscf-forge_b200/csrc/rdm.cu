@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "profile.cuh"
+#include "rdm_fused.cuh"
 
 namespace csffci {
 
@@ -468,7 +469,7 @@ static int tslab_tile_launch(int norb, long long Nb, int nla, int nlb, const csf
   return check_launch("rdm T slab");
 }
 
-__global__ void k_rdm_assemble(int norb, const double* __restrict__ G, const double* __restrict__ d1,
+__global__ void k_rdm_assemble(int norb, const double* __restrict__ G, int ld, const double* __restrict__ d1,
                                double* dm2) {
   const int n = norb, n2 = n * n;
   long long tot = (long long)n2 * n2;
@@ -478,7 +479,7 @@ __global__ void k_rdm_assemble(int norb, const double* __restrict__ G, const dou
     int q = (int)((t / n2) % n);
     int r = (int)((t / n) % n);
     int s = (int)(t % n);
-    double v = G[(long long)(q * n + p) * n2 + r * n + s];
+    double v = G[(long long)(q * n + p) * ld + r * n + s];
     if (q == r) v -= d1[s * n + p];
     dm2[t] = v;
   }
@@ -486,7 +487,7 @@ __global__ void k_rdm_assemble(int norb, const double* __restrict__ G, const dou
 
 // spin-resolved assembly: dm2[p][q][r][s] = G[(qp)][(rs)] - d_qr d1[p][s]
 // (same-spin blocks) or G[(qp)][(rs)] (alpha-beta block, d1 == NULL)
-__global__ void k_rdm_assemble_s(int norb, const double* __restrict__ G, const double* __restrict__ d1,
+__global__ void k_rdm_assemble_s(int norb, const double* __restrict__ G, int ld, const double* __restrict__ d1,
                                  double* dm2) {
   const int n = norb, n2 = n * n;
   long long tot = (long long)n2 * n2;
@@ -496,7 +497,7 @@ __global__ void k_rdm_assemble_s(int norb, const double* __restrict__ G, const d
     int q = (int)((t / n2) % n);
     int r = (int)((t / n) % n);
     int s = (int)(t % n);
-    double v = G[(long long)(q * n + p) * n2 + r * n + s];
+    double v = G[(long long)(q * n + p) * ld + r * n + s];
     if (d1 && q == r) v -= d1[p * n + s];
     dm2[t] = v;
   }
@@ -505,11 +506,11 @@ __global__ void k_rdm_assemble_s(int norb, const double* __restrict__ G, const d
 // <E_xy> from the Gram of the 2-RDM: sum_r <E_xy E_rr> = <E_xy N> = N <E_xy>
 // (bra and ket both have N electrons of the spin the Gram is taken over),
 // so d1t[x][y] = (1/N) sum_r G[(y,x)][(r,r)] without another pass over T
-__global__ void k_d1_from_gram(int norb, const double* __restrict__ G, double inv_n, double* d1t) {
+__global__ void k_d1_from_gram(int norb, const double* __restrict__ G, int ld, double inv_n, double* d1t) {
   const int n = norb, n2 = n * n;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n2; t += gridDim.x * blockDim.x) {
     const int x = t / n, y = t - x * n;
-    const double* row = G + (long long)(y * n + x) * n2;
+    const double* row = G + (long long)(y * n + x) * ld;
     double acc = 0.0;
     for (int r = 0; r < n; ++r) acc += row[r * n + r];
     d1t[t] = acc * inv_n;
@@ -521,6 +522,28 @@ __global__ void k_transpose_small(int n, const double* in, double* out) {
     int i = t / n, j = t - i * n;
     out[j * n + i] = in[t];
   }
+}
+
+// the fused kernel's description of one Gram: S/A rows of one vector, or
+// the ordered rows of bra (its spin) against those of ket
+static RdmFusedJob fused_job(int norb, int neleca, int nelecb, const csffci_link_t* la, const csffci_link_t* lb,
+                             const double* bra, const double* ket, bool one, int spin_bra, int spin_ket) {
+  RdmFusedJob J;
+  J.norb = norb;
+  J.nla = neleca * (norb - neleca + 1);
+  J.nlb = nelecb * (norb - nelecb + 1);
+  J.nsrc = one ? 1 : 2;
+  J.sa = one ? 1 : 0;
+  J.la = la;
+  J.lb = lb;
+  J.src[0] = bra;
+  J.src[1] = ket;
+  J.spin[0] = spin_bra;
+  J.spin[1] = spin_ket;
+  J.Na = (long long)host_binom(norb, neleca);
+  J.Nb = (long long)host_binom(norb, nelecb);
+  J.sym = nullptr;
+  return J;
 }
 
 }  // namespace csffci
@@ -557,7 +580,9 @@ size_t csffci_rdm12_workspace(int norb, int neleca, int nelecb) {
   size_t partd = gram_dmma_workspace((int)n2, (int)n2, S);
   size_t part1 = gram_workspace(1, (int)n2, S);
   if (partd > part) part = partd;
-  return t + g + (part > part1 ? part : part1) + 1024;
+  const size_t slab = t + g + (part > part1 ? part : part1) + 1024;
+  const size_t fused = rdm_fused_workspace(norb, (long long)host_binom(norb, nelecb), nelecb * (norb - nelecb + 1));
+  return slab > fused ? slab : fused;
 }
 
 int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
@@ -573,14 +598,38 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
     set_error("rdm12: workspace of %zu bytes < %zu required", work_bytes, need);
     return CSFFCI_ERR_MEMORY;
   }
+  const bool same = (bra == ket);
+  int st;
+  RdmFusedJob J = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 3, 3);
+  if (dm2 && ndet > 0 && rdm_fused_fits(J)) {
+    double* M = rdm_fused_m(work);
+    const int ld = rdm_fused_ld(J);
+    const int ne = neleca + nelecb;
+    if (same) {
+      if (neleca == nelecb) {
+        int* bad = (int*)(M + (size_t)ld * ld);
+        if ((st = rdm_sym_check(ket, Na, bad, stream))) return st;
+        J.sym = bad;
+      }
+      if ((st = rdm_fused_run(J, work, stream))) return st;
+      return rdm_assemble_sa(J, M, ne, dm1, dm2, stream);
+    }
+    if ((st = rdm_fused_run(J, work, stream))) return st;
+    double* d1t = (double*)work;  // the partial sums are consumed
+    const double* G = M + ld / 2;
+    k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, G, ld, ne > 0 ? 1.0 / ne : 0.0, d1t);
+    if ((st = check_launch("rdm1 from the Gram"))) return st;
+    k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1t, dm1);
+    if ((st = check_launch("rdm1 transpose"))) return st;
+    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, ld, dm1, dm2);
+    return check_launch("rdm2 assemble");
+  }
   long long S = ndet < (1ll << 18) ? ndet : (1ll << 18);
   double* Tk = (double*)work;
   double* Tb = Tk + (size_t)S * n2;
   double* G = Tb + (size_t)S * n2;
   double* d1t = G + (size_t)n2 * n2;
   double* part = d1t + 2 * (size_t)n2;
-  const bool same = (bra == ket);
-  int st;
   for (long long J0 = 0; J0 < ndet; J0 += S) {
     long long s = (ndet - J0 < S) ? ndet - J0 : S;
     const int accumulate = J0 > 0;
@@ -599,13 +648,13 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   }
   if (dm2) {
     const int ne = neleca + nelecb;
-    k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, G, ne > 0 ? 1.0 / ne : 0.0, d1t);
+    k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, G, n2, ne > 0 ? 1.0 / ne : 0.0, d1t);
     if ((st = check_launch("rdm1 from the Gram"))) return st;
   }
   k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1t, dm1);
   if ((st = check_launch("rdm1 transpose"))) return st;
   if (dm2) {
-    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, dm1, dm2);
+    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, n2, dm1, dm2);
     return check_launch("rdm2 assemble");
   }
   return CSFFCI_OK;
@@ -626,7 +675,9 @@ size_t csffci_rdm12s_workspace(int norb, int neleca, int nelecb) {
   size_t partd = gram_dmma_workspace((int)n2, (int)n2, S);
   size_t part1 = gram_workspace(1, (int)n2, S);
   if (partd > part) part = partd;
-  return t + g + (part > part1 ? part : part1) + 1024;
+  const size_t slab = t + g + (part > part1 ? part : part1) + 1024;
+  const size_t fused = rdm_fused_workspace(norb, (long long)host_binom(norb, nelecb), nelecb * (norb - nelecb + 1));
+  return slab > fused ? slab : fused;
 }
 
 int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
@@ -646,6 +697,43 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
     set_error("rdm12s: workspace of %zu bytes < %zu required", work_bytes, need);
     return CSFFCI_ERR_MEMORY;
   }
+  const bool same = (bra == ket);
+  const bool two = dm2aa != nullptr;
+  int st;
+  if (two && ndet > 0) {
+    RdmFusedJob Jaa = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 1, 1);
+    RdmFusedJob Jbb = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 2, 2);
+    RdmFusedJob Jab = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, false, 1, 2);
+    Jab.sa = same ? 1 : 0;
+    if (rdm_fused_fits(Jaa) && rdm_fused_fits(Jbb) && rdm_fused_fits(Jab)) {
+      double* M = rdm_fused_m(work);
+      if (same) {
+        if ((st = rdm_fused_run(Jaa, work, stream))) return st;
+        if ((st = rdm_assemble_sa(Jaa, M, neleca, dm1a, dm2aa, stream))) return st;
+        if ((st = rdm_fused_run(Jbb, work, stream))) return st;
+        if ((st = rdm_assemble_sa(Jbb, M, nelecb, dm1b, dm2bb, stream))) return st;
+        if ((st = rdm_fused_run(Jab, work, stream))) return st;
+        return rdm_assemble_sa_ab(Jab, M, dm2ab, stream);
+      }
+      const int ld = rdm_fused_ld(Jab);
+      const double* G = M + ld / 2;
+      double* d1t = (double*)work;  // the partial sums are consumed
+      const int gs = grid_for((long long)n2 * n2, 256, 148 * 8);
+      for (int s = 0; s < 2; ++s) {
+        const int ne = s ? nelecb : neleca;
+        if ((st = rdm_fused_run(s ? Jbb : Jaa, work, stream))) return st;
+        k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, G, ld, ne > 0 ? 1.0 / ne : 0.0, d1t);
+        if ((st = check_launch("rdm1 from the Gram"))) return st;
+        k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1t, s ? dm1b : dm1a);
+        if ((st = check_launch("rdm1 transpose"))) return st;
+        k_rdm_assemble_s<<<gs, 256, 0, stream>>>(norb, G, ld, d1t, s ? dm2bb : dm2aa);
+        if ((st = check_launch("rdm2 assemble"))) return st;
+      }
+      if ((st = rdm_fused_run(Jab, work, stream))) return st;
+      k_rdm_assemble_s<<<gs, 256, 0, stream>>>(norb, G, ld, nullptr, dm2ab);
+      return check_launch("rdm2ab assemble");
+    }
+  }
   const long long S = rdm12s_slab(ndet);
   double* Tka = (double*)work;  // <J|E^alpha_pq|ket>
   double* Tkb = Tka + (size_t)S * n2;
@@ -657,9 +745,6 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   double* d1at = Gbb + (size_t)n2 * n2;
   double* d1bt = d1at + n2;
   double* part = d1bt + 2 * (size_t)n2;
-  const bool same = (bra == ket);
-  const bool two = dm2aa != nullptr;
-  int st;
   for (long long J0 = 0; J0 < ndet; J0 += S) {
     const long long s = (ndet - J0 < S) ? ndet - J0 : S;
     const int accumulate = J0 > 0;
@@ -683,9 +768,9 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   }
   if (two) {
     // same-spin Grams: sum_r <E^s_xy E^s_rr> = N_s <E^s_xy>
-    k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, Gaa, neleca > 0 ? 1.0 / neleca : 0.0, d1at);
+    k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, Gaa, n2, neleca > 0 ? 1.0 / neleca : 0.0, d1at);
     if ((st = check_launch("rdm1a from the Gram"))) return st;
-    k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, Gbb, nelecb > 0 ? 1.0 / nelecb : 0.0, d1bt);
+    k_d1_from_gram<<<grid_for(n2, 256), 256, 0, stream>>>(norb, Gbb, n2, nelecb > 0 ? 1.0 / nelecb : 0.0, d1bt);
     if ((st = check_launch("rdm1b from the Gram"))) return st;
   }
   k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1at, dm1a);
@@ -695,11 +780,11 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   if (two) {
     const int g = grid_for((long long)n2 * n2, 256, 148 * 8);
     // same-spin: <p+ r+ s q> = <E_pq E_rs> - d_qr <p+ s> = ... - d_qr dm1[s][p]
-    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gaa, d1at, dm2aa);
+    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gaa, n2, d1at, dm2aa);
     if ((st = check_launch("rdm2aa assemble"))) return st;
-    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gab, nullptr, dm2ab);
+    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gab, n2, nullptr, dm2ab);
     if ((st = check_launch("rdm2ab assemble"))) return st;
-    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gbb, d1bt, dm2bb);
+    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gbb, n2, d1bt, dm2bb);
     return check_launch("rdm2bb assemble");
   }
   return CSFFCI_OK;
