@@ -11,164 +11,57 @@
 #include "common.cuh"
 #include "profile.cuh"
 #include "batch_internal.cuh"
+#include "transform_tile.cuh"
 
 namespace csffci {
 
 // ---------------------------------------------------------------------------
 // transforms
 // ---------------------------------------------------------------------------
-constexpr int BT_M = 32, BT_N = 32, BT_K = 16;
-
-__device__ __forceinline__ int find_job(const int64_t* begin, int njobs, int64_t u, int hint) {
-  int j = hint;
-  while (j + 1 < njobs && begin[j + 1] <= u) ++j;
-  return j;
-}
-
-// Blocks with few CSFs (ncsf <= BR_MAX_NCSF) and few determinants per
-// configuration are most of the determinants below 13 orbitals (norb 12,
-// (6,6): 92 % of them in blocks of 6..70 determinants and 2..14 CSFs), and
-// a 32 x 32 output tile would leave most of its columns empty there.  Such
-// a job is cut into units of 256 (vector, configuration) rows instead, one
-// row per thread: the row's determinants are gathered through its mask
-// row and contracted with umat (read as warp-uniform loads: every thread
-// of a unit is in the same job) into NC register sums.  The sums run over
-// k in increasing order with fma, as the tile path's do, so both paths give
-// the same bits.
-constexpr int BR_ROWS = 256, BR_MAX_NCSF = 16, BR_MAX_NDET = 256;
-
-__host__ __device__ inline bool row_job(const csffci_transform_job_t& J) {
-  return J.ncsf <= BR_MAX_NCSF && J.ndet <= BR_MAX_NDET;
-}
-
-template <int NC>
-__device__ __forceinline__ void transform_row(const csffci_transform_job_t& J, int64_t vec, int64_t conf,
-                                              int reverse) {
-  const int nd = J.ndet, nc = J.ncsf;
-  const uint32_t* mk = J.mask + J.csd_offset + conf * nd;
-  if (!reverse) {
-    double acc[NC];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) acc[k] = 0.0;
-    const double* xv = J.x + vec * J.ldx;
-    for (int d = 0; d < nd; ++d) {
-      const double v = xv[mk[d]];
-      const double* u = J.umat + (int64_t)d * nc;
-#pragma unroll
-      for (int k = 0; k < NC; ++k)
-        if (k < nc) acc[k] = fma(v, u[k], acc[k]);
-    }
-    double* yo = J.y + vec * J.ldy + J.csf_offset + conf * nc;
-#pragma unroll
-    for (int k = 0; k < NC; ++k)
-      if (k < nc) yo[k] = J.sign * acc[k];
-  } else {
-    double cin[NC];
-    const double* xi = J.x + vec * J.ldx + J.csf_offset + conf * nc;
-#pragma unroll
-    for (int k = 0; k < NC; ++k) cin[k] = k < nc ? xi[k] : 0.0;
-    double* yv = J.y + vec * J.ldy;
-    for (int d = 0; d < nd; ++d) {
-      const double* u = J.umat + (int64_t)d * nc;
-      double acc = 0.0;
-#pragma unroll
-      for (int k = 0; k < NC; ++k)
-        if (k < nc) acc = fma(cin[k], u[k], acc);
-      yv[mk[d]] = J.sign * acc;
-    }
+// the last job whose tile_begin is at most u: 32 probes a round, so that a
+// table of hundreds of jobs costs two dependent loads (walking from the first
+// job took most of a launch over 120 jobs)
+__device__ __forceinline__ int find_job(const csffci_transform_job_t* jobs, int njobs, int64_t u, int lane) {
+  int lo = 0, hi = njobs;  // the answer is in [lo, hi)
+  while (hi - lo > 1) {
+    const int step = (hi - lo + 31) / 32;
+    const int at = lo + lane * step;
+    const bool le = at < hi && jobs[at].tile_begin <= u;
+    const int last = 31 - __clz((int)__ballot_sync(0xffffffffu, le));  // lane 0's job is always at or before u
+    lo += last * step;
+    hi = min(hi, lo + step);
   }
+  return lo;
 }
 
-// One tile = 32 (vec, conf) rows x 32 output columns of one job, or, for a
-// row job, 256 rows.
-__global__ void __launch_bounds__(256) k_transform_batch(const csffci_transform_job_t* jobs, int njobs,
-                                                         int64_t total_tiles, int reverse) {
-  __shared__ double As[BT_K][BT_M + 1];
-  __shared__ double Bs[BT_K][BT_N + 1];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  int j = 0;
+// One task = the CTA task of transform_tile.cuh of one job (one npair block of
+// one problem); pad holds the tile class and the column chunks.
+__global__ void __launch_bounds__(XF_W * 32, 2) k_transform_batch(const csffci_transform_job_t* jobs, int njobs,
+                                                                  int64_t total_tiles, int reverse) {
+  __shared__ double red[XF_RED];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int64_t tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    while (j + 1 < njobs && jobs[j + 1].tile_begin <= tile) ++j;
-    const csffci_transform_job_t& J = jobs[j];
-    const int nv = J.live ? min(J.nvec, *J.live) : J.nvec;
-    const int64_t M = (int64_t)nv * J.nconf;
-    const int64_t lt = tile - J.tile_begin;
-    if (row_job(J)) {
-      const int64_t m = lt * BR_ROWS + tid;
-      if (m < M) {
-        const csffci_transform_job_t Jr = J;  // in registers: the stores below cannot alias it
-        const int64_t vec = m / Jr.nconf, conf = m - vec * Jr.nconf;
-        if (Jr.ncsf <= 2) transform_row<2>(Jr, vec, conf, reverse);
-        else if (Jr.ncsf <= 4) transform_row<4>(Jr, vec, conf, reverse);
-        else if (Jr.ncsf <= 8) transform_row<8>(Jr, vec, conf, reverse);
-        else transform_row<BR_MAX_NCSF>(Jr, vec, conf, reverse);
-      }
-      continue;
-    }
-    const int N = reverse ? J.ndet : J.ncsf;
-    const int K = reverse ? J.ncsf : J.ndet;
-    const int ntn = (N + BT_N - 1) / BT_N;
-    const int64_t m0 = (lt / ntn) * BT_M;
-    const int n0 = (int)(lt % ntn) * BT_N;
-    if (m0 >= M) continue;  // rows of vectors that are not live (uniform per block)
-    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-    for (int k0 = 0; k0 < K; k0 += BT_K) {
-      for (int e = tid; e < BT_M * BT_K; e += 256) {
-        const int row = e / BT_K, kk = e - row * BT_K;
-        const int64_t m = m0 + row;
-        double v = 0.0;
-        if (m < M && k0 + kk < K) {
-          const int64_t vec = m / J.nconf, conf = m - vec * J.nconf;
-          if (!reverse) {
-            const uint32_t d = J.mask[J.csd_offset + conf * J.ndet + k0 + kk];
-            v = J.x[vec * J.ldx + d];
-          } else {
-            v = J.x[vec * J.ldx + J.csf_offset + conf * J.ncsf + k0 + kk];
-          }
-        }
-        As[kk][row] = v;
-      }
-      for (int e = tid; e < BT_N * BT_K; e += 256) {
-        double v = 0.0;
-        if (!reverse) {
-          const int kk = e / BT_N, col = e - kk * BT_N;
-          if (k0 + kk < K && n0 + col < N) v = J.umat[(int64_t)(k0 + kk) * J.ncsf + n0 + col];
-          Bs[kk][col] = v;
-        } else {
-          const int col = e / BT_K, kk = e - col * BT_K;
-          if (k0 + kk < K && n0 + col < N) v = J.umat[(int64_t)(n0 + col) * J.ncsf + k0 + kk];
-          Bs[kk][col] = v;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < BT_K; ++kk) {
-        const double a0 = As[kk][ty * 2], a1 = As[kk][ty * 2 + 1];
-        const double b0 = Bs[kk][tx * 2], b1 = Bs[kk][tx * 2 + 1];
-        acc[0][0] = fma(a0, b0, acc[0][0]);
-        acc[0][1] = fma(a0, b1, acc[0][1]);
-        acc[1][0] = fma(a1, b0, acc[1][0]);
-        acc[1][1] = fma(a1, b1, acc[1][1]);
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int a = 0; a < 2; ++a) {
-      const int64_t m = m0 + ty * 2 + a;
-      if (m >= M) continue;
-      const int64_t vec = m / J.nconf, conf = m - vec * J.nconf;
-#pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        const int n = n0 + tx * 2 + b;
-        if (n >= N) continue;
-        const double v = J.sign * acc[a][b];
-        if (!reverse) {
-          J.y[vec * J.ldy + J.csf_offset + conf * J.ncsf + n] = v;
-        } else {
-          J.y[vec * J.ldy + J.mask[J.csd_offset + conf * J.ndet + n]] = v;
-        }
-      }
-    }
+    const csffci_transform_job_t& J = jobs[find_job(jobs, njobs, tile, lane)];
+    XfTile B;
+    B.nvec = J.live ? min(J.nvec, *J.live) : J.nvec;
+    if (B.nvec <= 0) continue;  // uniform over the CTA
+    B.x = J.x;
+    B.y = J.y;
+    B.mask = J.mask + J.csd_offset;
+    B.u = J.umat;
+    B.z = nullptr;
+    B.sel = nullptr;
+    B.ldx = J.ldx;
+    B.ldy = J.ldy;
+    B.csf_off = J.csf_offset;
+    B.nconf = J.nconf;
+    B.ndet = J.ndet;
+    B.ncsf = J.ncsf;
+    B.sign = J.sign;
+    const int cls = J.pad & 7, nchunk = J.pad >> 3;
+    const int64_t t = tile - J.tile_begin;
+    if (reverse) xf_run<XF_CSF2DET>(B, nullptr, cls, t, nchunk, lane, warp, red);
+    else xf_run<XF_DET2CSF>(B, nullptr, cls, t, nchunk, lane, warp, red);
   }
 }
 
@@ -261,9 +154,9 @@ int transform_batch_prepare(int reverse, int njobs, csffci_transform_job_t* jobs
     csffci_transform_job_t& J = jobs[i];
     CSF_REQUIRE(J.x && J.y && J.mask && J.umat && J.ncsf > 0 && J.ndet > 0, "transform_batch: job %d incomplete", i);
     J.tile_begin = tiles;
-    const int64_t M = (int64_t)J.nvec * J.nconf;
-    const int N = reverse ? J.ndet : J.ncsf;
-    tiles += row_job(J) ? (M + BR_ROWS - 1) / BR_ROWS : ((M + BT_M - 1) / BT_M) * ((N + BT_N - 1) / BT_N);
+    const XfShape sh = xf_shape(J.nconf, J.nvec, reverse ? J.ndet : J.ncsf, reverse ? J.ncsf : J.ndet);
+    J.pad = sh.cls | sh.nchunk << 3;
+    tiles += sh.ntask;
   }
   *total_tiles = tiles;
   return CSFFCI_OK;
@@ -273,7 +166,7 @@ int transform_batch_launch(int reverse, const csffci_transform_job_t* jobs_dev, 
                            cudaStream_t stream) {
   if (tiles == 0 || njobs == 0) return CSFFCI_OK;
   ProfScope ps("k_transform_batch", stream);
-  k_transform_batch<<<grid_for(tiles, 1, 148 * 8), 256, 0, stream>>>(jobs_dev, njobs, tiles, reverse);
+  k_transform_batch<<<grid_for(tiles, 1, 148 * 2), XF_W * 32, 0, stream>>>(jobs_dev, njobs, tiles, reverse);
   return check_launch("transform_batch");
 }
 

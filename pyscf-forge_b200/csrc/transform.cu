@@ -1,291 +1,334 @@
-// det <-> CSF transforms and the CSF diagonal.
+// det <-> CSF transforms and the CSF diagonal of one space.
 //
-// Per npair block the reference gathers x[:, csd_mask block] into a
-// (nvec*nconf, ndet) matrix, multiplies it by +-umat and scatters into the CSF
-// vector (pyscf/csf_fci/csfstring.py:641-658).  Here each block is one tiled
-// FP64 GEMM whose A-operand loader performs the csd_mask gather (det->CSF)
-// and whose store performs the csd_mask scatter (CSF->det); csd_mask is a
-// permutation, so the scatter has no conflicts.  HBM-bound: every CI element
-// is read once and written once per call.
+// The reference works npair block by npair block: it gathers x[:, csd_mask
+// block] into a (nvec*nconf, ndet) matrix, multiplies it by +-umat and scatters
+// into the CSF vector (pyscf/csf_fci/csfstring.py:641-658).  Here one launch
+// takes every block (transform_tile.cuh): its CTAs walk over the tasks of all
+// blocks, those that share a tile (long K, few rows) first.
+//
+// What bounds it: the random 8-byte accesses through csd_mask (one 32-byte
+// sector each), then latency.  Measured, block by block launches of 64 x 64
+// GEMM tiles and a thread per configuration -> this:
+//   CAS(14,14) triplet, 2 vectors  CSF->det 0.91 -> 0.36 ms, det->CSF 1.01 -> 0.29 ms
+//   CAS(12,12) singlet, 3 vectors  CSF->det 0.38 -> 0.08 ms, det->CSF 0.42 -> 0.05 ms
+//   CAS(16,16) singlet, 1 vector   CSF->det 4.9 -> 3.2 ms, det->CSF 3.4 -> 2.3 ms
+//   CAS(14,14) triplet diagonal    2.75 -> 0.34 ms
+#include <string.h>
+
 #include "common.cuh"
 #include "profile.cuh"
+#include "transform_tile.cuh"
 
 namespace csffci {
 
-enum { MODE_DET2CSF = 0, MODE_CSF2DET = 1 };
+constexpr int XF_MAXB = 24;  // blocks of a launch (npair = 0..22 at norb 22)
 
-struct BlockGemmArgs {
-  const double* x;
-  double* y;
-  int64_t ldx, ldy;
+struct XfBlock {
   const uint32_t* mask;
-  const double* umat;
-  int64_t csd_off, csf_off, nconf;
-  const int32_t* conf_sel;  // selected configurations (point-group symmetry) or NULL
-  int ndet, ncsf;
-  int nvec;
+  const double* u;
+  const double* z;
+  const int32_t* sel;
+  int64_t csf_off, nconf, sconf, task0;
   double sign;
+  int ndet, ncsf, nspin, npair, cls, nchunk;
 };
 
-constexpr int TBM = 64, TBN = 64, TBK = 16;
+struct XfArgs {
+  const double* x;
+  double* y;
+  const double* eri;
+  int64_t ldx, ldy, ntask;
+  int nvec, nb, norb;
+  XfBlock b[XF_MAXB];
+};
 
 template <int MODE>
-__global__ void __launch_bounds__(256) k_block_gemm(BlockGemmArgs g) {
-  __shared__ double As[TBK][TBM + 1];
-  __shared__ double Bs[TBK][TBN + 1];
-  const int64_t M = (int64_t)g.nvec * g.nconf;
-  const int N = (MODE == MODE_DET2CSF) ? g.ncsf : g.ndet;
-  const int K = (MODE == MODE_DET2CSF) ? g.ndet : g.ncsf;
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int64_t ntile_m = (M + TBM - 1) / TBM;
-  const int ntile_n = (N + TBN - 1) / TBN;
-  for (int64_t tile = blockIdx.x; tile < ntile_m * ntile_n; tile += gridDim.x) {
-    const int64_t m0 = (tile / ntile_n) * TBM;
-    const int n0 = (int)(tile % ntile_n) * TBN;
-    double acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    for (int k0 = 0; k0 < K; k0 += TBK) {
-      // A tile: 64 rows x 16 k; thread loads (row = tid/16 + 16*r, k = tid%16)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        int row = ty + 16 * r;
-        int kk = tx;
-        int64_t m = m0 + row;
-        double v = 0.0;
-        if (m < M && k0 + kk < K) {
-          int64_t vec = m / g.nconf, conf = m - vec * g.nconf;
-          if (MODE == MODE_DET2CSF) {
-            const int64_t cf = g.conf_sel ? g.conf_sel[conf] : conf;
-            uint32_t d = g.mask[g.csd_off + cf * g.ndet + k0 + kk];
-            v = g.x[vec * g.ldx + d];
-          } else {
-            v = g.x[vec * g.ldx + g.csf_off + conf * g.ncsf + k0 + kk];
-          }
-        }
-        As[kk][row] = v;
-      }
-      // B tile: 16 k x 64 n
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        double v = 0.0;
-        if (MODE == MODE_DET2CSF) {
-          int kk = ty, col = tx + 16 * r;
-          if (k0 + kk < K && n0 + col < N) v = g.umat[(int64_t)(k0 + kk) * g.ncsf + n0 + col];
-          Bs[kk][col] = v;
-        } else {
-          int kk = tx, col = ty + 16 * r;
-          if (k0 + kk < K && n0 + col < N) v = g.umat[(int64_t)(n0 + col) * g.ncsf + k0 + kk];
-          Bs[kk][col] = v;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < TBK; ++kk) {
-        double a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-      }
-      __syncthreads();
+__global__ void __launch_bounds__(XF_W * 32, 2) k_transform(const __grid_constant__ XfArgs g) {
+  __shared__ double red[XF_RED];
+  __shared__ double kx[MODE == XF_HDIAG ? 256 : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (MODE == XF_HDIAG) {
+    const int np = g.norb * (g.norb + 1) / 2;
+    for (int i = threadIdx.x; i < 256; i += XF_W * 32) {
+      const int p = i >> 4, q = i & 15;
+      const int pq = pair_index(p, q);
+      kx[i] = p < g.norb && q < g.norb ? g.eri[(int64_t)pq * np + pq] : 0.0;
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int64_t m = m0 + ty * 4 + i;
-      if (m >= M) continue;
-      int64_t vec = m / g.nconf, conf = m - vec * g.nconf;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        int n = n0 + tx * 4 + j;
-        if (n >= N) continue;
-        double v = g.sign * acc[i][j];
-        if (MODE == MODE_DET2CSF) {
-          g.y[vec * g.ldy + g.csf_off + conf * g.ncsf + n] = v;
-        } else {
-          const int64_t cf = g.conf_sel ? g.conf_sel[conf] : conf;
-          uint32_t d = g.mask[g.csd_off + cf * g.ndet + n];
-          g.y[vec * g.ldy + d] = v;
-        }
-      }
-    }
-  }
-}
-
-// Blocks with few determinants and CSFs per configuration (at CAS(16,16)
-// the npair >= 3 blocks: at most 252 determinants and 42 CSFs, 98 % of the
-// configurations and 70 % of the determinants) make poor 64x64 GEMM tiles:
-// N = ncsf and K = ndet are far below the tile, so most of the tile's work
-// is padding.  Here one thread takes one (vector, configuration): the
-// block's umat sits in shared memory (every thread of a warp reads the same
-// element, a broadcast), and the configuration's gathered determinant
-// values (det->CSF) or its CSF coefficients (CSF->det) meet it in
-// registers.  The sums run over the determinants (det->CSF) or the CSFs
-// (CSF->det) in ascending order with the same fused multiply-adds as the
-// GEMM path, so both give the same bits.
-constexpr int SMALL_MAX_NCSF = 48;
-constexpr size_t SMALL_MAX_UMAT_BYTES = 96 * 1024;
-
-template <int MODE, int NC>
-__global__ void __launch_bounds__(256) k_block_small(BlockGemmArgs g) {
-  extern __shared__ double Us[];  // umat [ndet][ncsf]
-  const int nd = g.ndet, nc = g.ncsf;
-  for (int i = threadIdx.x; i < nd * nc; i += blockDim.x) Us[i] = g.umat[i];
-  __syncthreads();
-  const int64_t M = (int64_t)g.nvec * g.nconf;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M;
-       m += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t vec = m / g.nconf, conf = m - vec * g.nconf;
-    const int64_t cf = g.conf_sel ? g.conf_sel[conf] : conf;
-    const uint32_t* mk = g.mask + g.csd_off + cf * nd;
-    if (MODE == MODE_DET2CSF) {
-      double acc[NC];
-#pragma unroll
-      for (int k = 0; k < NC; ++k) acc[k] = 0.0;
-      const double* xv = g.x + vec * g.ldx;
-      for (int x = 0; x < nd; ++x) {
-        const double v = xv[mk[x]];
-        const double* u = Us + x * nc;
-#pragma unroll
-        for (int k = 0; k < NC; ++k)
-          if (k < nc) acc[k] = fma(v, u[k], acc[k]);
-      }
-      double* yo = g.y + vec * g.ldy + g.csf_off + conf * nc;
-#pragma unroll
-      for (int k = 0; k < NC; ++k)
-        if (k < nc) yo[k] = g.sign * acc[k];
-    } else {
-      double cin[NC];
-      const double* xi = g.x + vec * g.ldx + g.csf_off + conf * nc;
-#pragma unroll
-      for (int k = 0; k < NC; ++k) cin[k] = k < nc ? xi[k] : 0.0;
-      double* yv = g.y + vec * g.ldy;
-      for (int x = 0; x < nd; ++x) {
-        const double* u = Us + x * nc;
-        double sacc = 0.0;
-#pragma unroll
-        for (int k = 0; k < NC; ++k)
-          if (k < nc) sacc = fma(cin[k], u[k], sacc);
-        yv[mk[x]] = g.sign * sacc;
-      }
-    }
-  }
-}
-
-// profiler names per npair block (kernel timing by block)
-static const char* block_kernel_name(bool small, int npair) {
-  static const char* sm[9] = {"k_block_small_np0", "k_block_small_np1", "k_block_small_np2", "k_block_small_np3",
-                              "k_block_small_np4", "k_block_small_np5", "k_block_small_np6", "k_block_small_np7",
-                              "k_block_small_np8+"};
-  static const char* gm[9] = {"k_block_gemm_np0", "k_block_gemm_np1", "k_block_gemm_np2", "k_block_gemm_np3",
-                              "k_block_gemm_np4", "k_block_gemm_np5", "k_block_gemm_np6", "k_block_gemm_np7",
-                              "k_block_gemm_np8+"};
-  const int i = npair < 0 ? 0 : npair > 8 ? 8 : npair;
-  return small ? sm[i] : gm[i];
-}
-
-template <int MODE, int NC>
-static int launch_small(const BlockGemmArgs& g, cudaStream_t stream, int npair) {
-  const size_t smem = (size_t)g.ndet * g.ncsf * sizeof(double);
-  auto kern = k_block_small<MODE, NC>;
-  if (smem > 48 * 1024) CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t M = (int64_t)g.nvec * g.nconf;
-  {
-    ProfScope ps_(block_kernel_name(true, npair), stream);
-    kern<<<grid_for(M, 256, 148 * 8), 256, smem, stream>>>(g);
-  }
-  return check_launch("det/csf transform (small blocks)");
-}
-
-template <int MODE>
-static int run_small(const BlockGemmArgs& g, cudaStream_t stream, int npair) {
-  if (g.ncsf <= 2) return launch_small<MODE, 2>(g, stream, npair);
-  if (g.ncsf <= 8) return launch_small<MODE, 8>(g, stream, npair);
-  if (g.ncsf <= 16) return launch_small<MODE, 16>(g, stream, npair);
-  if (g.ncsf <= 32) return launch_small<MODE, 32>(g, stream, npair);
-  return launch_small<MODE, SMALL_MAX_NCSF>(g, stream, npair);
-}
-
-static bool small_block(const csffci_block_t& B) {
-  return B.ncsf <= SMALL_MAX_NCSF && (size_t)B.ndet * B.ncsf * sizeof(double) <= SMALL_MAX_UMAT_BYTES &&
-         B.ndet <= 256;
-}
-
-// det -> CSF blocks with few (vector, configuration) rows and a long K (at
-// CAS(16,16) npair 0: 1 configuration x 12870 determinants x 1430 CSFs, and
-// npair 1: 240 x 3432 x 429): the 64 x 64 GEMM tiles leave most SMs idle
-// and walk K alone.  Here a CTA takes 16 rows x 32 CSF columns and its 8
-// warps split K: the rows' gathered determinant values are staged in shared
-// memory a chunk of K at a time (coalesced mask reads, independent
-// gathers), each lane keeps the 16 sums of its column, and the 8 warp
-// partials are added in a fixed order at the end.
-constexpr int TK_M = 16, TK_N = 32, TK_KC = 512, TK_W = 8;
-
-constexpr size_t TK_SMEM = (size_t)TK_M * TK_KC * sizeof(double);  // 64 KB (dynamic)
-static_assert((size_t)TK_W * TK_M * (TK_N + 1) * sizeof(double) <= TK_SMEM, "the partials reuse the chunk buffer");
-
-__global__ void __launch_bounds__(TK_W * 32) k_block_tallk(BlockGemmArgs g) {
-  extern __shared__ double tk_smem[];
-  double (*Xs)[TK_KC] = reinterpret_cast<double (*)[TK_KC]>(tk_smem);              // gathered chunk
-  double (*Ps)[TK_M][TK_N + 1] = reinterpret_cast<double (*)[TK_M][TK_N + 1]>(tk_smem);  // warp partials
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t M = (int64_t)g.nvec * g.nconf;
-  const int N = g.ncsf, K = g.ndet;
-  const int ntn = (N + TK_N - 1) / TK_N;
-  const int64_t ntiles = ((M + TK_M - 1) / TK_M) * ntn;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t m0 = (tile / ntn) * TK_M;
-    const int n0 = (int)(tile % ntn) * TK_N;
-    const int n = n0 + lane;
-    double acc[TK_M];
-#pragma unroll
-    for (int i = 0; i < TK_M; ++i) acc[i] = 0.0;
-    for (int k0 = 0; k0 < K; k0 += TK_KC) {
-      const int kc = min(TK_KC, K - k0);
-      __syncthreads();  // the previous chunk is consumed
-      for (int e = tid; e < TK_M * TK_KC; e += TK_W * 32) {
-        const int r = e / TK_KC, kk = e - r * TK_KC;
-        const int64_t m = m0 + r;
-        double v = 0.0;
-        if (m < M && kk < kc) {
-          const int64_t vec = m / g.nconf, conf = m - vec * g.nconf;
-          const int64_t cf = g.conf_sel ? g.conf_sel[conf] : conf;
-          v = g.x[vec * g.ldx + g.mask[g.csd_off + cf * g.ndet + k0 + kk]];
-        }
-        Xs[r][kk] = v;
-      }
-      __syncthreads();
-      const int kw = (kc + TK_W - 1) / TK_W;  // k per warp in this chunk
-      const int kb = warp * kw, ke = min(kc, kb + kw);
-      if (n < N)
-        for (int kk = kb; kk < ke; ++kk) {
-          const double u = g.umat[(int64_t)(k0 + kk) * N + n];
-#pragma unroll
-          for (int i = 0; i < TK_M; ++i) acc[i] = fma(Xs[i][kk], u, acc[i]);
-        }
-    }
-    __syncthreads();  // every warp is done with the last chunk (Ps overlays Xs)
-#pragma unroll
-    for (int i = 0; i < TK_M; ++i) Ps[warp][i][lane] = acc[i];
     __syncthreads();
-    for (int e = tid; e < TK_M * TK_N; e += TK_W * 32) {
-      const int i = e / TK_N, j = e - i * TK_N;
-      const int64_t m = m0 + i;
-      if (m >= M || n0 + j >= N) continue;
-      double v = 0.0;
-#pragma unroll
-      for (int w = 0; w < TK_W; ++w) v += Ps[w][i][j];
-      const int64_t vec = m / g.nconf, conf = m - vec * g.nconf;
-      g.y[vec * g.ldy + g.csf_off + conf * N + n0 + j] = g.sign * v;
-    }
   }
+  int j = 0;
+  for (int64_t task = blockIdx.x; task < g.ntask; task += gridDim.x) {
+    while (j + 1 < g.nb && g.b[j + 1].task0 <= task) ++j;
+    const XfBlock& b = g.b[j];
+    XfTile B;
+    B.x = g.x;
+    B.y = g.y;
+    B.mask = b.mask;
+    B.u = b.u;
+    B.z = b.z;
+    B.sel = b.sel;
+    B.ldx = g.ldx;
+    B.ldy = g.ldy;
+    B.csf_off = b.csf_off;
+    B.nconf = b.nconf;
+    B.ndet = b.ndet;
+    B.ncsf = b.ncsf;
+    B.nvec = g.nvec;
+    B.sign = b.sign;
+    XfOrb o;
+    o.kx = kx;
+    o.norb = g.norb;
+    o.npair = b.npair;
+    o.nspin = b.nspin;
+    o.sconf = b.sconf;
+    xf_run<MODE>(B, &o, b.cls, task - b.task0, b.nchunk, lane, warp, red);
+  }
+}
+
+// Spaces whose vectors outgrow the L2: the same tiles in an order that keeps a
+// configuration's neighbours together.  All configurations with the same
+// occupation (empty, single, double) of the norb / 2 upper orbitals touch the
+// same small sub-matrices of the determinant vector: alpha and beta strings
+// are in ascending order, so a fixed upper part is a contiguous range of
+// each, tens of determinants long.  The configurations of such a group are,
+// in every npair block, a rectangle of (doubly occupied string, singly
+// occupied string) ranks, since both are ranked in ascending order too, and
+// its size depends on the numbers of doubly and singly occupied upper
+// orbitals alone; so a warp finds its group and tile from its number with a
+// table of those numbers (XfUp), group after group.  Sectors are then read
+// once, or completed, while they are in L2.  In block order every 8-byte
+// access beyond the L2 costs its own sector: a probe with a random
+// permutation gives 155 G stores/s and 210 G loads/s in 40 MB, 35 and 73 in
+// 188 MB, 29 and 63 in 640 MB.
+constexpr int XF_UP_MAX = 45;     // (doubly, singly) counts of up to 8 upper orbitals
+constexpr int XF_UP_BLOCKS = 12;  // npair blocks
+constexpr int64_t XF_UP_ELEMENTS = 8 << 20;  // 64 MiB: half of the L2
+constexpr int64_t XF_L2_BYTES = 126ll << 20;
+
+struct XfUp {
+  int n, low, nk;  // counts in the table; lower orbitals; blocks with shared tiles (first in XfArgs)
+  int64_t nkt;     // their tasks
+  int64_t start[XF_UP_MAX + 1];                  // first warp task
+  unsigned char d[XF_UP_MAX], s[XF_UP_MAX];      // doubly, singly occupied
+  uint32_t tile[XF_UP_MAX][XF_UP_BLOCKS + 1];    // first tile of each block within a group
+};
+
+__global__ void __launch_bounds__(XF_W * 32, 2) k_csf2det_up(const __grid_constant__ XfArgs g,
+                                                             const __grid_constant__ XfUp up) {
+  __shared__ double red[XF_RED];
+  __shared__ uint32_t bn[17][18];  // binomials (16 orbitals)
+  for (int i = threadIdx.x; i < 17 * 18; i += XF_W * 32) bn[i / 18][i % 18] = (uint32_t)binom(i / 18, i % 18);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto tile_of = [&](const XfBlock& b) {
+    XfTile B;
+    B.x = g.x;
+    B.y = g.y;
+    B.mask = b.mask;
+    B.u = b.u;
+    B.z = nullptr;
+    B.sel = nullptr;
+    B.ldx = g.ldx;
+    B.ldy = g.ldy;
+    B.csf_off = b.csf_off;
+    B.nconf = b.nconf;
+    B.ndet = b.ndet;
+    B.ncsf = b.ncsf;
+    B.nvec = g.nvec;
+    B.sign = b.sign;
+    return B;
+  };
+  int64_t t = blockIdx.x;
+  for (; t < up.nkt; t += gridDim.x) {
+    int j = 0;
+    while (j + 1 < up.nk && g.b[j + 1].task0 <= t) ++j;
+    const XfBlock& b = g.b[j];
+    const XfTile B = tile_of(b);
+    if (b.cls == 4) xf_shared<XF_CSF2DET, 1>(B, nullptr, t - b.task0, b.nchunk, lane, warp, red);
+    else if (b.cls == 5) xf_shared<XF_CSF2DET, 2>(B, nullptr, t - b.task0, b.nchunk, lane, warp, red);
+    else xf_shared<XF_CSF2DET, 4>(B, nullptr, t - b.task0, b.nchunk, lane, warp, red);
+  }
+  const int nh = g.norb - up.low;
+  int e = 0;
+  for (int64_t w = (t - up.nkt) * XF_W + warp; w < up.start[up.n]; w += (int64_t)gridDim.x * XF_W) {
+    while (up.start[e + 1] <= w) ++e;
+    // group number q among those with these counts: upper strings
+    const uint32_t per = up.tile[e][g.nb - up.nk];
+    const uint32_t rest = (uint32_t)(w - up.start[e]);
+    const uint32_t q = rest / per;
+    uint32_t tl = rest - q * per;
+    const int cd = up.d[e], cs = up.s[e];
+    int j = 0;
+    while (up.tile[e][j + 1] <= tl) ++j;
+    tl -= up.tile[e][j];
+    const XfBlock& b = g.b[up.nk + j];
+    const int pd = b.npair - cd, ps = b.nspin - cs;
+    // upper orbitals from the top: the strings of rank qd (doubly occupied)
+    // and qs (singly, among the others), and with them the colex ranks of the
+    // block's strings whose lower part is the first of its kind
+    const uint32_t nsing = bn[nh - cd][cs];
+    uint32_t qd = q / nsing, qs = q - qd * nsing, d0 = 0, s0 = 0;
+    int i = cd, k = cs, f = nh - cd;
+    for (int p = nh - 1; p >= 0; --p) {
+      const uint32_t c = bn[p][i];
+      if (i > 0 && c <= qd) {
+        qd -= c;
+        d0 += bn[up.low + p][pd + i--];
+      } else {
+        --f;
+        const uint32_t cq = bn[f][k];
+        if (k > 0 && cq <= qs) {
+          qs -= cq;
+          s0 += bn[up.low - pd + f][ps + k--];
+        }
+      }
+    }
+    const uint32_t ns = bn[up.low - pd][ps], rows = bn[up.low][pd] * ns;
+    // chunks of a row tile on neighbouring warps: walking over them in one warp
+    // left its sectors incomplete for longer (12.8 ms against 3.6 at CAS(16,16))
+    const uint32_t mt = tl / b.nchunk, chunk = tl - mt * b.nchunk;
+    uint32_t cf[1][2];
+    bool in[1][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t m = mt * 16 + 8 * h + (lane >> 2);
+      in[0][h] = m < rows;
+      m = min(m, rows - 1);
+      const uint32_t di = m / ns;
+      cf[0][h] = (d0 + di) * (uint32_t)b.sconf + s0 + (m - di * ns);
+    }
+    const XfTile B = tile_of(b);
+    if (b.cls == 0) xf_rows_tile<XF_CSF2DET, 1, 1>(B, nullptr, cf, cf, in, chunk * 8, lane);
+    else if (b.cls == 1) xf_rows_tile<XF_CSF2DET, 1, 2>(B, nullptr, cf, cf, in, chunk * 16, lane);
+    else xf_rows_tile<XF_CSF2DET, 1, 4>(B, nullptr, cf, cf, in, chunk * 32, lane);
+  }
+}
+
+// the orbital count behind the blocks' configuration counts (0: not to be had)
+static int xf_norb(const csffci_block_t* blocks, int nblock) {
+  for (int n = 1; n <= 22; ++n) {
+    bool ok = true, fixed = false;
+    for (int b = 0; b < nblock && ok; ++b) {
+      const csffci_block_t& S = blocks[b];
+      if (S.npair < 0 || S.nspin < 0 || S.npair + S.nspin > n || S.conf_sel != nullptr)
+        ok = false;
+      else
+        ok = (int64_t)(host_binom(n, S.npair) * host_binom(n - S.npair, S.nspin)) == S.nconf;
+      fixed = fixed || S.npair > 0 || S.nspin > 0;
+    }
+    if (ok && fixed) return n;
+  }
+  return 0;
+}
+
+// the table of a launch whose blocks nk.. are in the upper-orbital order
+static void xf_up(XfUp& up, const XfArgs& g) {
+  const int nh = g.norb / 2;
+  up.low = g.norb - nh;
+  up.nk = 0;
+  while (up.nk < g.nb && g.b[up.nk].cls >= 4) ++up.nk;
+  up.nkt = up.nk < g.nb ? g.b[up.nk].task0 : g.ntask;
+  up.n = 0;
+  up.start[0] = 0;
+  for (int cd = 0; cd <= nh; ++cd)
+    for (int cs = 0; cs + cd <= nh; ++cs) {
+      const int e = up.n;
+      uint32_t t = 0;
+      for (int j = up.nk; j < g.nb; ++j) {
+        const XfBlock& b = g.b[j];
+        const int pd = b.npair - cd, ps = b.nspin - cs;
+        up.tile[e][j - up.nk] = t;
+        if (pd >= 0 && ps >= 0 && pd + ps <= up.low)
+          t += (uint32_t)((host_binom(up.low, pd) * host_binom(up.low - pd, ps) + 15) / 16) * b.nchunk;
+      }
+      up.tile[e][g.nb - up.nk] = t;
+      if (t == 0) continue;
+      up.d[e] = (unsigned char)cd;
+      up.s[e] = (unsigned char)cs;
+      up.start[e + 1] = up.start[e] + (int64_t)(host_binom(nh, cd) * host_binom(nh - cd, cs)) * t;
+      up.n = e + 1;
+    }
+}
+
+template <int MODE>
+static int run_blocks(int nvec, const double* x, int64_t ldx, double* y, int64_t ldy, const uint32_t* mask,
+                      const csffci_block_t* blocks, int nblock, cudaStream_t stream, int norb = 0,
+                      const double* eri = nullptr) {
+  int bi = 0;
+  while (bi < nblock) {  // one launch unless a caller lists more than XF_MAXB blocks
+    XfArgs g;
+    memset(&g, 0, sizeof(g));
+    g.x = x;
+    g.y = y;
+    g.eri = eri;
+    g.ldx = ldx;
+    g.ldy = ldy;
+    g.nvec = nvec;
+    g.norb = norb;
+    const int b0 = bi;
+    bi = nblock - b0 < XF_MAXB ? nblock : b0 + XF_MAXB;
+    int64_t ndet = 0;
+    for (int b = b0; b < bi; ++b) ndet += blocks[b].nconf * blocks[b].ndet;
+    bool upper = false;
+    if (MODE == XF_CSF2DET && ndet * nvec >= XF_UP_ELEMENTS && bi - b0 <= XF_UP_BLOCKS) {
+      g.norb = xf_norb(blocks + b0, bi - b0);
+      upper = g.norb >= 8 && g.norb <= 16;
+    }
+    for (int pass = 0; pass < 2; ++pass)  // tiles shared by a CTA first
+      for (int b = b0; b < bi; ++b) {
+        const csffci_block_t& S = blocks[b];
+        if (S.nconf == 0 || S.ndet == 0) continue;
+        // CSF -> det writes the zeros of a block without CSFs as well, but
+        // where a selection is in force the caller has zeroed everything
+        if (S.ncsf == 0 && (MODE != XF_CSF2DET || S.conf_sel != nullptr)) continue;
+        CSF_REQUIRE(S.umat != nullptr || S.ncsf == 0, "transform: block %d has no umat", b);
+        CSF_REQUIRE(MODE != XF_HDIAG || S.nspin < 2 || S.zmat != nullptr, "hdiag_csf: block %d has no zmat", b);
+        XfShape sh = xf_shape(S.nconf, nvec, MODE == XF_CSF2DET ? S.ndet : S.ncsf,
+                                    MODE == XF_CSF2DET ? S.ncsf : S.ndet);
+        if ((sh.cls >= 4) != (pass == 0)) continue;
+        if (upper && sh.cls < 4) {  // one row tile x up to 32 columns
+          const int nt = ((MODE == XF_CSF2DET ? S.ndet : S.ncsf) + 7) / 8;
+          sh.cls = nt <= 1 ? 0 : nt <= 2 ? 1 : 2;
+          sh.nchunk = (nt + xf_cols(sh.cls) - 1) / xf_cols(sh.cls);
+          sh.ntask = 1;  // found through the table
+        }
+        XfBlock& d = g.b[g.nb++];
+        d.mask = mask + S.csd_offset;
+        d.u = S.umat;
+        d.z = S.zmat;
+        d.sel = S.conf_sel;
+        d.csf_off = S.csf_offset;
+        d.nconf = S.nconf;
+        d.sconf = g.norb > 0 ? (int64_t)host_binom(g.norb - S.npair, S.nspin) : 1;
+        d.sign = S.sign;
+        d.ndet = S.ndet;
+        d.ncsf = S.ncsf;
+        d.nspin = S.nspin;
+        d.npair = S.npair;
+        d.cls = sh.cls;
+        d.nchunk = sh.nchunk;
+        d.task0 = g.ntask;
+        g.ntask += sh.ntask;
+      }
+    if (g.ntask == 0) continue;
+    const char* name = MODE == XF_HDIAG ? "k_hdiag_csf" : MODE == XF_CSF2DET ? "k_csf2det" : "k_det2csf";
+    if (upper) {
+      XfUp up;
+      xf_up(up, g);
+      const int64_t tasks = up.nkt + (up.start[up.n] + XF_W - 1) / XF_W;
+      ProfScope ps_(name, stream);
+      // beyond the L2 one CTA per SM: fewer tiles in flight, fewer sectors left
+      // incomplete (CAS(16,16) 3.6 -> 3.2 ms; CAS(14,14) is faster with two)
+      const int ctas = ndet * (int64_t)sizeof(double) > XF_L2_BYTES ? 1 : 2;
+      k_csf2det_up<<<grid_for(tasks, 1, 148 * ctas), XF_W * 32, 0, stream>>>(g, up);
+    } else {
+      ProfScope ps_(name, stream);
+      k_transform<MODE><<<grid_for(g.ntask, 1, 148 * 2), XF_W * 32, 0, stream>>>(g);
+    }
+    const int st = check_launch("det/csf transform");
+    if (st) return st;
+  }
+  return CSFFCI_OK;
 }
 
 __global__ void k_zero_rows(double* y, int64_t ldy, int nvec, int64_t n) {
@@ -294,59 +337,6 @@ __global__ void k_zero_rows(double* y, int64_t ldy, int nvec, int64_t n) {
     int64_t v = i / n;
     y[v * ldy + (i - v * n)] = 0.0;
   }
-}
-
-template <int MODE>
-static int run_blocks(int nvec, const double* x, int64_t ldx, double* y, int64_t ldy,
-                      const uint32_t* mask, const csffci_block_t* blocks, int nblock,
-                      cudaStream_t stream) {
-  for (int b = 0; b < nblock; ++b) {
-    const csffci_block_t& B = blocks[b];
-    if (B.ncsf == 0 || B.nconf == 0) continue;
-    CSF_REQUIRE(B.umat != nullptr, "transform: block %d has no umat", b);
-    BlockGemmArgs g;
-    g.x = x;
-    g.y = y;
-    g.ldx = ldx;
-    g.ldy = ldy;
-    g.mask = mask;
-    g.umat = B.umat;
-    g.csd_off = B.csd_offset;
-    g.csf_off = B.csf_offset;
-    g.nconf = B.nconf;
-    g.conf_sel = B.conf_sel;
-    g.ndet = B.ndet;
-    g.ncsf = B.ncsf;
-    g.nvec = nvec;
-    g.sign = B.sign;
-    if (small_block(B)) {
-      const int st = run_small<MODE>(g, stream, B.npair);
-      if (st) return st;
-      continue;
-    }
-    int64_t M = (int64_t)nvec * B.nconf;
-    int N = (MODE == MODE_DET2CSF) ? B.ncsf : B.ndet;
-    int64_t tiles = ((M + TBM - 1) / TBM) * ((N + TBN - 1) / TBN);
-    if (MODE == MODE_DET2CSF && tiles < 2 * 148 && B.ndet >= 4 * TK_KC) {
-      // few GEMM tiles over a long K: the K-split kernel
-      const int64_t tk = ((M + TK_M - 1) / TK_M) * ((N + TK_N - 1) / TK_N);
-      CSF_CUDA(cudaFuncSetAttribute(k_block_tallk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TK_SMEM));
-      {
-        ProfScope ps_(block_kernel_name(false, B.npair), stream);
-        k_block_tallk<<<grid_for(tk, 1, 148 * 3), TK_W * 32, TK_SMEM, stream>>>(g);
-      }
-      const int st = check_launch("det->CSF transform (long K)");
-      if (st) return st;
-      continue;
-    }
-    {
-      ProfScope ps_(block_kernel_name(false, B.npair), stream);
-      k_block_gemm<MODE><<<grid_for(tiles, 1, 148 * 8), 256, 0, stream>>>(g);
-    }
-    int st = check_launch("det/csf transform");
-    if (st) return st;
-  }
-  return CSFFCI_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -416,7 +406,7 @@ int csffci_det2csf(int nvec, const double* x_det, int64_t ld_det, double* x_csf,
                    cudaStream_t stream) {
   CSF_REQUIRE(nvec >= 0 && blocks != nullptr && nblock >= 0, "det2csf: bad arguments");
   if (nvec == 0) return CSFFCI_OK;
-  return run_blocks<MODE_DET2CSF>(nvec, x_det, ld_det, x_csf, ld_csf, csd_mask, blocks, nblock,
+  return run_blocks<XF_DET2CSF>(nvec, x_det, ld_det, x_csf, ld_csf, csd_mask, blocks, nblock,
                                   stream);
 }
 
@@ -425,11 +415,12 @@ int csffci_csf2det(int nvec, const double* x_csf, int64_t ld_csf, double* x_det,
                    int nblock, cudaStream_t stream) {
   CSF_REQUIRE(nvec >= 0 && blocks != nullptr && nblock >= 0, "csf2det: bad arguments");
   if (nvec == 0) return CSFFCI_OK;
-  // determinants of blocks without CSFs (and every other one, for
-  // simplicity of the contract) start from zero
+  // determinants outside a selection start from zero; those of a block
+  // without CSFs are written as zeros by its own tasks
   bool full = true;
   for (int b = 0; b < nblock; ++b)
-    if ((blocks[b].ncsf == 0 && blocks[b].nconf > 0) || blocks[b].conf_sel != nullptr) full = false;
+    if (blocks[b].conf_sel != nullptr || (blocks[b].ncsf == 0 && blocks[b].nconf > 0 && blocks[b].ndet == 0))
+      full = false;
   if (!full) {
     {
       ProfScope ps_("k_zero_rows", stream);
@@ -439,14 +430,27 @@ int csffci_csf2det(int nvec, const double* x_csf, int64_t ld_csf, double* x_det,
     int st = check_launch("csf2det zero");
     if (st) return st;
   }
-  return run_blocks<MODE_CSF2DET>(nvec, x_csf, ld_csf, x_det, ld_det, csd_mask, blocks, nblock,
-                                  stream);
+  // a vector larger than the L2 at a time: with several, the sectors of one are
+  // evicted half written while the others' are (CAS(16,16), 4 vectors: 15.9 ms
+  // together, 13.5 ms one by one)
+  if (ndet * (int64_t)sizeof(double) > XF_L2_BYTES) {
+    for (int v = 0; v < nvec; ++v) {
+      const int st = run_blocks<XF_CSF2DET>(1, x_csf + v * ld_csf, ld_csf, x_det + v * ld_det, ld_det, csd_mask, blocks,
+                                            nblock, stream);
+      if (st) return st;
+    }
+    return CSFFCI_OK;
+  }
+  return run_blocks<XF_CSF2DET>(nvec, x_csf, ld_csf, x_det, ld_det, csd_mask, blocks, nblock, stream);
 }
 
 int csffci_hdiag_csf(int norb, int neleca, int nelecb, const double* hdiag_det, const double* eri,
                      const uint32_t* csd_mask, const csffci_block_t* blocks, int nblock,
                      double* hdiag_csf, cudaStream_t stream) {
   CSF_REQUIRE(norb >= 0 && norb <= 63 && blocks != nullptr, "hdiag_csf: bad arguments");
+  if (norb <= 16)
+    return run_blocks<XF_HDIAG>(1, hdiag_det, 0, hdiag_csf, 0, csd_mask, blocks, nblock, stream, norb, eri);
+  // more than 16 orbitals (4 bits no longer name one): a thread per CSF
   int npair_orb = norb * (norb + 1) / 2;
   for (int b = 0; b < nblock; ++b) {
     const csffci_block_t& B = blocks[b];
