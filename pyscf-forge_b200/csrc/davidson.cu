@@ -75,34 +75,43 @@ __global__ void k_precond_dots(int64_t n, const double* __restrict__ r, const do
   }
 }
 
-__global__ void k_precond_sum(const double* part, int npart, double* out2) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    for (int i = 0; i < npart; ++i) {
-      a += part[2 * i];
-      b += part[2 * i + 1];
+// the two sums over npart partials by one block of 256 threads (thread t adds
+// partials t, t + 256, ... in order, then a fixed tree); by one thread they
+// took 24 us
+__device__ __forceinline__ void precond_total(const double* part, int npart, double* s0, double* s1) {
+  double a = 0.0, b = 0.0;
+  for (int i = threadIdx.x; i < npart; i += 256) {
+    a += part[2 * i];
+    b += part[2 * i + 1];
+  }
+  s0[threadIdx.x] = a;
+  s1[threadIdx.x] = b;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) {
+      s0[threadIdx.x] += s0[threadIdx.x + w];
+      s1[threadIdx.x] += s1[threadIdx.x + w];
     }
-    out2[0] = a;
-    out2[1] = b;
+    __syncthreads();
   }
 }
 
-__global__ void k_precond_apply(int64_t n, const double* __restrict__ r, const double* __restrict__ x,
-                                const double* __restrict__ hd, double e, double shift, int mode,
-                                double e1_given, const double* part, int npart, double* t) {
-  __shared__ double e1s;
+__global__ void __launch_bounds__(256) k_precond_sum(const double* part, int npart, double* out2) {
+  __shared__ double s0[256], s1[256];
+  precond_total(part, npart, s0, s1);
   if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    if (mode == 1) {
-      for (int i = 0; i < npart; ++i) {
-        a += part[2 * i];
-        b += part[2 * i + 1];
-      }
-    }
-    e1s = mode == 2 ? e1_given : ((mode == 1 && b != 0.0) ? a / b : 0.0);
+    out2[0] = s0[0];
+    out2[1] = s1[0];
   }
-  __syncthreads();
-  const double e1 = e1s;
+}
+
+__global__ void __launch_bounds__(256) k_precond_apply(int64_t n, const double* __restrict__ r,
+                                                       const double* __restrict__ x, const double* __restrict__ hd,
+                                                       double e, double shift, int mode, double e1_given,
+                                                       const double* part, int npart, double* t) {
+  __shared__ double s0[256], s1[256];
+  if (mode == 1) precond_total(part, npart, s0, s1);
+  const double e1 = mode == 2 ? e1_given : (mode == 1 && s1[0] != 0.0) ? s0[0] / s1[0] : 0.0;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
        k += (int64_t)gridDim.x * blockDim.x)
     t[k] = (r[k] - e1 * x[k]) * precond_inv(hd[k], e, shift);
@@ -139,7 +148,7 @@ int csffci_precond_dots(int64_t n, const double* r, const double* x, const doubl
   }
   int st = check_launch("precond dots");
   if (st) return st;
-  k_precond_sum<<<1, 32, 0, stream>>>(work, nblk, out2);
+  k_precond_sum<<<1, 256, 0, stream>>>(work, nblk, out2);
   return check_launch("precond dots sum");
 }
 

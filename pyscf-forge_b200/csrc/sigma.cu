@@ -150,27 +150,59 @@ __global__ void k_sigma(SigmaArgs g) {
   }
 }
 
-// out[a][b] (+)= s[a][b] + eta * s[b][a]   (square n x n)
-__global__ void k_sym_add(const double* __restrict__ s, double* out, long long n, double eta,
-                          int accumulate) {
-  __shared__ double tile[32][33];
-  long long ntile = (n + 31) / 32;
-  for (long long t = blockIdx.x; t < ntile * ntile; t += gridDim.x) {
-    long long ti = t / ntile, tj = t - ti * ntile;
-    // load s[tj block rows][ti block cols] transposed
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-      long long row = tj * 32 + r, col = ti * 32 + threadIdx.x;
-      tile[r][threadIdx.x] = (row < n && col < n) ? s[row * n + col] : 0.0;
+// Tile pair t of an n x n matrix in 32 x 32 tiles: (ti, tj), ti <= tj, row by
+// row of the upper triangle.
+__device__ __forceinline__ void tile_pair(long long t, long long nt, long long* ti, long long* tj) {
+  // rows 0..i-1 hold i nt - i (i - 1) / 2 pairs
+  const double q = 2.0 * (double)nt + 1.0;
+  long long i = (long long)((q - sqrt(q * q - 8.0 * (double)t)) * 0.5);
+  if (i < 0) i = 0;
+  while (i > 0 && i * nt - i * (i - 1) / 2 > t) --i;
+  while ((i + 1) * nt - (i + 1) * i / 2 <= t) ++i;
+  *ti = i;
+  *tj = i + t - (i * nt - i * (i - 1) / 2);
+}
+
+// out[a][b] (+)= s[a][b] + eta * s[b][a]   (square n x n).  HBM-bound: a block
+// (32 x 8) takes a tile and its mirror together, so each element is read once
+// and written once (CAS(16,16), 2.65 GB: 0.84 -> 0.65 ms against reading both
+// tiles for each).
+__global__ void __launch_bounds__(256) k_sym_add(const double* __restrict__ s, double* out, long long n, double eta,
+                                                 int accumulate) {
+  __shared__ double ta[32][33], tb[32][33];
+  const long long nt = (n + 31) / 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  for (long long t = blockIdx.x; t < nt * (nt + 1) / 2; t += gridDim.x) {
+    long long ti, tj;
+    tile_pair(t, nt, &ti, &tj);
+    double a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long r = ti * 32 + ty + 8 * k, c = tj * 32 + tx;
+      a[k] = (r < n && c < n) ? s[r * n + c] : 0.0;
+      const long long r2 = tj * 32 + ty + 8 * k, c2 = ti * 32 + tx;
+      b[k] = (r2 < n && c2 < n) ? s[r2 * n + c2] : 0.0;
+    }
+    __syncthreads();  // the previous pair is consumed
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      ta[ty + 8 * k][tx] = a[k];
+      tb[ty + 8 * k][tx] = b[k];
     }
     __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-      long long row = ti * 32 + r, col = tj * 32 + threadIdx.x;
-      if (row < n && col < n) {
-        double v = s[row * n + col] + eta * tile[threadIdx.x][r];
-        out[row * n + col] = accumulate ? out[row * n + col] + v : v;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long r = ti * 32 + ty + 8 * k, c = tj * 32 + tx;
+      if (r < n && c < n) {
+        const double v = a[k] + eta * tb[tx][ty + 8 * k];
+        out[r * n + c] = accumulate ? out[r * n + c] + v : v;
+      }
+      const long long r2 = tj * 32 + ty + 8 * k, c2 = ti * 32 + tx;
+      if (ti != tj && r2 < n && c2 < n) {
+        const double v = b[k] + eta * ta[tx][ty + 8 * k];
+        out[r2 * n + c2] = accumulate ? out[r2 * n + c2] + v : v;
       }
     }
-    __syncthreads();
   }
 }
 
@@ -225,51 +257,72 @@ __global__ void k_det_finish_sym(const long long* __restrict__ w, double* out, l
   }
 }
 
-// per-block maxima of |c - c^T|, |c + c^T|, |c| over a square n x n matrix
-__global__ void k_parity_part(const double* __restrict__ c, long long n, double* part) {
-  __shared__ double s0[256], s1[256], s2[256];
-  double a = 0.0, b = 0.0, m = 0.0;
-  long long tot = n * n;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot;
-       i += (long long)gridDim.x * blockDim.x) {
-    long long r = i / n, q = i - r * n;
-    if (q > r) continue;
-    double x = c[i], y = c[q * n + r];
-    a = fmax(a, fabs(x - y));
-    b = fmax(b, fabs(x + y));
-    m = fmax(m, fmax(fabs(x), fabs(y)));
+// maxima of three values over the threads of a block (256), in s
+__device__ __forceinline__ void parity_max(double a, double b, double m, double (*s)[3], double* out) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
+    b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
   }
-  s0[threadIdx.x] = a;
-  s1[threadIdx.x] = b;
-  s2[threadIdx.x] = m;
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  if ((tid & 31) == 0) {
+    s[tid >> 5][0] = a;
+    s[tid >> 5][1] = b;
+    s[tid >> 5][2] = m;
+  }
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      s0[threadIdx.x] = fmax(s0[threadIdx.x], s0[threadIdx.x + w]);
-      s1[threadIdx.x] = fmax(s1[threadIdx.x], s1[threadIdx.x + w]);
-      s2[threadIdx.x] = fmax(s2[threadIdx.x], s2[threadIdx.x + w]);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    part[3 * blockIdx.x] = s0[0];
-    part[3 * blockIdx.x + 1] = s1[0];
-    part[3 * blockIdx.x + 2] = s2[0];
+  if (tid < 3) {
+    double v = 0.0;
+    for (int w = 0; w < 8; ++w) v = fmax(v, s[w][tid]);
+    out[tid] = v;
   }
 }
 
-__global__ void k_parity_final(const double* part, int np, double* out3) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double a = 0, b = 0, m = 0;
-    for (int i = 0; i < np; ++i) {
-      a = fmax(a, part[3 * i]);
-      b = fmax(b, part[3 * i + 1]);
-      m = fmax(m, part[3 * i + 2]);
+// per-block maxima of |c - c^T|, |c + c^T|, |c| over a square n x n matrix, a
+// tile with its mirror at a time (both read once, in rows).  A launch of one
+// block writes the result itself.
+__global__ void __launch_bounds__(256) k_parity_part(const double* __restrict__ c, long long n, double* part) {
+  __shared__ double tile[32][33];
+  __shared__ double red[8][3];
+  const long long nt = (n + 31) / 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  double a = 0.0, b = 0.0, m = 0.0;
+  for (long long t = blockIdx.x; t < nt * (nt + 1) / 2; t += gridDim.x) {
+    long long ti, tj;
+    tile_pair(t, nt, &ti, &tj);
+    double x[4], y[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long r = ti * 32 + ty + 8 * k, q = tj * 32 + tx;
+      x[k] = (r < n && q < n) ? c[r * n + q] : 0.0;
+      const long long r2 = tj * 32 + ty + 8 * k, q2 = ti * 32 + tx;
+      y[k] = (r2 < n && q2 < n) ? c[r2 * n + q2] : 0.0;
     }
-    out3[0] = a;
-    out3[1] = b;
-    out3[2] = m;
+    __syncthreads();  // the previous pair is consumed
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tile[ty + 8 * k][tx] = y[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const double z = tile[tx][ty + 8 * k];
+      a = fmax(a, fabs(x[k] - z));
+      b = fmax(b, fabs(x[k] + z));
+      m = fmax(m, fmax(fabs(x[k]), fabs(z)));
+    }
   }
+  parity_max(a, b, m, red, part + 3 * blockIdx.x);
+}
+
+__global__ void __launch_bounds__(256) k_parity_final(const double* part, int np, double* out3) {
+  __shared__ double red[8][3];
+  double a = 0.0, b = 0.0, m = 0.0;
+  for (int i = threadIdx.x; i < np; i += 256) {
+    a = fmax(a, part[3 * i]);
+    b = fmax(b, part[3 * i + 1]);
+    m = fmax(m, part[3 * i + 2]);
+  }
+  parity_max(a, b, m, red, out3);
 }
 
 struct SigmaConfig {
@@ -343,10 +396,14 @@ int csffci_spin_parity(int64_t n, const double* c, double* out3, void* work, siz
               (size_t)(3 * np) * sizeof(double));
     return CSFFCI_ERR_MEMORY;
   }
-  k_parity_part<<<np, 256, 0, stream>>>(c, n, (double*)work);
+  // the final pass by one thread took 63 us, more than the sigma of a small
+  // space; by a block of 256 it takes 3
+  const long long pairs = ((n + 31) / 32) * ((n + 31) / 32 + 1) / 2;
+  const int nb = pairs < np ? (int)(pairs > 0 ? pairs : 1) : np;
+  k_parity_part<<<nb, dim3(32, 8), 0, stream>>>(c, n, nb == 1 ? out3 : (double*)work);
   int st = check_launch("spin_parity");
-  if (st) return st;
-  k_parity_final<<<1, 32, 0, stream>>>((double*)work, np, out3);
+  if (st || nb == 1) return st;
+  k_parity_final<<<1, 256, 0, stream>>>((double*)work, nb, out3);
   return check_launch("spin_parity final");
 }
 
@@ -423,7 +480,7 @@ static int sigma_exec(int norb, int neleca, int nelecb, const double* h2e, const
     if (sym) {
       dim3 blk(32, 8);
       ProfScope ps("k_sym_add", stream);
-      long long tiles = ((Na + 31) / 32) * ((Na + 31) / 32);
+      const long long nt = (Na + 31) / 32, tiles = nt * (nt + 1) / 2;
       k_sym_add<<<grid_for(tiles, 1, 148 * 16), blk, 0, stream>>>(target, sigma, Na, (double)eta,
                                                                  accumulate ? 1 : 0);
       return check_launch("sigma symmetric add");
@@ -476,7 +533,7 @@ static int sigma_exec(int norb, int neleca, int nelecb, const double* h2e, const
   if (sym) {
     dim3 blk(32, 8);
     ProfScope ps("k_sym_add", stream);
-    long long tiles = ((Na + 31) / 32) * ((Na + 31) / 32);
+    const long long nt = (Na + 31) / 32, tiles = nt * (nt + 1) / 2;
     k_sym_add<<<grid_for(tiles, 1, 148 * 16), blk, 0, stream>>>(target, sigma, Na, (double)eta,
                                                                accumulate ? 1 : 0);
     return check_launch("sigma symmetric add");
