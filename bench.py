@@ -288,7 +288,7 @@ def run_ours(args, rank_env):
     ms = e0.elapsed_time(e1) / args.steps
     ms = max_over_ranks(ms, world)
     value = world * 1000.0 / ms
-    kname = next((k for k in ("k_sigma_wsr", "k_sigma_wsr_bulk", "k_sigma_ws", "k_sigma_rr", "k_sigma")
+    kname = next((k for k in ("k_sigma_wsr", "k_sigma_wsr_bulk", "k_sigma_ws", "k_sigma_mp", "k_sigma_rr", "k_sigma")
                   if k in prof), "k_sigma_rr")
     k_cnt, k_ms = prof.get(kname, (0, 0.0))
     traffic = TRAFFIC.get((args.workload, kname))

@@ -262,7 +262,8 @@ int csffci_sigma_plan_bind(csffci_sigma_plan_t* plan, void* work, size_t work_by
 int csffci_sigma_plan_execute(const csffci_sigma_plan_t* plan, const double* ci, double* sigma, int eta,
                               int flags, cudaStream_t stream);
 /* the kernel the plan runs: 0..3 register-resident tile variants, 4, 5
- * and 7 the warp-specialised kernels, -2 the shared-memory-h2e kernel */
+ * and 7 the warp-specialised kernels (4 up to 13 orbitals with FP64 adds: the
+ * one by pair rows), -2 the shared-memory-h2e kernel */
 int csffci_sigma_plan_variant(const csffci_sigma_plan_t* plan);
 void csffci_sigma_plan_destroy(csffci_sigma_plan_t* plan);
 

@@ -1,0 +1,622 @@
+// sigma for 4 to 13 orbitals: MMA warps in pairs of column tiles, mover warps
+// by pair rows (tile variant 4 of these sizes; one problem or a job table).
+//
+// As in k_sigma_ws, MMA warps hold h2e fragments in registers and mover warps
+// form D and scatter V.  What differs, and why:
+//
+//   - D and V are separate buffers (two stages each) and every hand-over is an
+//     mbarrier per stage, so no MMA warp waits for another one: in k_sigma_ws V
+//     overwrites D behind a barrier of all MMA warps, and the warps of a
+//     scheduler, which owns one FP64 tensor pipe, stop together.
+//   - A tile is 32 columns.  Warps 0.. take 16 pair rows x 16 columns (two of
+//     them share a row tile), four more the last 16 (or 8) rows x 8 columns
+//     each, so that every scheduler carries the same number of MMAs.
+//   - The movers work by pair rows, lanes over the 32 columns.  The beta links
+//     of a tile are turned into a table [pair row][column] -> (target, sign)
+//     in shared memory (a column has at most one link per pair row), so that a
+//     row of D = +-c[Ka][J] +- c[Ja][K] is made in registers and stored once:
+//     no zero rows, no read-modify-write, no order between alpha and beta, and
+//     every access of D, V and the table is a row.  k_sigma_ws went link by
+//     link: random rows, four shared accesses a link with bank conflicts.
+//   - The alpha values of the next tile are loaded into registers and its beta
+//     links copied to shared memory a tile ahead; row Ja of c and the alpha
+//     rows' addresses are double-buffered, so that the scatter of the last row
+//     runs behind the gather of the next.
+//   - The shares of the CTAs are tiles, not rows: the small spaces have fewer
+//     rows than the GPU has SMs.
+//
+// What bounds it: a mover's shared-memory accesses depend on one another and
+// take 200 to 400 cycles under the MMA warps' load, so there are 12 movers (4:
+// 478 us at 12 orbitals, 12: 300 us).  12 orbitals (6,6): 470 us, 280 us of it
+// FP64 MMAs at the 37.1 TFLOP/s peak (60%); without its MMAs or without its
+// adds the kernel would still take 90% of that.  Against the fastest kernel
+// before it: 8 orbitals (4,4) singlet 12.4 -> 5.2 us, 12 (6,6) 580 -> 470 us,
+// 13 (7,6) 2595 -> 2020 us.
+//
+// The CTAs (one per SM) take equal, contiguous shares of the tiles of all rows
+// of all live jobs, in rounds (see MPArgs::rounds).
+#include <math.h>
+#include <string.h>
+
+#include "sigma_ws.cuh"
+
+namespace csffci {
+
+constexpr int MP_NB = 32;    // columns of a tile
+constexpr int MP_DD = 36;    // row stride of D: = 4 (mod 16), conflict-free B fragments
+constexpr int MP_DV = 40;    // row stride of V: = 8 (mod 16), conflict-free 16-byte stores
+constexpr int MP_TS = 33;    // row stride of the link table
+constexpr int MP_POLLS = 1 << 22;
+constexpr long long MP_ROUND = 48ll << 20;  // bytes of c and sigma that a round goes through
+constexpr long long MP_MAX_TILES = 60000;  // tiles of a CTA: the table tag has 16 bits
+
+struct MPArgs {
+  const csffci_sigma_job_t* jobs;  // device table (BATCH) ...
+  csffci_sigma_job_t job0;         // ... or the one job
+  int njobs, npair;
+  // The list of tiles is cut into rounds and each round among the CTAs.  In
+  // one round a CTA would stay with its own problems, and all of a large
+  // table's vectors (20 problems of 12 orbitals: 270 MB) would be in use at
+  // once, their random adds past the L2 cache.
+  int rounds;
+  unsigned off_v, off_a, off_t, off_lk, off_crow, off_al, off_job, off_bar;
+  int crow_ld, lk_ld;  // elements between the two row and link buffers
+};
+
+// PT row tiles in pairs of column tiles, TAIL: 0 none, 1 a 16-row tile, 2 an
+// 8-row tile split over four warps; 12 movers
+template <int KS, int PT, int TAIL, bool BATCH>
+struct MPLayout {
+  static constexpr int NPAIRW = 2 * PT;
+  static constexpr int NMMA = NPAIRW + (TAIL ? 4 : 0);
+  static constexpr int NMOV = 12;
+  static constexpr int NTH = (NMMA + NMOV) * 32;
+  static constexpr int ROWS = 16 * PT + (TAIL == 1 ? 16 : TAIL == 2 ? 8 : 0);  // rows of V
+  static constexpr int RPM = (ROWS + NMOV - 1) / NMOV;                         // pair rows of a mover
+  // Registers.  With 12 MMA warps the launch has 80 a thread, split again by
+  // setmaxnreg; the k-steps from KR on are then read from shared memory.  The
+  // movers of a job table hold what for one problem is in constant memory or
+  // in uniform registers: 56 would spill (20 problems of 12 orbitals 8.28 ms),
+  // 72 do not (6.83 ms).  At 13 orbitals shared memory has no room for more.
+  static constexpr bool SPLIT = NMMA == 12;
+  static constexpr int KR = KS <= 14 ? KS : KS > 20 ? 17 : BATCH ? 12 : 17;
+  static constexpr int AT = (KS - KR) * (PT + (TAIL ? 1 : 0)) * 64;  // elements of that part of h2e
+  static constexpr int REG_LAUNCH = 65536 / NTH / 8 * 8;
+  static constexpr int REG_MMA = BATCH && KS <= 20 ? 88 : 104, REG_MOV = 160 - REG_MMA;
+  static_assert(NPAIRW % 4 == 0, "equal MMA shares on the four schedulers");
+  static_assert(!SPLIT || NMMA * 32 * REG_MMA + NMOV * 32 * REG_MOV <= NTH * REG_LAUNCH, "fits the launch's registers");
+};
+
+__device__ __forceinline__ void mp_arrive(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(ws_smem_addr(bar)) : "memory");
+}
+
+__device__ __forceinline__ bool mp_wait(unsigned long long* bar, unsigned parity) {
+  for (int i = 0; i < MP_POLLS; ++i)
+    if (ws_mbar_try_wait(bar, parity)) return true;
+  return false;
+}
+
+// tiles of a job: all columns, or those up to the diagonal (rows 32m..32m+31
+// have m + 1 tiles)
+__device__ __forceinline__ long long mp_tri(long long rows) {
+  const long long m = rows / MP_NB, r = rows - m * MP_NB;
+  return (MP_NB / 2) * m * (m + 1) + r * (m + 1);
+}
+__device__ __forceinline__ long long mp_job_tiles(const csffci_sigma_job_t& J) {
+  if (J.live != nullptr && J.live_index >= *J.live) return 0;
+  return J.sym ? mp_tri(J.Na) : J.Na * ((J.Nb + MP_NB - 1) / MP_NB);
+}
+
+// a tile of a job
+struct MPPos {
+  int ja;
+  int ct, nct;  // column tile, column tiles of the row
+};
+
+// what the movers read of a job of a table
+struct MPJob {
+  const double* ci;
+  double* out;
+  const csffci_link_t *link_a, *link_b;
+};
+
+struct MPShared {
+  double* D;
+  double* V;
+  double* A;  // k-steps from KR on: [step][row tile][row][4]
+  unsigned* T;
+  uint2* lk;  // raw links, two tiles
+  double* crow;
+  uint2* al;
+  MPJob* job;
+  unsigned long long* bar;  // D full, D empty, V full, V empty, two each
+};
+
+// the job of tile *t of the list, by a warp (32 jobs at a time); *t becomes its
+// number in the job
+template <bool BATCH>
+__device__ __forceinline__ int mp_find(const MPArgs& g, int lane, long long* t) {
+  if constexpr (BATCH) {
+    for (int j0 = 0; j0 < g.njobs; j0 += 32) {
+      const long long own = j0 + lane < g.njobs ? mp_job_tiles(g.jobs[j0 + lane]) : 0;
+      long long upto = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
+      }
+      const unsigned past = __ballot_sync(0xffffffffu, *t < upto);
+      if (past) {
+        const int l = __ffs(past) - 1;
+        *t -= __shfl_sync(0xffffffffu, upto - own, l);
+        return j0 + l;
+      }
+      *t -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return g.njobs - 1;
+  }
+  return 0;
+}
+
+__device__ __forceinline__ int mp_nct(int ja, int Nb, int sym) { return ((sym ? ja + 1 : Nb) + MP_NB - 1) / MP_NB; }
+
+__device__ __forceinline__ MPPos mp_pos(long long t, int Nb, int sym) {
+  MPPos p;
+  if (sym) {
+    long long m = (long long)((sqrt(1.0 + 0.25 * (double)t) - 1.0) * 0.5);
+    while ((MP_NB / 2) * m * (m + 1) > t) --m;
+    while ((MP_NB / 2) * (m + 1) * (m + 2) <= t) ++m;
+    const long long rem = t - (MP_NB / 2) * m * (m + 1);
+    p.ja = (int)(MP_NB * m + rem / (m + 1));
+    p.ct = (int)(rem % (m + 1));
+  } else {
+    const int nct = (Nb + MP_NB - 1) / MP_NB;
+    p.ja = (int)(t / nct);
+    p.ct = (int)(t - (long long)p.ja * nct);
+  }
+  p.nct = mp_nct(p.ja, Nb, sym);
+  return p;
+}
+
+// the next tile of the job; 1 on a new row
+__device__ __forceinline__ int mp_next(MPPos* p, int Nb, int sym) {
+  if (++p->ct < p->nct) return 0;
+  p->ct = 0;
+  ++p->ja;
+  p->nct = mp_nct(p->ja, Nb, sym);
+  return 1;
+}
+
+// Tiles it0 .. it0 + n - 1 of the CTA: those from tile t0 on of job Q.
+template <int KS, int PT, int TAIL, bool BATCH>
+__device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, const csffci_sigma_job_t& Q, long long t0,
+                                          int it0, int n, int mtid, int lane, int mw) {
+  using L = MPLayout<KS, PT, TAIL, BATCH>;
+  constexpr int NMOV = L::NMOV, MTH = NMOV * 32, RPM = L::RPM;
+  constexpr int RB = 4, RS = BATCH ? 2 : 4;  // pair rows gathered and scattered together
+  const int npair = g.npair;
+  const int dsz = L::ROWS > 4 * KS ? L::ROWS * MP_DD : 4 * KS * MP_DD, vsz = L::ROWS * MP_DV, tsz = npair * MP_TS;
+  bool ok = true;
+  const int Nb = (int)Q.Nb, sym = Q.sym, nlb = Q.nlb, end = it0 + n;
+  // what one problem has in constant memory is for a job table kept in shared
+  // memory: held in registers it would make the movers spill
+  if (BATCH) {
+    if (mtid == 0) *S.job = MPJob{Q.ci, sym ? Q.scratch : Q.sigma, Q.link_a, Q.link_b};
+    ws_bar_sync(5, MTH);
+  }
+  auto ci = [&]() { return BATCH ? S.job->ci : Q.ci; };
+  auto out = [&]() { return BATCH ? S.job->out : sym ? Q.scratch : Q.sigma; };
+  auto link_a = [&]() { return BATCH ? S.job->link_a : Q.link_a; };
+  auto link_b = [&]() { return BATCH ? S.job->link_b : Q.link_b; };
+  MPPos cur = mp_pos(t0, Nb, sym);
+  // the raw links of the next tile, copied asynchronously: entry e of its
+  // contiguous columns is link e % nlb of column e / nlb
+  MPPos ahead = cur;
+  auto load_links = [&](int it) {
+    const int ne = min(MP_NB, Nb - ahead.ct * MP_NB) * nlb;
+    const csffci_link_t* src = link_b() + ahead.ct * MP_NB * nlb;
+    uint2* const dst = S.lk + (it & 1) * g.lk_ld;
+#pragma unroll 1
+    for (int e = mtid; e < ne; e += MTH) cp_async8(&dst[e], &src[e]);
+    cp_async_commit();
+  };
+  // the table of tile it (each thread takes the entries that it copied)
+  auto build = [&](int it) {
+    const int ne = min(MP_NB, Nb - ahead.ct * MP_NB) * nlb;
+    const unsigned inv = (1u << 20) / (unsigned)max(nlb, 1) + 1u, tag = (unsigned)(it + 1) << 14;
+    unsigned* const T = S.T + it % 3 * tsz;
+    const uint2* const src = S.lk + (it & 1) * g.lk_ld;
+    cp_async_wait_all();
+#pragma unroll 4
+    for (int e = mtid; e < ne; e += MTH) {
+      const uint2 l = src[e];
+      T[rr_lpair(l) * MP_TS + (int)(((unsigned)e * inv) >> 20)] = l.x | tag | rr_lneg(l);
+    }
+  };
+  double va[RPM];      // alpha values of the next tile
+  unsigned sa = 0u;    // their signs
+  int par = 1;
+  int pja = 0, pct = 0, ppar = 0;  // the previous tile, whose V is scattered
+  load_links(it0);
+  build(it0);
+  if (it0 + 1 < end) {
+    mp_next(&ahead, Nb, sym);
+    load_links(it0 + 1);
+  }
+  int fresh = 1;  // a new row starts at the next tile
+  for (int it = it0; it <= end; ++it) {
+    if (it < end) {
+      const int s = it & 1;
+      if (fresh) {
+        par ^= 1;
+        uint2* const al = S.al + par * npair;
+        double* const cr = S.crow + par * g.crow_ld;
+#pragma unroll 1
+        for (int r = mtid; r < npair; r += MTH) al[r] = make_uint2(0u, 0u);
+        const double* const row = ci() + cur.ja * Nb;
+#pragma unroll 1
+        for (int i = mtid; i < Nb; i += MTH) cp_async8(&cr[i], &row[i]);
+        cp_async_commit();
+        ws_bar_sync(5, MTH);
+#pragma unroll 1
+        for (int l = mtid; l < Q.nla; l += MTH) {
+          const uint2 e = rr_link(&link_a()[cur.ja * Q.nla + l]);
+          al[rr_lpair(e)] = make_uint2(e.x * (unsigned)Nb, 1u | rr_lneg(e));
+        }
+        cp_async_wait_all();
+        ws_bar_sync(5, MTH);  // also: the table of this tile is complete
+      }
+      const uint2* const al = S.al + par * npair;
+      const int jend = sym ? cur.ja + 1 : Nb;
+      auto load_alpha = [&](int ct) {
+        const int j = ct * MP_NB + lane;
+        const double* const src = ci() + j;
+        sa = 0u;
+#pragma unroll
+        for (int i = 0; i < RPM; ++i) {
+          const int r = mw + i * NMOV;
+          const uint2 a = r < npair ? al[r] : make_uint2(0u, 0u);
+          va[i] = (a.y && j < jend) ? __ldg(&src[a.x]) : 0.0;
+          sa |= (a.y >> 31) << i;
+        }
+      };
+      if (fresh) load_alpha(cur.ct);
+      if (it >= 2 && ok) ok = mp_wait(&S.bar[2 + s], ((it >> 1) & 1) ^ 1);  // D of tile it-2 is consumed
+      const unsigned* const T = S.T + it % 3 * tsz + lane;
+      const unsigned tag = (unsigned)(it + 1) & 0xffffu;
+      const double* const cr = S.crow + par * g.crow_ld;
+      double* const D = S.D + s * dsz + lane;
+#pragma unroll
+      for (int i0 = 0; i0 < RPM; i0 += RB) {
+        unsigned t[RB];
+        double vb[RB];
+#pragma unroll
+        for (int k = 0; k < RB; ++k) {
+          const int r = mw + (i0 + k) * NMOV;
+          const bool in = i0 + k < RPM && r < npair;
+          t[k] = in ? T[r * MP_TS] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < RB; ++k) vb[k] = ((t[k] >> 14) & 0xffffu) == tag ? cr[t[k] & 0x3fffu] : 0.0;
+#pragma unroll
+        for (int k = 0; k < RB; ++k) {
+          const int r = mw + (i0 + k) * NMOV;
+          if (i0 + k < RPM && r < npair)
+            D[r * MP_DD] = rr_flip(va[i0 + k < RPM ? i0 + k : 0], (sa << (31 - i0 - k)) & 0x80000000u) +
+                           rr_flip(vb[k], t[k] & 0x80000000u);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mp_arrive(&S.bar[s]);  // this warp's rows of D are there
+      // the next tile's alpha values (same row), table and links
+      if (it + 1 < end) {
+        if (cur.ct + 1 < cur.nct) load_alpha(cur.ct + 1);
+        build(it + 1);
+        if (it + 2 < end) {
+          mp_next(&ahead, Nb, sym);
+          load_links(it + 2);
+        }
+      }
+    }
+    if (it > it0) {
+      // scatter V of the previous tile
+      const int s = (it - 1) & 1;
+      if (ok) ok = mp_wait(&S.bar[4 + s], ((it - 1) >> 1) & 1);
+      const uint2* const al = S.al + ppar * npair;
+      const unsigned* const T = S.T + (it - 1) % 3 * tsz + lane;
+      const unsigned tag = (unsigned)it & 0xffffu;
+      const double* const V = S.V + s * vsz + lane;
+      double* const orow = out() + pja * Nb;
+      const int j = pct * MP_NB + lane;
+      const bool inb = j < (sym ? pja + 1 : Nb), ina = sym ? j < pja : inb;
+      double* const ocol = out() + j;
+#pragma unroll
+      for (int i0 = 0; i0 < RPM; i0 += RS) {
+        unsigned t[RS];
+        uint2 a[RS];
+        double v[RS];
+#pragma unroll
+        for (int k = 0; k < RS; ++k) {
+          const int r = mw + (i0 + k) * NMOV;
+          const bool in = i0 + k < RPM && r < npair;
+          t[k] = in ? T[r * MP_TS] : 0u;
+          a[k] = in ? al[r] : make_uint2(0u, 0u);
+          v[k] = in ? V[r * MP_DV] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < RS; ++k) {
+          if (inb && ((t[k] >> 14) & 0xffffu) == tag) rr_red(&orow[t[k] & 0x3fffu], rr_flip(v[k], t[k] & 0x80000000u));
+          if (ina && a[k].y) rr_red(&ocol[a[k].x], rr_flip(v[k], a[k].y & 0x80000000u));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mp_arrive(&S.bar[6 + s]);  // V of the previous tile is consumed
+    }
+    if (it < end) {
+      pja = cur.ja;
+      pct = cur.ct;
+      ppar = par;
+      fresh = mp_next(&cur, Nb, sym);
+    }
+    ws_bar_sync(5, MTH);  // the table of tile it+1 is complete, that of it-1 is free
+  }
+  return ok;
+}
+
+template <int KS, int PT, int TAIL, bool BATCH>
+__global__ void __launch_bounds__(MPLayout<KS, PT, TAIL, BATCH>::NTH, 1) k_sigma_mp(const __grid_constant__ MPArgs g) {
+  using L = MPLayout<KS, PT, TAIL, BATCH>;
+  constexpr int NTH = L::NTH;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int npair = g.npair;
+  MPShared S;
+  S.D = (double*)smraw;
+  S.V = (double*)(smraw + g.off_v);
+  S.A = (double*)(smraw + g.off_a);
+  S.T = (unsigned*)(smraw + g.off_t);
+  S.lk = (uint2*)(smraw + g.off_lk);
+  S.crow = (double*)(smraw + g.off_crow);
+  S.al = (uint2*)(smraw + g.off_al);
+  S.job = (MPJob*)(smraw + g.off_job);
+  S.bar = (unsigned long long*)(smraw + g.off_bar);
+  constexpr int DR = L::ROWS > 4 * KS ? L::ROWS : 4 * KS;
+  constexpr int dsz = DR * MP_DD, vsz = L::ROWS * MP_DV;
+  __shared__ long long total_s;
+  __shared__ int bad_s;
+  for (int i = tid; i < 2 * dsz; i += NTH) S.D[i] = 0.0;  // rows past npair stay zero
+  for (int i = tid; i < 3 * npair * MP_TS; i += NTH) S.T[i] = 0u;
+  if (tid == 0) {
+    total_s = 0;
+    bad_s = 0;
+    for (int i = 0; i < 2; ++i) {
+      ws_mbar_init(&S.bar[i], L::NMOV);
+      ws_mbar_init(&S.bar[2 + i], L::NMMA);
+      ws_mbar_init(&S.bar[4 + i], L::NMMA);
+      ws_mbar_init(&S.bar[6 + i], L::NMOV);
+    }
+    ws_mbar_init_fence();
+  }
+  __syncthreads();
+  if (BATCH) {
+    long long t = 0;
+    for (int i = tid; i < g.njobs; i += NTH) t += mp_job_tiles(g.jobs[i]);
+    if (t) atomicAdd((unsigned long long*)&total_s, (unsigned long long)t);
+    __syncthreads();
+  }
+  const long long total = BATCH ? total_s : mp_job_tiles(g.job0);
+  const long long shares = (long long)gridDim.x * g.rounds;
+
+  if (warp < L::NMMA) {
+    if constexpr (L::SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(L::REG_MMA));
+    const int gq = lane >> 2, tq = lane & 3;
+    const bool pair = warp < L::NPAIRW;
+    // pair warps: row tile warp / 2, columns 16 (warp & 1)..; tail warps: the
+    // last rows, columns 8 (warp - NPAIRW)..
+    const int r0 = (pair ? warp / 2 : PT) * 16 + gq, r1 = r0 + 8;
+    const int c0 = pair ? 16 * (warp & 1) : 8 * (warp - L::NPAIRW);
+    constexpr int KR = L::KR, NRT = PT + (TAIL ? 1 : 0);
+    double a0[KR], a1[KR];
+    const int rt = pair ? warp / 2 : PT;
+    double* const as = S.A + rt * 64 + lane;
+    auto load_a = [&](const double* h2e) {
+      auto at = [&](int r, int k) {
+        const int c = 4 * k + tq;
+        return r < npair && c < npair ? h2e[(long long)r * npair + c] : 0.0;
+      };
+#pragma unroll
+      for (int k = 0; k < KR; ++k) {
+        a0[k] = at(r0, k);
+        a1[k] = at(r1, k);
+      }
+      if constexpr (KS > KR) {  // shared by the warps of a row tile
+        const int nth = pair ? 64 : 128;
+        ws_bar_sync(6 + rt, nth);
+        for (int k = KR; k < KS; ++k) {
+          as[(k - KR) * NRT * 64] = at(r0, k);
+          as[(k - KR) * NRT * 64 + 32] = at(r1, k);
+        }
+        ws_bar_sync(6 + rt, nth);
+      }
+    };
+    bool ok = true;
+    int it = 0;
+    for (int r = 0; r < g.rounds; ++r) {
+      const long long q = (long long)r * gridDim.x + blockIdx.x;
+      long long t0 = total * q / shares;
+      const int n = it + (int)(total * (q + 1) / shares - t0);
+      if (it == n) continue;
+      for (int jb = mp_find<BATCH>(g, lane, &t0); it < n; ++jb) {  // job by job
+        const csffci_sigma_job_t& Q = BATCH ? g.jobs[jb] : g.job0;
+        const int end = BATCH ? it + (int)min((long long)(n - it), mp_job_tiles(Q) - t0) : n;
+        t0 = 0;
+        if (end == it) continue;
+        load_a(Q.h2e);
+        for (; it < end; ++it) {
+          const int s = it & 1;
+          const unsigned ph = (it >> 1) & 1;
+          if (ok) ok = mp_wait(&S.bar[s], ph);
+          const double* Db = S.D + s * dsz + tq * MP_DD + gq + c0;
+          double acc[2][4];
+#pragma unroll
+          for (int t = 0; t < 2; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0;
+          if (pair) {
+#pragma unroll
+            for (int k = 0; k < KS; ++k) {
+              const double x0 = k < KR ? a0[k < KR ? k : 0] : as[(k - KR) * NRT * 64];
+              const double x1 = k < KR ? a1[k < KR ? k : 0] : as[(k - KR) * NRT * 64 + 32];
+              rr_dmma16(acc[0], x0, x1, Db[4 * k * MP_DD]);
+              rr_dmma16(acc[1], x0, x1, Db[4 * k * MP_DD + 8]);
+            }
+          } else if (TAIL == 1) {
+            // two sums over alternate k-steps: the products of one would wait on each other
+#pragma unroll
+            for (int k = 0; k < KS; ++k)
+              rr_dmma16(acc[k & 1], k < KR ? a0[k < KR ? k : 0] : as[(k - KR) * NRT * 64],
+                        k < KR ? a1[k < KR ? k : 0] : as[(k - KR) * NRT * 64 + 32], Db[4 * k * MP_DD]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[0][i] += acc[1][i];
+          } else {
+#pragma unroll
+            for (int k = 0; k < KS; ++k)
+              ws_dmma(acc[k & 1][0], acc[k & 1][1], k < KR ? a0[k < KR ? k : 0] : as[(k - KR) * NRT * 64], Db[4 * k * MP_DD]);
+            acc[0][0] += acc[1][0];
+            acc[0][1] += acc[1][1];
+          }
+          __syncwarp();
+          if (lane == 0) mp_arrive(&S.bar[2 + s]);  // this warp has read D
+          if (it >= 2 && ok) ok = mp_wait(&S.bar[6 + s], ph ^ 1);  // V of tile it-2 is scattered
+          double* const V = S.V + s * vsz + c0 + 2 * tq;
+          *reinterpret_cast<double2*>(&V[r0 * MP_DV]) = make_double2(acc[0][0], acc[0][1]);
+          if (pair || TAIL == 1) *reinterpret_cast<double2*>(&V[r1 * MP_DV]) = make_double2(acc[0][2], acc[0][3]);
+          if (pair) {
+            *reinterpret_cast<double2*>(&V[r0 * MP_DV + 8]) = make_double2(acc[1][0], acc[1][1]);
+            *reinterpret_cast<double2*>(&V[r1 * MP_DV + 8]) = make_double2(acc[1][2], acc[1][3]);
+          }
+          __syncwarp();
+          if (lane == 0) mp_arrive(&S.bar[4 + s]);  // this warp's part of V is there
+        }
+      }
+    }
+    if (!ok) bad_s = 1;
+  } else {
+    if constexpr (L::SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(L::REG_MOV));
+    const int mw = warp - L::NMMA;
+    int it = 0;
+    for (int r = 0; r < g.rounds; ++r) {
+      const long long q = (long long)r * gridDim.x + blockIdx.x;
+      long long t0 = total * q / shares;
+      const int n = it + (int)(total * (q + 1) / shares - t0);
+      if (it == n) continue;
+      for (int jb = mp_find<BATCH>(g, lane, &t0); it < n; ++jb) {
+        const csffci_sigma_job_t& Q = BATCH ? g.jobs[jb] : g.job0;
+        const int m = BATCH ? (int)min((long long)(n - it), mp_job_tiles(Q) - t0) : n - it;
+        if (m > 0 && !mp_movers<KS, PT, TAIL, BATCH>(g, S, Q, t0, it, m, mw * 32 + lane, lane, mw)) bad_s = 1;
+        t0 = 0;
+        it += m;
+      }
+    }
+  }
+  __syncthreads();
+  // a hand-over that never came shows as NaN
+  if (bad_s && warp == 0) {
+    long long t = total * blockIdx.x / shares;
+    const int jb = mp_find<BATCH>(g, lane, &t);
+    const csffci_sigma_job_t& J = BATCH ? g.jobs[jb] : g.job0;
+    if (lane == 0) atomicAdd(J.sym ? J.scratch : J.sigma, __longlong_as_double(0x7ff8000000000000ll));
+  }
+}
+
+long long sigma_mp_tiles(const csffci_sigma_job_t& J) {
+  const long long m = J.Na / MP_NB, r = J.Na - m * MP_NB;
+  return J.sym ? (MP_NB / 2) * m * (m + 1) + r * (m + 1) : J.Na * ((J.Nb + MP_NB - 1) / MP_NB);
+}
+
+bool sigma_mp_supported(int norb) { return norb >= 4 && norb <= 13; }
+
+template <int KS, int PT, int TAIL, bool BATCH>
+static int mp_launch_as(int norb, MPArgs& g, long long max_nb, int max_nlb, long long max_tiles,
+                     long long nelem, cudaStream_t stream) {
+  using L = MPLayout<KS, PT, TAIL, BATCH>;
+  constexpr int DR = L::ROWS > 4 * KS ? L::ROWS : 4 * KS;
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += (bytes + 15) & ~(size_t)15;
+    return (unsigned)o;
+  };
+  take((size_t)2 * DR * MP_DD * sizeof(double));
+  g.off_v = take((size_t)2 * L::ROWS * MP_DV * sizeof(double));
+  g.off_a = take((size_t)L::AT * sizeof(double));
+  g.off_t = take((size_t)3 * g.npair * MP_TS * sizeof(unsigned));
+  g.lk_ld = MP_NB * max_nlb;
+  g.off_lk = take((size_t)2 * g.lk_ld * sizeof(uint2));
+  g.crow_ld = (int)((max_nb + 1) & ~1ll);
+  g.off_crow = take((size_t)2 * g.crow_ld * sizeof(double));
+  g.off_al = take((size_t)2 * g.npair * sizeof(uint2));
+  g.off_job = take(sizeof(MPJob));
+  g.off_bar = take(8 * sizeof(unsigned long long));
+  if (off > 227 * 1024 - 256) {
+    set_error("sigma: row-pair tiles exceed shared memory (%zu)", off);
+    return CSFFCI_ERR_INVALID;
+  }
+  auto kern = k_sigma_mp<KS, PT, TAIL, BATCH>;
+  if (L::SPLIT) {
+    // setmaxnreg re-splits the registers of the launch; with fewer the raise
+    // would wait forever
+    cudaFuncAttributes fa;
+    CSF_CUDA(cudaFuncGetAttributes(&fa, kern));
+    if (fa.numRegs != L::REG_LAUNCH) {
+      set_error("sigma: row-pair kernel compiled to %d registers per thread, not %d", fa.numRegs, L::REG_LAUNCH);
+      return CSFFCI_ERR_INVALID;
+    }
+  }
+  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)off));
+  // one CTA per SM; more of them where a share would outgrow the table tags
+  const long long need = (max_tiles + MP_MAX_TILES - 1) / MP_MAX_TILES;
+  const int grid = (int)(max_tiles < 148 ? (max_tiles > 0 ? max_tiles : 1) : need > 148 ? need : 148);
+  g.rounds = (int)(nelem * 16 / MP_ROUND + 1);
+  if (g.rounds > 256) g.rounds = 256;
+  static const char* names[10] = {"k_sigma_mp_n4", "k_sigma_mp_n5", "k_sigma_mp_n6",  "k_sigma_mp_n7",  "k_sigma_mp_n8",
+                                  "k_sigma_mp_n9", "k_sigma_mp_n10", "k_sigma_mp_n11", "k_sigma_mp_n12", "k_sigma_mp_n13"};
+  ProfScope ps(BATCH ? names[norb - 4] : "k_sigma_mp", stream);
+  kern<<<grid, L::NTH, off, stream>>>(g);
+  return check_launch("sigma (pair rows)");
+}
+
+template <int KS, int PT, int TAIL>
+static int mp_launch(int norb, MPArgs& g, long long max_nb, int max_nlb, long long max_tiles, long long nelem,
+                     cudaStream_t stream) {
+  return g.jobs ? mp_launch_as<KS, PT, TAIL, true>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream)
+                : mp_launch_as<KS, PT, TAIL, false>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+}
+
+// max_tiles: tiles of all jobs when every one is live
+int sigma_mp_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, const csffci_sigma_job_t& job0,
+                    long long max_nb, int max_nlb, long long max_tiles,
+                     long long nelem, cudaStream_t stream) {
+  MPArgs g;
+  memset(&g, 0, sizeof(g));
+  g.jobs = jobs_dev;
+  g.job0 = job0;
+  g.njobs = jobs_dev ? njobs : 1;
+  g.npair = norb * (norb + 1) / 2;
+  switch (norb) {  // KS = ceil(npair / 4); 10, 15, 21, 28, 36, 45, 55, 66, 78, 91 pair rows
+    case 4: return mp_launch<3, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 5: return mp_launch<4, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 6: return mp_launch<6, 2, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 7: return mp_launch<7, 2, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 8: return mp_launch<9, 2, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 9: return mp_launch<12, 2, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 10: return mp_launch<14, 4, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 11: return mp_launch<17, 4, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 12: return mp_launch<20, 4, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 13: return mp_launch<23, 6, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    default: break;
+  }
+  set_error("sigma: no row-pair kernel for norb %d", norb);
+  return CSFFCI_ERR_INVALID;
+}
+
+}  // namespace csffci

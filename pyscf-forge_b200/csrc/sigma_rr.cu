@@ -42,13 +42,11 @@ static bool rr_aligned8(const void* p) { return ((uintptr_t)p & 7u) == 0; }
 // Tile shapes (rows per warp, n-tiles of 8 columns): 16-row warps halve
 // the B-fragment traffic but need 2*KS + 4*NT doubles of registers per lane;
 // with 9 warps (norb 15,16) an SMSP holds 3 warps, i.e. at most 168
-// registers, so those sizes have no (16, 4) instance.  Where the
-// warp-specialised kernel is not the default (rr_default_variant), the
-// fastest shapes measured on B200 for one singlet/doublet problem are
-// (16, 2) up to norb 10 and at 13, (8, 2) for 11-12, (8, 4) from 14 (the
-// two-n-tile shapes run 2-3 CTAs per SM at small norb); CSFFCI_SIGMA_VARIANT
-// overrides the choice and the batched solver's autotuner picks per orbital
-// count.
+// registers, so those sizes have no (16, 4) instance.  The warp-specialised
+// kernels are the default from 4 orbitals on (rr_default_variant);
+// CSFFCI_SIGMA_VARIANT overrides the choice and the batched solver's
+// autotuner picks per orbital count (many small problems of 6, 7 or 10
+// orbitals run a few percent faster with a tile shape or variant 7).
 static const int kVariantShape[RR_NVARIANT][2] = {{16, 4}, {8, 4}, {16, 2}, {8, 2}};
 
 bool rr_variant_valid(int norb, int v) { return v >= 0 && v < RR_NVARIANT && !(v == 0 && norb >= 15); }
@@ -68,30 +66,29 @@ int sigma_rr_single_variant(int norb) {
     if ((v == RR_VARIANT_WSR || v == RR_VARIANT_WSR_BULK) && sigma_wsr_supported(norb)) return v;
     if (rr_variant_valid(norb, v)) return v;
   }
-  // measured on B200 (one problem), best tile shape -> k_sigma_ws: 10
-  // orbitals (5,5) singlet 0.044 -> 0.042 ms, 11 (6,5) 0.191 -> 0.167 ms,
-  // 12 (6,6) singlet 0.444 -> 0.349 ms, 12 (7,6) 0.572 -> 0.507 ms, 14
-  // singlet 7.61 -> 6.31 ms, 15: 31.1 -> 25.8 ms, 16: 148.8 -> 129.5 ms and
-  // 116 ms (k_sigma_wsr, registers re-split between the roles); at 13 the
-  // warp-specialised kernel is no faster, at 9 and below the tile shapes
-  // are faster
+  // 16 orbitals, one singlet: 148.8 ms (best tile shape), 129.5 ms
+  // (k_sigma_ws), 117 ms (k_sigma_wsr, registers re-split between the roles)
   if (sigma_wsr_supported(norb)) return RR_VARIANT_WSR;
   return rr_default_variant(norb);
 }
 
-// job tables (and one problem below 16 orbitals): the warp-specialised
-// kernel at 10..12 and 14..16 orbitals (the C3 batch of 128 problems: norb
-// 12 jobs 24.6 -> 23.2 ms per launch, norb 11 4.40 -> 3.99 ms, norb 10
-// 0.89 -> 0.85 ms against the best tile shape); the batched solver's
-// autotuner times every variant on its own job tables
+// Job tables and one problem below 16 orbitals: variant 4 from 4 orbitals on,
+// up to 13 k_sigma_mp, then k_sigma_ws.  Measured on B200, the best of the
+// other kernels -> k_sigma_mp (kernel time, us), one problem: 6 orbitals
+// (3,3) singlet 7.6 -> 4.5, 8 (4,4) singlet 12.4 -> 5.2, 9 (4,4) singlet
+// 17.2 -> 9.1, 11 (6,5) 159 -> 117, 12 (6,6) singlet 340 -> 278, 13 (7,6)
+// 2595 -> 2020; tables of 20 large problems: 10 orbitals 383 -> 403, 11
+// 1650 -> 1435, 12 7440 -> 6830; of 30 small ones: 8 orbitals 25 -> 22, 10
+// 68 -> 62, 12 198 -> 172.  k_sigma_ws against the best tile shape: 14
+// orbitals singlet 7.61 -> 6.31 ms, 15: 31.1 -> 25.8 ms.  The batched
+// solver's autotuner times every variant on its own job tables.
 int rr_default_variant(int norb) {
   const char* env = getenv("CSFFCI_SIGMA_VARIANT");
   if (env) {
     const int v = atoi(env);
     if (batch_variant_valid(norb, v)) return v;
   }
-  if (norb >= 10 && norb != 13 && sigma_ws_supported(norb)) return RR_VARIANT_WS;
-  return norb <= 10 || norb == 13 ? 2 : norb <= 12 ? 3 : 1;
+  return sigma_ws_supported(norb) ? RR_VARIANT_WS : 2;
 }
 
 // fill the bookkeeping fields of the jobs; returns the largest Nb, nla, nlb
@@ -122,7 +119,8 @@ static void rr_prepare(int norb, int njobs, csffci_sigma_job_t* jobs, long long*
 
 int sigma_rr_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev,
                     const csffci_sigma_job_t& job0, long long total_units, long long max_nb,
-                    int max_nla, int max_nlb, cudaStream_t stream, int variant, long long det_stride) {
+                    int max_nla, int max_nlb, cudaStream_t stream, int variant, long long det_stride,
+                    long long mp_tiles, long long nelem) {
   const int npair = norb * (norb + 1) / 2;
   const int ks = (npair + 3) / 4;
   if (det_stride)  // the deterministic scatter exists in the warp-specialised kernel only
@@ -130,6 +128,9 @@ int sigma_rr_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev,
                            det_stride);
   if (variant < 0 && !jobs_dev) variant = sigma_rr_single_variant(norb);
   if (variant < 0) variant = rr_default_variant(norb);
+  if (variant == RR_VARIANT_WS && sigma_mp_supported(norb))  // the deterministic scatter went above
+    return sigma_mp_launch(norb, njobs, jobs_dev, job0, max_nb, max_nlb,
+                           jobs_dev ? mp_tiles : sigma_mp_tiles(job0), nelem, stream);
   if (variant == RR_VARIANT_WS || variant == RR_VARIANT_WS16)
     return sigma_ws_launch(norb, njobs, jobs_dev, job0, total_units, max_nb, max_nla, max_nlb, stream,
                            variant == RR_VARIANT_WS16 ? 16 : 8);
@@ -347,6 +348,8 @@ int sigma_batch_prepare(int norb, int njobs, csffci_sigma_job_t* jobs, SigmaBatc
   for (int i = 0; i < njobs; ++i)
     if (jobs[i].sym) info->ntiles = jobs[i].tile_begin + ((jobs[i].Na + 31) / 32) * ((jobs[i].Na + 31) / 32);
   info->job0 = jobs[0];
+  info->mp_tiles = 0;
+  for (int i = 0; i < njobs; ++i) info->mp_tiles += sigma_mp_tiles(jobs[i]);
   info->det = (jobs[0].flags & CSFFCI_SIGMA_JOB_DETERMINISTIC) ? 1 : 0;
   if (info->det) info->variant = RR_VARIANT_WS;  // the only kernel with the deterministic scatter
   return CSFFCI_OK;
@@ -379,7 +382,7 @@ int sigma_batch_launch(const SigmaBatchInfo& info, const csffci_sigma_job_t* dj,
     return check_launch("sigma_batch deterministic symmetric finish");
   }
   st = table ? sigma_rr_launch(info.norb, njobs, dj, info.job0, info.total_units, info.max_nb,
-                               info.max_nla, info.max_nlb, stream, info.variant)
+                               info.max_nla, info.max_nlb, stream, info.variant, 0, info.mp_tiles, info.nelem)
              : sigma_rr_launch(info.norb, 1, nullptr, info.job0, info.total_units, info.max_nb,
                                info.max_nla, info.max_nlb, stream, info.variant);
   if (st) return st;

@@ -58,11 +58,19 @@ __device__ __forceinline__ void det_add3(double* p, long long stride, double x) 
   atomicAdd(w + 2 * stride, (unsigned long long)(long long)h2);
 }
 
+// FP64 add to global memory.  The vectors' addresses come from a job in
+// memory, and for a pointer of unknown space the compiler also lays down the
+// add to shared memory (a compare-and-swap loop) and its registers.
+__device__ __forceinline__ void rr_red(double* p, double x) {
+  __builtin_assume(__isGlobal(p));
+  atomicAdd(p, x);
+}
+
 // one scattered contribution: an FP64 atomic, or the three digit atomics
 template <bool DET>
 __device__ __forceinline__ void ws_out_add(double* p, double x, long long stride) {
   if (DET) det_add3(p, stride, x);
-  else atomicAdd(p, x);
+  else rr_red(p, x);
 }
 
 // Alpha link of the current row Ja as the tile loops use it: the offset
@@ -393,7 +401,7 @@ __global__ void __launch_bounds__(RRLayout<MT, MW, NT>::NW * 32, (rr_min_blocks<
             const int nlb = sjob.nlb;
             for (int m = warp * MPW + ml; m < nlb; m += NW * MPW) {
               const uint2 e = rr_link(&Lt[jl * LS + m]);
-              atomicAdd(&orow[e.x], rr_flip(D[rr_lpair(e) * ds + jl], rr_lneg(e)));
+              rr_red(&orow[e.x], rr_flip(D[rr_lpair(e) * ds + jl], rr_lneg(e)));
             }
             // alpha scatter sigma[Ka][Jb] through the links of Ja (coalesced
             // over Jb); in the spin-symmetric mode only Jb < Ja
@@ -403,7 +411,7 @@ __global__ void __launch_bounds__(RRLayout<MT, MW, NT>::NW * 32, (rr_min_blocks<
               const int nla = sjob.nla;
               for (int l = warp * MPW + ml; l < nla; l += NW * MPW) {
                 const RRAlpha a = al[l];
-                atomicAdd(&ocol[a.off], rr_flip(D[a.drow + jl], a.neg));
+                rr_red(&ocol[a.off], rr_flip(D[a.drow + jl], a.neg));
               }
             }
           }
@@ -465,13 +473,18 @@ constexpr int RR_VARIANT_WSR_BULK = 6;
 bool sigma_wsr_supported(int norb);
 int sigma_wsr_launch(int norb, const csffci_sigma_job_t& job0, long long total_units, long long max_nb,
                      int max_nla, int max_nlb, cudaStream_t stream, bool bulk);
+// variant 4 without the deterministic scatter at 4..13 orbitals (sigma_mp.cu)
+bool sigma_mp_supported(int norb);
+int sigma_mp_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, const csffci_sigma_job_t& job0,
+                    long long max_nb, int max_nlb, long long max_tiles, long long nelem, cudaStream_t stream);
+long long sigma_mp_tiles(const csffci_sigma_job_t& J);  // host: tiles of a prepared job
 bool rr_variant_valid(int norb, int v);
 // the variants a job table may run: the tile shapes and the warp-specialised kernel
 bool batch_variant_valid(int norb, int v);
 int rr_default_variant(int norb);
 int sigma_rr_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, const csffci_sigma_job_t& job0,
                     long long total_units, long long max_nb, int max_nla, int max_nlb, cudaStream_t stream,
-                    int variant, long long det_stride = 0);
+                    int variant, long long det_stride = 0, long long mp_tiles = 0, long long nelem = 0);
 int rr_dispatch_v0(int norb, RRArgs& g, size_t smem, cudaStream_t stream);  // (16, 4)
 int rr_dispatch_v1(int norb, RRArgs& g, size_t smem, cudaStream_t stream);  // (8, 4)
 int rr_dispatch_v2(int norb, RRArgs& g, size_t smem, cudaStream_t stream);  // (16, 2)

@@ -1,6 +1,7 @@
-// Warp-specialised variant of the register-resident sigma kernel, 4..16
-// orbitals: tile variant 4 (one MMA warp per 8 rows) and, up to 12 orbitals,
-// variant 7 (one MMA warp per 16 rows, m16n8k4, in CTAs of 8 warps).  Either
+// Warp-specialised variant of the register-resident sigma kernel: tile variant
+// 4 at 14..16 orbitals (one MMA warp per 8 rows; below that k_sigma_mp, and
+// here only the deterministic scatter) and, at 8..12 orbitals, variant 7 (one
+// MMA warp per 16 rows, m16n8k4, in CTAs of 8 warps).  Either
 // runs one problem or a job table of many (BATCH: each unit's job is looked
 // up between two barrier-9 syncs, gated jobs are skipped by both roles); the
 // form with 8-row warps also has the deterministic scatter (DET: integer
@@ -268,11 +269,17 @@ static int launch_ws(RRArgs& g, size_t smem, cudaStream_t stream) {
   constexpr int NTH = WSLayout<MT, MW>::NTOT * 32;
   // 16-row MMA warps: 8-warp CTAs, two per SM
   constexpr int MINB = MW == 16 ? 2 : ws_min_blocks(NORB);
-  // the deterministic scatter: one problem, 8-row MMA warps only
+  // the deterministic scatter: 8-row MMA warps only; up to 13 orbitals those
+  // have nothing else (k_sigma_mp takes the FP64 atomics)
+  constexpr bool ONLY_DET = MW == 8 && NORB <= 13;
+  if (ONLY_DET && !g.det_stride) {
+    set_error("sigma: no warp-specialised kernel with FP64 atomics here for norb %d", NORB);
+    return CSFFCI_ERR_INVALID;
+  }
   auto kern = g.jobs ? ((MW == 8 && g.det_stride) ? k_sigma_ws<KS, MT, MW, true, MINB, MW == 8>
-                                                  : k_sigma_ws<KS, MT, MW, true, MINB>)
+                                                  : k_sigma_ws<KS, MT, MW, true, MINB, ONLY_DET>)
                      : ((MW == 8 && g.det_stride) ? k_sigma_ws<KS, MT, MW, false, MINB, MW == 8>
-                                                  : k_sigma_ws<KS, MT, MW, false, MINB>);
+                                                  : k_sigma_ws<KS, MT, MW, false, MINB, ONLY_DET>);
   CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, nsm = 148, per_sm = 0;
   CSF_CUDA(cudaGetDevice(&dev));
@@ -286,14 +293,11 @@ static int launch_ws(RRArgs& g, size_t smem, cudaStream_t stream) {
   ws_split_last_round(g, grid);
   if (grid > g.total_units) grid = g.total_units;
   if (grid < 1) return CSFFCI_OK;
-  static const char* names8[17] = {"", "", "", "", "k_sigma_ws_n4", "k_sigma_ws_n5", "k_sigma_ws_n6",
-                                   "k_sigma_ws_n7", "k_sigma_ws_n8", "k_sigma_ws_n9",
-                                   "k_sigma_ws_n10", "k_sigma_ws_n11", "k_sigma_ws_n12", "k_sigma_ws_n13",
-                                   "k_sigma_ws_n14", "k_sigma_ws_n15", "k_sigma_ws_n16"};
+  static const char* names8[3] = {"k_sigma_ws_n14", "k_sigma_ws_n15", "k_sigma_ws_n16"};
   static const char* names16[13] = {"", "", "", "", "", "", "", "", "k_sigma_ws16_n8", "k_sigma_ws16_n9",
                                     "k_sigma_ws16_n10", "k_sigma_ws16_n11", "k_sigma_ws16_n12"};
   const char* name = MW == 16 ? (g.jobs ? names16[NORB <= 12 ? NORB : 0] : "k_sigma_ws16")
-                              : (g.jobs ? names8[NORB] : g.det_stride ? "k_sigma_ws_det" : "k_sigma_ws");
+                              : (g.det_stride ? "k_sigma_ws_det" : g.jobs ? names8[NORB >= 14 ? NORB - 14 : 0] : "k_sigma_ws");
   ProfScope ps(name, stream);
   kern<<<(int)grid, NTH, smem, stream>>>(g);
   return check_launch("sigma (warp-specialised)");
