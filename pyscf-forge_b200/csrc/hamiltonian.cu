@@ -45,37 +45,95 @@ __global__ void k_absorb_h2e(int norb, int npair, const double* h1e, const doubl
 //   e1[I] = sum_{i in I} h[i][i] + 1/2 sum_{i,j in I} (J_ij - K_ij)
 //   jv[I][q] = sum_{i in I} J_iq          (only for the alpha strings)
 // with J_ij = (ii|jj) = eri[ii][jj], K_ij = (ij|ji) = eri[ij][ij].
-__global__ void k_string_energy(int norb, int nelec, int npair, unsigned long long nstr,
-                                const double* h, const double* eri, double* e1, double* jv,
-                                uint64_t* strs_out) {
-  for (unsigned long long I = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; I < nstr;
-       I += (unsigned long long)gridDim.x * blockDim.x) {
-    unsigned long long s = str_unrank(norb, nelec, I);
-    if (strs_out) strs_out[I] = s;
+//
+// A warp per string of either spin, its lanes over q: the sums are chains of
+// loads, so what counts is how many run at once (one thread per string left
+// most of the GPU idle: 45 us a spin at 14 orbitals and 7 electrons, now
+// 10 us for both in one launch).
+__global__ void __launch_bounds__(128) k_string_energy(int norb, int neleca, int nelecb, int npair,
+                                                       unsigned long long na, unsigned long long nb,
+                                                       const double* __restrict__ ha, const double* __restrict__ hb,
+                                                       const double* __restrict__ eri, double* ea, double* ja,
+                                                       double* eb, uint64_t* sb) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  for (unsigned long long w = blockIdx.x * (unsigned long long)(blockDim.x >> 5) + (threadIdx.x >> 5); w < na + nb;
+       w += nw) {
+    const bool alpha = w < na;
+    const unsigned long long I = alpha ? w : w - na;
+    const unsigned long long s = str_unrank(norb, alpha ? neleca : nelecb, I);
+    const double* const h = alpha ? ha : hb;
     double e = 0.0;
-    for (int i = 0; i < norb; ++i) {
-      if (!((s >> i) & 1ull)) continue;
-      e += h[i * norb + i];
-      int ii = pair_index(i, i);
-      for (int j = 0; j < norb; ++j) {
-        if (!((s >> j) & 1ull)) continue;
-        int jj = pair_index(j, j), ij = pair_index(i, j);
-        e += 0.5 * (eri[(int64_t)ii * npair + jj] - eri[(int64_t)ij * npair + ij]);
-      }
+    for (int q = lane; q < norb; q += 32) {
+      const int qq = pair_index(q, q);
+      double j = 0.0, k = 0.0;
+#pragma unroll 4
+      for (int i = 0; i < norb; ++i)
+        if ((s >> i) & 1ull) {
+          const int iq = pair_index(i, q);
+          j += eri[(int64_t)pair_index(i, i) * npair + qq];
+          k += eri[(int64_t)iq * npair + iq];
+        }
+      if ((s >> q) & 1ull) e += h[q * norb + q] + 0.5 * (j - k);
+      if (alpha) ja[I * norb + q] = j;
     }
-    e1[I] = e;
-    if (jv) {
-      for (int q = 0; q < norb; ++q) {
-        int qq = pair_index(q, q);
-        double acc = 0.0;
-        for (int i = 0; i < norb; ++i)
-          if ((s >> i) & 1ull) acc += eri[(int64_t)pair_index(i, i) * npair + qq];
-        jv[I * norb + q] = acc;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+    if (lane == 0) {
+      if (alpha) {
+        ea[I] = e;
+      } else {
+        eb[I] = e;
+        sb[I] = s;
       }
     }
   }
 }
 
+// hdiag[ia][ib] = ea + eb + sum over the orbitals q of ib of ja[ia][q], by
+// tables of the sums over HD_BITS orbitals at a time, for HD_ROWS rows ia a
+// block: two table reads an element at 14 orbitals instead of a loop over 7
+// electrons (110 -> 26 us for 94 MB, which take 15 us to write).
+constexpr int HD_BITS = 7, HD_ROWS = 4;
+__global__ void __launch_bounds__(256) k_hdiag_det_table(int norb, unsigned long long Na, unsigned long long Nb,
+                                                         const double* __restrict__ ea, const double* __restrict__ eb,
+                                                         const double* __restrict__ ja, const uint64_t* __restrict__ sb,
+                                                         double* hdiag) {
+  extern __shared__ double hd_tab[];  // [chunk][row][2^HD_BITS]
+  constexpr int TS = 1 << HD_BITS;
+  const int nch = (norb + HD_BITS - 1) / HD_BITS;
+  const unsigned long long r0 = (unsigned long long)blockIdx.x * HD_ROWS;
+  for (int t = threadIdx.x; t < nch * HD_ROWS * TS; t += blockDim.x) {
+    const int m = t & (TS - 1), r = (t >> HD_BITS) % HD_ROWS, c = (t >> HD_BITS) / HD_ROWS;
+    const int q0 = c * HD_BITS;
+    double v = 0.0;
+    if (r0 + r < Na && q0 + (32 - __clz(m)) <= norb)
+      for (int b = m; b; b &= b - 1) v += ja[(r0 + r) * norb + q0 + __ffs(b) - 1];
+    hd_tab[t] = v;
+  }
+  double e[HD_ROWS];
+#pragma unroll
+  for (int r = 0; r < HD_ROWS; ++r) e[r] = r0 + r < Na ? ea[r0 + r] : 0.0;
+  __syncthreads();
+  for (unsigned long long ib = blockIdx.y * (unsigned long long)blockDim.x + threadIdx.x; ib < Nb;
+       ib += (unsigned long long)gridDim.y * blockDim.x) {
+    const double x = eb[ib];
+    double v[HD_ROWS];
+#pragma unroll
+    for (int r = 0; r < HD_ROWS; ++r) v[r] = e[r] + x;
+    unsigned long long s = sb[ib];
+    for (int c = 0; c < nch; ++c, s >>= HD_BITS) {
+      const double* const tab = hd_tab + c * HD_ROWS * TS + ((int)s & (TS - 1));
+#pragma unroll
+      for (int r = 0; r < HD_ROWS; ++r) v[r] += tab[r * TS];
+    }
+#pragma unroll
+    for (int r = 0; r < HD_ROWS; ++r)
+      if (r0 + r < Na) hdiag[(r0 + r) * Nb + ib] = v[r];
+  }
+}
+
+// the same, element by element
 __global__ void k_hdiag_det(int norb, unsigned long long Na, unsigned long long Nb,
                             const double* __restrict__ ea, const double* __restrict__ eb,
                             const double* __restrict__ ja, const uint64_t* __restrict__ sb,
@@ -94,6 +152,31 @@ __global__ void k_hdiag_det(int norb, unsigned long long Na, unsigned long long 
     }
     hdiag[t] = v;
   }
+}
+
+// both launches of the determinant diagonal; ea, ja, eb and sb are scratch
+static int hdiag_det_run(int norb, int neleca, int nelecb, unsigned long long Na, unsigned long long Nb,
+                         const double* h1a, const double* h1b, const double* eri, double* ea, double* ja, double* eb,
+                         uint64_t* sb, double* hdiag, cudaStream_t stream) {
+  const int npair = norb * (norb + 1) / 2;
+  k_string_energy<<<grid_for((long long)(Na + Nb) * 32, 128), 128, 0, stream>>>(norb, neleca, nelecb, npair, Na, Nb,
+                                                                                h1a, h1b, eri, ea, ja, eb, sb);
+  const int st = check_launch("hdiag_det strings");
+  if (st) return st;
+  ProfScope ps_("k_hdiag_det", stream);
+  const unsigned long long nx = (Na + HD_ROWS - 1) / HD_ROWS;
+  // a row has to be longer than a table for the tables to pay
+  if (Nb >= (1u << HD_BITS) && nx <= 0x7fffffffull) {
+    // the columns are split where the rows leave the GPU idle (8 blocks a SM)
+    unsigned long long ny = (148 * 8 + nx - 1) / nx, most = (Nb + 1023) / 1024;
+    if (ny > most) ny = most;
+    const size_t smem = (size_t)((norb + HD_BITS - 1) / HD_BITS) * HD_ROWS * (1 << HD_BITS) * sizeof(double);
+    k_hdiag_det_table<<<dim3((unsigned)nx, (unsigned)ny), 256, smem, stream>>>(norb, Na, Nb, ea, eb, ja, sb, hdiag);
+  } else {
+    k_hdiag_det<<<grid_for((long long)(Na * Nb), 256, 148 * 32), 256, 0, stream>>>(norb, Na, Nb, ea, eb, ja, sb,
+                                                                                  hdiag);
+  }
+  return check_launch("hdiag_det");
 }
 
 // ---------------------------------------------------------------------------
@@ -203,6 +286,81 @@ __global__ void k_contract_1e(int norb, unsigned long long Na, unsigned long lon
   }
 }
 
+// The same for C1_ROWS rows ka a block: their rows of c, their alpha links
+// (coefficient and row) and hb in shared memory, and every beta link read once
+// for all of them.  Element by element each of the nla + nlb links cost two
+// dependent loads and a look at h, at 11% of the issue slots.  11 orbitals
+// (6,5): 41 us, now 20 us, most of it the latency of the rows of c that the
+// alpha links read from L2.
+constexpr int C1_ROWS = 4;
+struct C1Link {
+  double v;
+  long long off;
+};
+__global__ void __launch_bounds__(256) k_contract_1e_rows(int norb, long long Na, int Nb, int nla, int nlb,
+                                                          const double* __restrict__ ha, const double* __restrict__ hb,
+                                                          const csffci_link_t* __restrict__ la,
+                                                          const csffci_link_t* __restrict__ lb,
+                                                          const double* __restrict__ ci, double* sigma) {
+  extern __shared__ __align__(16) unsigned char c1_smem[];
+  double* const crow = (double*)c1_smem;                          // [C1_ROWS][Nb]
+  C1Link* const al = (C1Link*)(c1_smem + (((size_t)C1_ROWS * Nb * sizeof(double) + 15) & ~(size_t)15));
+  double* const hs = (double*)(al + (size_t)C1_ROWS * nla);       // [norb][norb]
+  const long long r0 = (long long)blockIdx.x * C1_ROWS;
+  const int nr = (int)min((long long)C1_ROWS, Na - r0);
+  for (int t = threadIdx.x; t < C1_ROWS * Nb; t += blockDim.x) crow[t] = t < nr * Nb ? ci[r0 * Nb + t] : 0.0;
+  for (int t = threadIdx.x; t < C1_ROWS * nla; t += blockDim.x) {
+    C1Link x{0.0, 0};
+    if (t < nr * nla) {
+      const csffci_link_t e = la[r0 * nla + t];
+      x.v = e.sign * ha[(e.op >> 8) * norb + (e.op & 0xff)];
+      x.off = (long long)e.addr * Nb;
+    }
+    al[t] = x;
+  }
+  for (int t = threadIdx.x; t < norb * norb; t += blockDim.x) hs[t] = hb[t];
+  __syncthreads();
+  for (int kb = blockIdx.y * blockDim.x + threadIdx.x; kb < Nb; kb += gridDim.y * blockDim.x) {
+    double acc[C1_ROWS];
+#pragma unroll
+    for (int r = 0; r < C1_ROWS; ++r) acc[r] = 0.0;
+    // loads in batches of 16: left to itself the compiler waits for each
+    const double* const cb = ci + kb;
+    for (int l0 = 0; l0 < nla; l0 += 4) {
+      double x[4][C1_ROWS];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int r = 0; r < C1_ROWS; ++r) x[k][r] = l0 + k < nla ? __ldg(&cb[al[r * nla + l0 + k].off]) : 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int r = 0; r < C1_ROWS; ++r)
+          if (l0 + k < nla) acc[r] += al[r * nla + l0 + k].v * x[k][r];
+    }
+    // a link is two loads, not one per field: address; op, sign and pad
+    const unsigned* const L = reinterpret_cast<const unsigned*>(lb + (long long)kb * nlb);
+    for (int l0 = 0; l0 < nlb; l0 += 8) {
+      unsigned to[8], w[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        to[k] = l0 + k < nlb ? __ldg(&L[2 * (l0 + k)]) : 0u;
+        w[k] = l0 + k < nlb ? __ldg(&L[2 * (l0 + k) + 1]) : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const double v = (double)((int)(w[k] << 8) >> 24) * hs[((w[k] >> 8) & 0xffu) * norb + (w[k] & 0xffu)];
+#pragma unroll
+        for (int r = 0; r < C1_ROWS; ++r)
+          if (l0 + k < nlb) acc[r] += v * crow[r * Nb + to[k]];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < C1_ROWS; ++r)
+      if (r < nr) sigma[(r0 + r) * Nb + kb] += acc[r];
+  }
+}
+
 }  // namespace csffci
 
 using namespace csffci;
@@ -235,26 +393,12 @@ int csffci_hdiag_det(int norb, int neleca, int nelecb, const double* h1a, const 
     set_error("hdiag_det: workspace of %zu bytes < %zu required", work_bytes, need);
     return CSFFCI_ERR_MEMORY;
   }
-  int npair = norb * (norb + 1) / 2;
   unsigned long long Na = host_binom(norb, neleca), Nb = host_binom(norb, nelecb);
   double* ea = (double*)work;
   double* ja = ea + Na;
   double* eb = ja + Na * norb;
   uint64_t* sb = (uint64_t*)(eb + Nb);
-  k_string_energy<<<grid_for((long long)Na, 128), 128, 0, stream>>>(norb, neleca, npair, Na, h1a,
-                                                                    eri, ea, ja, nullptr);
-  int st = check_launch("hdiag_det alpha strings");
-  if (st) return st;
-  k_string_energy<<<grid_for((long long)Nb, 128), 128, 0, stream>>>(norb, nelecb, npair, Nb, h1b,
-                                                                    eri, eb, nullptr, sb);
-  st = check_launch("hdiag_det beta strings");
-  if (st) return st;
-  {
-    ProfScope ps_("k_hdiag_det", stream);
-    k_hdiag_det<<<grid_for((long long)(Na * Nb), 256, 148 * 32), 256, 0, stream>>>(norb, Na, Nb, ea,
-                                                                                    eb, ja, sb, hdiag);
-  }
-  return check_launch("hdiag_det");
+  return hdiag_det_run(norb, neleca, nelecb, Na, Nb, h1a, h1b, eri, ea, ja, eb, sb, hdiag, stream);
 }
 
 int csffci_pspace_h0(int norb, int neleca, int nelecb, const double* h1a, const double* h1b,
@@ -278,6 +422,20 @@ int csffci_contract_1e(int norb, int neleca, int nelecb, const double* h1a, cons
   CSF_REQUIRE(norb >= 1 && norb <= 63, "contract_1e: bad norb %d", norb);
   unsigned long long Na = host_binom(norb, neleca), Nb = host_binom(norb, nelecb);
   int nla = neleca * (norb - neleca + 1), nlb = nelecb * (norb - nelecb + 1);
+  // rows that fit in shared memory (7000 columns at 16 orbitals)
+  const size_t smem = (((size_t)C1_ROWS * Nb * sizeof(double) + 15) & ~(size_t)15) +
+                      (size_t)C1_ROWS * nla * sizeof(C1Link) + (size_t)norb * norb * sizeof(double);
+  if (Na > 0 && Nb > 0 && Na < (1ull << 31) && Nb < (1ull << 24) && smem <= 227 * 1024 - 1024) {
+    if (smem > 48 * 1024)
+      CSF_CUDA(cudaFuncSetAttribute(k_contract_1e_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const long long nx = ((long long)Na + C1_ROWS - 1) / C1_ROWS;
+    // few rows: the columns are split as well
+    long long ny = (2 * 148 + nx - 1) / nx, most = ((long long)Nb + 255) / 256;
+    if (ny > most) ny = most;
+    k_contract_1e_rows<<<dim3((unsigned)nx, (unsigned)ny), 256, smem, stream>>>(
+        norb, (long long)Na, (int)Nb, nla, nlb, h1a, h1b, link_a, link_b, ci, sigma);
+    return check_launch("contract_1e");
+  }
   k_contract_1e<<<grid_for((long long)(Na * Nb), 256, 148 * 32), 256, 0, stream>>>(
       norb, Na, Nb, nla, nlb, h1a, h1b, link_a, link_b, ci, sigma);
   return check_launch("contract_1e");
@@ -382,20 +540,9 @@ extern "C" int csffci_hdiag_det_noalloc(int norb, int neleca, int nelecb, const 
   }
   // Every entry of the scratch that the kernels read is written first by the
   // same call (ea, ja, eb and the beta strings), so nothing needs clearing.
-  const int npair = norb * (norb + 1) / 2;
   double* ea = (double*)base;
   double* ja = ea + Na;
   double* eb = ja + Na * norb;
   uint64_t* sb = (uint64_t*)(eb + Nb);
-  k_string_energy<<<grid_for((long long)Na, 128), 128, 0, stream>>>(norb, neleca, npair, Na, h1a,
-                                                                    eri, ea, ja, nullptr);
-  int st = check_launch("hdiag_det_noalloc alpha strings");
-  if (st) return st;
-  k_string_energy<<<grid_for((long long)Nb, 128), 128, 0, stream>>>(norb, nelecb, npair, Nb, h1b,
-                                                                    eri, eb, nullptr, sb);
-  st = check_launch("hdiag_det_noalloc beta strings");
-  if (st) return st;
-  k_hdiag_det<<<grid_for((long long)(Na * Nb), 256, 148 * 32), 256, 0, stream>>>(norb, Na, Nb, ea,
-                                                                                  eb, ja, sb, hdiag);
-  return check_launch("hdiag_det_noalloc");
+  return hdiag_det_run(norb, neleca, nelecb, Na, Nb, h1a, h1b, eri, ea, ja, eb, sb, hdiag, stream);
 }
