@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from .. import _capi
-from .._runtime import device, eri_pair_matrix, like_input, ptr, require_cuda, stream, to_dev
+from .._runtime import dev_eri_pair_matrix, device, like_input, ptr, require_cuda, stream, to_dev
 from ..fci import direct_spin1
 from ..fci.davidson import DiagPrecond, davidson, gram
 from ..fci.direct_spin1 import _unpack_nelec
@@ -53,15 +53,19 @@ class H2eff:
 
 def make_hdiag_det(fci, h1e, eri, norb, nelec):
     """csf.py:66-68 (two-component h1e)."""
-    ha, hb = unpack_h1e_ab(h1e)
-    return direct_spin1.dev_make_hdiag(ha, hb, eri_pair_matrix(eri, norb), norb, _unpack_nelec(nelec))
+    if isinstance(h1e, torch.Tensor) and h1e.is_cuda:  # used where it is
+        h = h1e.detach()
+        ha, hb = (h[0], h[1]) if h.ndim == 3 and h.shape[0] == 2 else (h, h)
+    else:
+        ha, hb = unpack_h1e_ab(h1e)
+    return direct_spin1.dev_make_hdiag(ha, hb, dev_eri_pair_matrix(eri, norb), norb, _unpack_nelec(nelec))
 
 
 def make_hdiag_csf(h1e, eri, norb, nelec, transformer, hdiag_det=None, max_memory=None):
     """csf.py:70-144, computed configuration by configuration on the device
     (no (nconf, ndet, ndet) blocks are materialised, so no MemoryError path
     is needed)."""
-    eri4 = to_dev(eri_pair_matrix(eri, norb))
+    eri4 = dev_eri_pair_matrix(eri, norb)
     if hdiag_det is None:
         hdiag_det = make_hdiag_det(None, h1e, eri, norb, nelec)
     return transformer.dev_hdiag_csf(to_dev(hdiag_det).reshape(-1), eri4)
@@ -137,7 +141,7 @@ def pspace(fci, h1e, eri, norb, nelec, transformer, hdiag_det=None, hdiag_csf=No
     if max_memory is None:
         max_memory = getattr(fci, 'max_memory', None)
     neleca, nelecb = _unpack_nelec(nelec)
-    eri4 = to_dev(eri_pair_matrix(eri, norb))
+    eri4 = dev_eri_pair_matrix(eri, norb)
     if hdiag_det is None:
         hdiag_det = make_hdiag_det(fci, h1e, eri, norb, nelec)
     hdiag_det = to_dev(hdiag_det).reshape(-1)
@@ -284,7 +288,7 @@ def kernel(fci, h1e, eri, norb, nelec, smult=None, idx_sym=None, ci0=None, tol=N
         precond = fci.make_precond(to_dev(hdiag_csf).reshape(-1)[idx_sym], pw, pv, pos[addr])
     h2e = fci.absorb_h1e(h1e, eri, norb, nelec, .5)
     if not isinstance(h2e, H2eff):
-        h2e = H2eff(to_dev(eri_pair_matrix(h2e, norb)))
+        h2e = H2eff(dev_eri_pair_matrix(h2e, norb))
     hop = _Hop(transformer, h2e, norb, nelec, deterministic=getattr(fci, 'deterministic_sigma', False))
 
     if ci0 is None:
@@ -454,7 +458,7 @@ class CSFFCISolver:
 
     def absorb_h1e(self, h1e, eri, norb, nelec, fac=1):
         h1e_c, h1e_s = unpack_h1e_cs(h1e)
-        h2e = direct_spin1.dev_absorb_h1e(h1e_c, eri_pair_matrix(eri, norb), norb, nelec, fac)
+        h2e = direct_spin1.dev_absorb_h1e(h1e_c, dev_eri_pair_matrix(eri, norb), norb, nelec, fac)
         return H2eff(h2e, h1e_s)
 
     def contract_2e(self, eri, fcivec, norb, nelec, link_index=None, out=None, **kwargs):
@@ -466,7 +470,7 @@ class CSFFCISolver:
         if isinstance(eri, H2eff):
             h2e, h1e_s = eri.h2e, eri.h1e_s
         else:
-            h2e, h1e_s = to_dev(eri_pair_matrix(eri, norb)), None
+            h2e, h1e_s = dev_eri_pair_matrix(eri, norb), None
         ci = to_dev(fcivec).reshape(-1)
         if out is not None and (not isinstance(out, torch.Tensor) or out.numel() != ci.numel()
                                 or out.dtype != torch.float64 or not out.is_contiguous()):

@@ -57,21 +57,37 @@ class DiagPrecond:
         self.hd_addr = None if addr is None else self.hdiag[self.addr].cpu().numpy()
 
     def __call__(self, r, e, x):
-        n = r.numel()
-        t = torch.empty_like(r)
+        return self.block([r], [e], [x]).reshape(r.shape)
+
+    def block(self, r, e, x):
+        """The corrections of several (r, e, x) as rows of one tensor.  What
+        the host needs of them (the two sums and the p-space elements) comes
+        over in one copy."""
+        k, n = len(r), r[0].numel()
+        t = torch.empty((k, n), dtype=r[0].dtype, device=r[0].device)
         nbytes = _capi.query("csffci_precond_workspace")
         ws = workspace("precond", nbytes)
         if self.pw is None:
-            _capi.call("csffci_precond", n, ptr(r), ptr(x), ptr(self.hdiag), float(e), self.shift, 1,
-                       0.0, ptr(t), ptr(ws), stream())
+            for i in range(k):
+                _capi.call("csffci_precond", n, ptr(r[i]), ptr(x[i]), ptr(self.hdiag), float(e[i]), self.shift, 1,
+                           0.0, ptr(t[i]), ptr(ws), stream())
             return t
-        dots = torch.empty(2, dtype=torch.float64, device=r.device)
-        _capi.call("csffci_precond_dots", n, ptr(r), ptr(x), ptr(self.hdiag), float(e), self.shift,
-                   ptr(dots), ptr(ws), stream())
-        a, b = dots.cpu().numpy()
+        na = self.addr.numel()
+        small = torch.empty((k, 2 + 2 * na), dtype=t.dtype, device=t.device)  # dots, x and r on the p-space
+        for i in range(k):
+            _capi.call("csffci_precond_dots", n, ptr(r[i]), ptr(x[i]), ptr(self.hdiag), float(e[i]), self.shift,
+                       ptr(small[i]), ptr(ws), stream())
+            torch.index_select(x[i].reshape(-1), 0, self.addr, out=small[i, 2:2 + na])
+            torch.index_select(r[i].reshape(-1), 0, self.addr, out=small[i, 2 + na:])
+        small = small.cpu().numpy()
+        for i in range(k):
+            e1 = self._e1(float(e[i]), small[i, 0], small[i, 1], small[i, 2:2 + na], small[i, 2 + na:])
+            _capi.call("csffci_precond", n, ptr(r[i]), ptr(x[i]), ptr(self.hdiag), float(e[i]), self.shift, 2,
+                       float(e1), ptr(t[i]), ptr(ws), stream())
+        return t
+
+    def _e1(self, e, a, b, xa, ra):
         es = e - self.shift
-        xa = x[self.addr].cpu().numpy()
-        ra = r[self.addr].cpu().numpy()
         hinv = 1.0 / (self.hd_addr - es)
         hinv[np.abs(hinv) > 1e8] = 1e8
         # replace the diagonal inverse on the p-space by the exact block
@@ -80,10 +96,7 @@ class DiagPrecond:
         h0e0inv = (self.pv / (self.pw - es)) @ self.pv.T
         a += xa @ (h0e0inv @ ra)
         b += xa @ (h0e0inv @ xa)
-        e1 = a / b if b != 0 else 0.0
-        _capi.call("csffci_precond", n, ptr(r), ptr(x), ptr(self.hdiag), float(e), self.shift, 2,
-                   float(e1), ptr(t), ptr(ws), stream())
-        return t
+        return a / b if b != 0 else 0.0
 
 
 def _orthonormalise_per_vector(V, m, new, lindep):
@@ -95,8 +108,7 @@ def _orthonormalise_per_vector(V, m, new, lindep):
         t = new[i:i + 1].clone()
         for _ in range(2):
             if m + len(added):
-                cf = gram(V[:m + len(added)], t).cpu().numpy().T
-                combine(t, V[:m + len(added)], -cf, beta=1.0)
+                combine(t, V[:m + len(added)], -gram(V[:m + len(added)], t).T, beta=1.0)
         nrm2 = float(gram(t, t).cpu().numpy()[0, 0])
         if nrm2 > lindep:
             V[m + len(added)].copy_(t[0] / np.sqrt(nrm2))
@@ -117,8 +129,7 @@ def _orthonormalise_into(V, m, new, lindep):
     T = new.clone()
     for _ in range(2):
         if m:
-            cf = gram(V[:m], T).cpu().numpy()          # (m, k)
-            combine(T, V[:m], -cf.T, beta=1.0)
+            combine(T, V[:m], -gram(V[:m], T).T, beta=1.0)  # coefficients (m, k) stay on the device
     G = gram(T, T).cpu().numpy()
     G = 0.5 * (G + G.T)
     acc = []
@@ -200,8 +211,9 @@ def davidson(aop, x0, precond, tol=1e-10, max_cycle=100, max_space=12, lindep=1e
             idx = list(range(k))
         e = w[idx]
         cc = np.ascontiguousarray(c[:, idx].T)
-        combine(X, V[:m], cc)
-        combine(AX, AV[:m], cc)
+        dcc = torch.as_tensor(cc, device=dev)
+        combine(X, V[:m], dcc)
+        combine(AX, AV[:m], dcc)
         R[:k].copy_(AX[:k])
         combine(R, X, -np.diag(e), beta=1.0)
         rn = np.sqrt(np.maximum(np.diag(gram(R[:k], R[:k]).cpu().numpy()), 0.0))
@@ -214,15 +226,16 @@ def davidson(aop, x0, precond, tol=1e-10, max_cycle=100, max_space=12, lindep=1e
         e_prev = e
         x_prev = np.zeros((k, space + nroots))
         x_prev[:, :m] = cc
-        ts = []
-        for i in range(k):
-            if conv[i]:
-                continue
-            t = precond(R[i], e[i], X[i]).reshape(1, -1)
-            nt = float(np.sqrt(max(gram(t, t).cpu().numpy()[0, 0], 0.0)))
-            if nt > 0.0:
-                ts.append(t / nt)
-        new = torch.cat(ts) if ts else X[:0]
+        act = [i for i in range(k) if not conv[i]]
+        if type(precond) is DiagPrecond:
+            t = precond.block([R[i] for i in act], e[act], [X[i] for i in act])
+        else:
+            t = torch.cat([precond(R[i], e[i], X[i]).reshape(1, -1) for i in act])
+        nt = np.sqrt(np.maximum(np.diag(gram(t, t).cpu().numpy()), 0.0))
+        keep = np.flatnonzero(nt > 0.0)
+        if len(keep) < len(act):
+            t = t[torch.as_tensor(keep, device=dev)]
+        new = t / torch.as_tensor(nt[keep], device=dev)[:, None] if len(keep) else X[:0]
         if m + new.shape[0] > space:
             # restart from the Ritz vectors (orthonormal, h diagonal)
             V[:k].copy_(X[:k])

@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from .. import _capi
-from .._runtime import (device, eri_pair_matrix, like_input, ptr, require_cuda, stream, to_dev,
+from .._runtime import (dev_eri_pair_matrix, device, like_input, ptr, require_cuda, stream, to_dev,
                         workspace)
 
 
@@ -262,7 +262,7 @@ def dev_rdm12s(bra, ket, norb, nelec, with_dm2=True):
 # ---------------------------------------------------------------------------
 
 def absorb_h1e(h1e, eri, norb, nelec, fac=1):
-    h2e = dev_absorb_h1e(h1e, eri_pair_matrix(eri, norb), norb, nelec, fac)
+    h2e = dev_absorb_h1e(h1e, dev_eri_pair_matrix(eri, norb), norb, nelec, fac)
     return like_input(h2e, eri)
 
 
@@ -273,13 +273,13 @@ def make_hdiag(h1e, eri, norb, nelec, compress=False):
         h1a, h1b = h1[0], h1[1]
     else:
         h1a = h1b = h1
-    out = dev_make_hdiag(h1a, h1b, eri_pair_matrix(eri, norb), norb, nelec)
+    out = dev_make_hdiag(h1a, h1b, dev_eri_pair_matrix(eri, norb), norb, nelec)
     return like_input(out, h1e)
 
 
 def contract_2e(eri, fcivec, norb, nelec, link_index=None):
     nelec = _unpack_nelec(nelec)
-    h2e = to_dev(eri_pair_matrix(eri, norb))
+    h2e = dev_eri_pair_matrix(eri, norb)
     ci = to_dev(fcivec)
     eta = dev_spin_parity(ci, num_strings(norb, nelec[0])) if nelec[0] == nelec[1] else None
     out = dev_contract_2e(h2e, ci.reshape(-1), norb, nelec, eta=eta)
