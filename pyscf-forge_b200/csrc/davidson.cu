@@ -40,6 +40,72 @@ __global__ void k_combine(int ny, double* y, int64_t ldy, double beta, int nx,
   }
 }
 
+// The same for vectors that give every SM its 8 blocks and more: E elements a
+// thread, so that 8 to 16 values of x are in flight whatever nx is, and RG
+// following ny, so that one row does not pay for the sums of four.  Bound by
+// HBM: 11 million determinants, 12 rows into one (1.23 GB) 320 -> 193 us, 15
+// into 3 435 -> 340 us.  At 226512 elements the form above is faster (12 rows
+// into 2 18 against 19 us): there are not blocks enough to lose any.
+template <int RG, int E>
+__global__ void k_combine_large(int ny, double* y, int64_t ldy, double beta, int nx, const double* __restrict__ x,
+                                int64_t ldx, const double* __restrict__ coef, int64_t n) {
+  extern __shared__ double cs[];  // coef rows padded with zeros to a multiple of RG
+  const int nyp = (ny + RG - 1) / RG * RG;
+  for (int i = threadIdx.x; i < nx * nyp; i += blockDim.x) cs[i] = i < nx * ny ? coef[i] : 0.0;
+  __syncthreads();
+  constexpr int CB_I = 4;
+  constexpr int64_t CH = 256 * E;
+  for (int64_t k0 = blockIdx.x * CH + threadIdx.x; k0 < n; k0 += gridDim.x * CH) {
+    for (int r0 = 0; r0 < ny; r0 += RG) {
+      double acc[RG][E];
+#pragma unroll
+      for (int rr = 0; rr < RG; ++rr)
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const int64_t k = k0 + 256 * e;
+          acc[rr][e] = (r0 + rr < ny && beta != 0.0 && k < n) ? beta * y[(int64_t)(r0 + rr) * ldy + k] : 0.0;
+        }
+      const double* c0 = cs + (int64_t)r0 * nx;
+      int i0 = 0;
+      for (; i0 + CB_I <= nx; i0 += CB_I) {
+        double xv[CB_I][E];
+#pragma unroll
+        for (int i = 0; i < CB_I; ++i)
+#pragma unroll
+          for (int e = 0; e < E; ++e)
+            xv[i][e] = k0 + 256 * e < n ? x[(int64_t)(i0 + i) * ldx + k0 + 256 * e] : 0.0;
+#pragma unroll
+        for (int i = 0; i < CB_I; ++i)
+#pragma unroll
+          for (int rr = 0; rr < RG; ++rr) {
+            const double c = c0[rr * nx + i0 + i];
+#pragma unroll
+            for (int e = 0; e < E; ++e) acc[rr][e] = fma(c, xv[i][e], acc[rr][e]);
+          }
+      }
+#pragma unroll 4
+      for (; i0 < nx; ++i0) {
+        double xv[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+          xv[e] = k0 + 256 * e < n ? x[(int64_t)i0 * ldx + k0 + 256 * e] : 0.0;
+#pragma unroll
+        for (int rr = 0; rr < RG; ++rr)
+#pragma unroll
+          for (int e = 0; e < E; ++e) acc[rr][e] = fma(c0[rr * nx + i0], xv[e], acc[rr][e]);
+      }
+#pragma unroll
+      for (int rr = 0; rr < RG; ++rr)
+        if (r0 + rr < ny)
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const int64_t k = k0 + 256 * e;
+            if (k < n) y[(int64_t)(r0 + rr) * ldy + k] = acc[rr][e];
+          }
+    }
+  }
+}
+
 // 1/(hdiag - (e - shift)) with the magnitude capped at 1e8 (cap value +1e8,
 // as the p-space preconditioner the reference uses through fci.make_precond)
 __device__ __forceinline__ double precond_inv(double h, double e, double shift) {
@@ -131,7 +197,12 @@ int csffci_combine(int ny, double* y, int64_t ldy, double beta, int nx, const do
   size_t sm = (size_t)nx * ((ny + CB_RG - 1) / CB_RG * CB_RG) * sizeof(double);
   {
     ProfScope ps_("k_combine", stream);
-    k_combine<<<grid_for(n, 256, 148 * 8), 256, sm, stream>>>(ny, y, ldy, beta, nx, x, ldx, coef, n);
+    if (n < 148ll * 8 * 256 * 2) {
+      k_combine<<<grid_for(n, 256, 148 * 8), 256, sm, stream>>>(ny, y, ldy, beta, nx, x, ldx, coef, n);
+    } else {
+      auto kern = ny == 1 ? k_combine_large<1, 4> : ny == 2 ? k_combine_large<2, 4> : k_combine_large<CB_RG, 2>;
+      kern<<<grid_for(n, 256 * (ny <= 2 ? 4 : 2), 148 * 8), 256, sm, stream>>>(ny, y, ldy, beta, nx, x, ldx, coef, n);
+    }
   }
   return check_launch("combine");
 }

@@ -20,64 +20,76 @@ namespace csffci {
 // skinny Gram for the Davidson projections: out[i][j] = sum_k X[i][k] Y[j][k]
 // with at most GS_MAXY vectors on one side (the new corrections or the Ritz
 // vectors) and at most GS_MAXX on the other (the subspace).  Each block
-// streams k-chunks of GS_NT*KT elements: the chunk of the narrow side stays
-// in registers while every row of the wide side is read once (coalesced,
-// KT loads per thread), so the kernel moves (nx + ny) * n * 8 bytes and is
-// bound by HBM bandwidth.  Per-warp sums accumulate in shared memory in a
-// fixed order; the block partials are summed over the blocks in a fixed
+// streams k-chunks of GS_NT*GS_KT elements: the chunk of the narrow side stays
+// in registers while the block's rows of the wide side are read once, RB rows
+// at a time (coalesced, RB*GS_KT loads per thread in flight; one row at a time
+// waited for its loads and its warp sum, 1.5 us a row).  The kernel moves
+// (nx + ny) * n * 8 bytes and is bound by that where there are chunks enough
+// for the GPU (11 million elements, 12 rows: 850 -> 186 us, 95%); below, the
+// rows are split over grid.y (36 rows of 226512, the call: 121 -> 30 us).  Per-warp sums accumulate in shared memory
+// in a fixed order; the block partials are summed over the blocks in a fixed
 // order as well, so results are bit-reproducible.
 // ---------------------------------------------------------------------------
-constexpr int GS_NT = 256, GS_MAXX = 64, GS_MAXY = 4;
+constexpr int GS_NT = 256, GS_KT = 8, GS_MAXX = 64, GS_MAXY = 4;
 
-template <int NY, int KT>
-__global__ void __launch_bounds__(GS_NT) k_gram_skinny(int nx, const double* __restrict__ x, int64_t ldx, int ny,
-                                                       const double* __restrict__ y, int64_t ldy, int64_t n,
+template <int NY, int RB>
+__global__ void __launch_bounds__(GS_NT) k_gram_skinny(int nx, int rows, const double* __restrict__ x, int64_t ldx,
+                                                       int ny, const double* __restrict__ y, int64_t ldy, int64_t n,
                                                        double* part) {
   __shared__ double wsum[GS_NT / 32][GS_MAXX][NY];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i0 = blockIdx.y * rows, i1 = min(nx, i0 + rows);
   for (int e = lane; e < GS_MAXX * NY; e += 32) (&wsum[warp][0][0])[e] = 0.0;
   __syncwarp();
-  constexpr int KC = GS_NT * KT;
+  constexpr int KC = GS_NT * GS_KT;
   for (int64_t k0 = (int64_t)blockIdx.x * KC; k0 < n; k0 += (int64_t)gridDim.x * KC) {
-    double yv[NY][KT];
+    double yv[NY][GS_KT];
 #pragma unroll
-    for (int q = 0; q < KT; ++q) {
+    for (int q = 0; q < GS_KT; ++q) {
       const int64_t k = k0 + tid + (int64_t)q * GS_NT;
 #pragma unroll
       for (int j = 0; j < NY; ++j) yv[j][q] = (j < ny && k < n) ? y[(int64_t)j * ldy + k] : 0.0;
     }
-    for (int i = 0; i < nx; ++i) {
-      const double* xi = x + (int64_t)i * ldx;
-      double sj[NY];
+    for (int i = i0; i < i1; i += RB) {
+      double xv[RB][GS_KT];
 #pragma unroll
-      for (int j = 0; j < NY; ++j) sj[j] = 0.0;
+      for (int r = 0; r < RB; ++r)
 #pragma unroll
-      for (int q = 0; q < KT; ++q) {
-        const int64_t k = k0 + tid + (int64_t)q * GS_NT;
-        const double xv = k < n ? xi[k] : 0.0;
+        for (int q = 0; q < GS_KT; ++q) {
+          const int64_t k = k0 + tid + (int64_t)q * GS_NT;
+          xv[r][q] = (i + r < i1 && k < n) ? x[(int64_t)(i + r) * ldx + k] : 0.0;
+        }
+      double sj[RB][NY];
 #pragma unroll
-        for (int j = 0; j < NY; ++j) sj[j] = fma(xv, yv[j][q], sj[j]);
-      }
+      for (int r = 0; r < RB; ++r)
 #pragma unroll
-      for (int j = 0; j < NY; ++j) {
-        double v = sj[j];
+        for (int j = 0; j < NY; ++j) {
+          sj[r][j] = 0.0;
 #pragma unroll
-        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        sj[j] = v;
-      }
+          for (int q = 0; q < GS_KT; ++q) sj[r][j] = fma(xv[r][q], yv[j][q], sj[r][j]);
+        }
+#pragma unroll
+      for (int o = 16; o; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+#pragma unroll
+          for (int j = 0; j < NY; ++j) sj[r][j] += __shfl_xor_sync(0xffffffffu, sj[r][j], o);
       if (lane == 0) {
 #pragma unroll
-        for (int j = 0; j < NY; ++j) wsum[warp][i][j] += sj[j];
+        for (int r = 0; r < RB; ++r)
+          if (i + r < i1)
+#pragma unroll
+            for (int j = 0; j < NY; ++j) wsum[warp][i + r - i0][j] += sj[r][j];
       }
     }
   }
   __syncthreads();
-  for (int e = tid; e < nx * NY; e += GS_NT) {
+  for (int e = tid; e < (i1 - i0) * NY; e += GS_NT) {
     const int i = e / NY, j = e - i * NY;
     double v = 0.0;
 #pragma unroll
     for (int w = 0; w < GS_NT / 32; ++w) v += wsum[w][i][j];
-    part[(int64_t)blockIdx.x * nx * NY + e] = v;
+    part[((int64_t)blockIdx.x * nx + i0) * NY + e] = v;
   }
 }
 
@@ -100,9 +112,8 @@ __global__ void k_gram_skinny_reduce(int nx, int ny, int ystride, int nblk, cons
 
 static int gram_skinny_ystride(int ny) { return ny <= 1 ? 1 : ny <= 2 ? 2 : 4; }
 
-static int gram_skinny_blocks(int64_t n, int ny) {
-  const int kt = ny <= 2 ? 16 : 8;
-  int64_t nb = (n + GS_NT * kt - 1) / (GS_NT * kt);
+static int gram_skinny_blocks(int64_t n) {
+  int64_t nb = (n + GS_NT * GS_KT - 1) / (GS_NT * GS_KT);
   if (nb > 148 * 4) nb = 148 * 4;
   return (int)(nb < 1 ? 1 : nb);
 }
@@ -113,7 +124,7 @@ static bool gram_skinny_fits(int nx, int ny) {
 
 static size_t gram_skinny_workspace(int nx, int ny, int64_t n) {
   if (!(ny <= GS_MAXY && nx <= GS_MAXX)) std::swap(nx, ny);
-  return (size_t)gram_skinny_blocks(n, ny) * nx * gram_skinny_ystride(ny) * sizeof(double);
+  return (size_t)gram_skinny_blocks(n) * nx * gram_skinny_ystride(ny) * sizeof(double);
 }
 
 static int gram_skinny_run(int nx, const double* x, int64_t ldx, int ny, const double* y, int64_t ldy, int64_t n,
@@ -125,16 +136,22 @@ static int gram_skinny_run(int nx, const double* x, int64_t ldx, int ny, const d
     std::swap(ldx, ldy);
     transposed = 1;
   }
-  const int nblk = gram_skinny_blocks(n, ny);
+  const int nblk = gram_skinny_blocks(n);
   const int ys = gram_skinny_ystride(ny);
+  // the rows are split until there are 4 blocks a SM, not below 4 rows (the
+  // narrow side is read again by every group)
+  int groups = (148 * 4 + nblk - 1) / nblk;
+  if (groups > (nx + 3) / 4) groups = (nx + 3) / 4;
+  const int rows = ((nx + groups - 1) / groups + 3) & ~3;
+  const dim3 grid(nblk, (nx + rows - 1) / rows);
   {
     ProfScope ps_("k_gram_skinny", stream);
     if (ys == 1)
-      k_gram_skinny<1, 16><<<nblk, GS_NT, 0, stream>>>(nx, x, ldx, ny, y, ldy, n, part);
+      k_gram_skinny<1, 4><<<grid, GS_NT, 0, stream>>>(nx, rows, x, ldx, ny, y, ldy, n, part);
     else if (ys == 2)
-      k_gram_skinny<2, 16><<<nblk, GS_NT, 0, stream>>>(nx, x, ldx, ny, y, ldy, n, part);
+      k_gram_skinny<2, 4><<<grid, GS_NT, 0, stream>>>(nx, rows, x, ldx, ny, y, ldy, n, part);
     else
-      k_gram_skinny<4, 8><<<nblk, GS_NT, 0, stream>>>(nx, x, ldx, ny, y, ldy, n, part);
+      k_gram_skinny<4, 2><<<grid, GS_NT, 0, stream>>>(nx, rows, x, ldx, ny, y, ldy, n, part);
   }
   int st = check_launch("gram (skinny)");
   if (st) return st;
