@@ -46,14 +46,14 @@ constexpr int MP_NB = 32;    // columns of a tile
 constexpr int MP_DD = 36;    // row stride of D: = 4 (mod 16), conflict-free B fragments
 constexpr int MP_DV = 40;    // row stride of V: = 8 (mod 16), conflict-free 16-byte stores
 constexpr int MP_TS = 33;    // row stride of the link table
+constexpr unsigned MP_LINK = 0x40000000u, MP_OFF = 0x1ffffu;  // table: a link is there; byte offset of its target
 constexpr int MP_POLLS = 1 << 22;
 constexpr long long MP_ROUND = 48ll << 20;  // bytes of c and sigma that a round goes through
-constexpr long long MP_MAX_TILES = 60000;  // tiles of a CTA: the table tag has 16 bits
 
 struct MPArgs {
   const csffci_sigma_job_t* jobs;  // device table (BATCH) ...
   csffci_sigma_job_t job0;         // ... or the one job
-  int njobs, npair;
+  int njobs;
   // The list of tiles is cut into rounds and each round among the CTAs.  In
   // one round a CTA would stay with its own problems, and all of a large
   // table's vectors (20 problems of 12 orbitals: 270 MB) would be in use at
@@ -65,8 +65,9 @@ struct MPArgs {
 
 // PT row tiles in pairs of column tiles, TAIL: 0 none, 1 a 16-row tile, 2 an
 // 8-row tile split over four warps; 12 movers
-template <int KS, int PT, int TAIL, bool BATCH>
+template <int NORB, int PT, int TAIL, bool BATCH>
 struct MPLayout {
+  static constexpr int NP = NORB * (NORB + 1) / 2, KS = (NP + 3) / 4;  // pair rows, k-steps of 4
   static constexpr int NPAIRW = 2 * PT;
   static constexpr int NMMA = NPAIRW + (TAIL ? 4 : 0);
   static constexpr int NMOV = 12;
@@ -83,6 +84,9 @@ struct MPLayout {
   static constexpr int AT = (KS - KR) * (PT + (TAIL ? 1 : 0)) * 64;  // elements of that part of h2e
   static constexpr int REG_LAUNCH = 65536 / NTH / 8 * 8;
   static constexpr int REG_MMA = BATCH && KS <= 20 ? 88 : 104, REG_MOV = 160 - REG_MMA;
+  static constexpr int DR = ROWS > 4 * KS ? ROWS : 4 * KS;  // rows of D
+  static constexpr int DSZ = DR * MP_DD, VSZ = ROWS * MP_DV, TSZ = NP * MP_TS;
+  static_assert(ROWS >= NP, "rows");
   static_assert(NPAIRW % 4 == 0, "equal MMA shares on the four schedulers");
   static_assert(!SPLIT || NMMA * 32 * REG_MMA + NMOV * 32 * REG_MOV <= NTH * REG_LAUNCH, "fits the launch's registers");
 };
@@ -189,15 +193,16 @@ __device__ __forceinline__ int mp_next(MPPos* p, int Nb, int sym) {
 }
 
 // Tiles it0 .. it0 + n - 1 of the CTA: those from tile t0 on of job Q.
-template <int KS, int PT, int TAIL, bool BATCH>
+template <int NORB, int PT, int TAIL, bool BATCH>
 __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, const csffci_sigma_job_t& Q, long long t0,
                                           int it0, int n, int mtid, int lane, int mw) {
-  using L = MPLayout<KS, PT, TAIL, BATCH>;
-  constexpr int NMOV = L::NMOV, MTH = NMOV * 32, RPM = L::RPM;
+  using L = MPLayout<NORB, PT, TAIL, BATCH>;
+  constexpr int NMOV = L::NMOV, MTH = NMOV * 32, RPM = L::RPM, NP = L::NP;
   constexpr int RB = 4, RS = BATCH ? 2 : 4;  // pair rows gathered and scattered together
-  const int npair = g.npair;
-  const int dsz = L::ROWS > 4 * KS ? L::ROWS * MP_DD : 4 * KS * MP_DD, vsz = L::ROWS * MP_DV, tsz = npair * MP_TS;
   bool ok = true;
+  // row i of this warp is pair row mw + i NMOV
+  auto in = [&](int i) { return i < RPM && (i * NMOV + NMOV <= NP || mw + i * NMOV < NP); };
+  const unsigned empty = (unsigned)(g.crow_ld - 1) * 8u;  // no link: the zero behind row Ja of c
   const int Nb = (int)Q.Nb, sym = Q.sym, nlb = Q.nlb, end = it0 + n;
   // what one problem has in constant memory is for a job table kept in shared
   // memory: held in registers it would make the movers spill
@@ -224,14 +229,14 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
   // the table of tile it (each thread takes the entries that it copied)
   auto build = [&](int it) {
     const int ne = min(MP_NB, Nb - ahead.ct * MP_NB) * nlb;
-    const unsigned inv = (1u << 20) / (unsigned)max(nlb, 1) + 1u, tag = (unsigned)(it + 1) << 14;
-    unsigned* const T = S.T + it % 3 * tsz;
+    const unsigned inv = (1u << 20) / (unsigned)max(nlb, 1) + 1u;
+    unsigned* const T = S.T + it % 3 * L::TSZ;
     const uint2* const src = S.lk + (it & 1) * g.lk_ld;
     cp_async_wait_all();
 #pragma unroll 4
     for (int e = mtid; e < ne; e += MTH) {
       const uint2 l = src[e];
-      T[rr_lpair(l) * MP_TS + (int)(((unsigned)e * inv) >> 20)] = l.x | tag | rr_lneg(l);
+      T[rr_lpair(l) * MP_TS + (int)(((unsigned)e * inv) >> 20)] = l.x * 8u | MP_LINK | rr_lneg(l);
     }
   };
   double va[RPM];      // alpha values of the next tile
@@ -250,10 +255,10 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
       const int s = it & 1;
       if (fresh) {
         par ^= 1;
-        uint2* const al = S.al + par * npair;
+        uint2* const al = S.al + par * NP;
         double* const cr = S.crow + par * g.crow_ld;
 #pragma unroll 1
-        for (int r = mtid; r < npair; r += MTH) al[r] = make_uint2(0u, 0u);
+        for (int r = mtid; r < NP; r += MTH) al[r] = make_uint2(0u, 0u);
         const double* const row = ci() + cur.ja * Nb;
 #pragma unroll 1
         for (int i = mtid; i < Nb; i += MTH) cp_async8(&cr[i], &row[i]);
@@ -267,7 +272,7 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
         cp_async_wait_all();
         ws_bar_sync(5, MTH);  // also: the table of this tile is complete
       }
-      const uint2* const al = S.al + par * npair;
+      const uint2* const al = S.al + par * NP + mw;
       const int jend = sym ? cur.ja + 1 : Nb;
       auto load_alpha = [&](int ct) {
         const int j = ct * MP_NB + lane;
@@ -275,37 +280,31 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
         sa = 0u;
 #pragma unroll
         for (int i = 0; i < RPM; ++i) {
-          const int r = mw + i * NMOV;
-          const uint2 a = r < npair ? al[r] : make_uint2(0u, 0u);
+          const uint2 a = in(i) ? al[i * NMOV] : make_uint2(0u, 0u);
           va[i] = (a.y && j < jend) ? __ldg(&src[a.x]) : 0.0;
           sa |= (a.y >> 31) << i;
         }
       };
       if (fresh) load_alpha(cur.ct);
       if (it >= 2 && ok) ok = mp_wait(&S.bar[2 + s], ((it >> 1) & 1) ^ 1);  // D of tile it-2 is consumed
-      const unsigned* const T = S.T + it % 3 * tsz + lane;
-      const unsigned tag = (unsigned)(it + 1) & 0xffffu;
-      const double* const cr = S.crow + par * g.crow_ld;
-      double* const D = S.D + s * dsz + lane;
+      const unsigned* const T = S.T + it % 3 * L::TSZ + mw * MP_TS + lane;
+      const char* const cr = reinterpret_cast<const char*>(S.crow + par * g.crow_ld);
+      double* const D = S.D + s * L::DSZ + mw * MP_DD + lane;
 #pragma unroll
       for (int i0 = 0; i0 < RPM; i0 += RB) {
         unsigned t[RB];
         double vb[RB];
 #pragma unroll
-        for (int k = 0; k < RB; ++k) {
-          const int r = mw + (i0 + k) * NMOV;
-          const bool in = i0 + k < RPM && r < npair;
-          t[k] = in ? T[r * MP_TS] : 0u;
-        }
+        for (int k = 0; k < RB; ++k) t[k] = in(i0 + k) ? T[(i0 + k) * NMOV * MP_TS] : empty;
 #pragma unroll
-        for (int k = 0; k < RB; ++k) vb[k] = ((t[k] >> 14) & 0xffffu) == tag ? cr[t[k] & 0x3fffu] : 0.0;
+        for (int k = 0; k < RB; ++k)
+          vb[k] = i0 + k < RPM ? *reinterpret_cast<const double*>(cr + (t[k] & MP_OFF)) : 0.0;
 #pragma unroll
-        for (int k = 0; k < RB; ++k) {
-          const int r = mw + (i0 + k) * NMOV;
-          if (i0 + k < RPM && r < npair)
-            D[r * MP_DD] = rr_flip(va[i0 + k < RPM ? i0 + k : 0], (sa << (31 - i0 - k)) & 0x80000000u) +
-                           rr_flip(vb[k], t[k] & 0x80000000u);
-        }
+        for (int k = 0; k < RB; ++k)
+          if (in(i0 + k))
+            D[(i0 + k) * NMOV * MP_DD] =
+                rr_flip(va[i0 + k < RPM ? i0 + k : 0], (sa << (31 - i0 - k)) & 0x80000000u) +
+                rr_flip(vb[k], t[k] & 0x80000000u);
       }
       __syncwarp();
       if (lane == 0) mp_arrive(&S.bar[s]);  // this warp's rows of D are there
@@ -323,11 +322,10 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
       // scatter V of the previous tile
       const int s = (it - 1) & 1;
       if (ok) ok = mp_wait(&S.bar[4 + s], ((it - 1) >> 1) & 1);
-      const uint2* const al = S.al + ppar * npair;
-      const unsigned* const T = S.T + (it - 1) % 3 * tsz + lane;
-      const unsigned tag = (unsigned)it & 0xffffu;
-      const double* const V = S.V + s * vsz + lane;
-      double* const orow = out() + pja * Nb;
+      const uint2* const al = S.al + ppar * NP + mw;
+      unsigned* const T = S.T + (it - 1) % 3 * L::TSZ + mw * MP_TS + lane;
+      const double* const V = S.V + s * L::VSZ + mw * MP_DV + lane;
+      char* const orow = reinterpret_cast<char*>(out() + pja * Nb);
       const int j = pct * MP_NB + lane;
       const bool inb = j < (sym ? pja + 1 : Nb), ina = sym ? j < pja : inb;
       double* const ocol = out() + j;
@@ -338,15 +336,16 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
         double v[RS];
 #pragma unroll
         for (int k = 0; k < RS; ++k) {
-          const int r = mw + (i0 + k) * NMOV;
-          const bool in = i0 + k < RPM && r < npair;
-          t[k] = in ? T[r * MP_TS] : 0u;
-          a[k] = in ? al[r] : make_uint2(0u, 0u);
-          v[k] = in ? V[r * MP_DV] : 0.0;
+          const bool is = in(i0 + k);
+          t[k] = is ? T[(i0 + k) * NMOV * MP_TS] : 0u;
+          a[k] = is ? al[(i0 + k) * NMOV] : make_uint2(0u, 0u);
+          v[k] = is ? V[(i0 + k) * NMOV * MP_DV] : 0.0;
         }
 #pragma unroll
         for (int k = 0; k < RS; ++k) {
-          if (inb && ((t[k] >> 14) & 0xffffu) == tag) rr_red(&orow[t[k] & 0x3fffu], rr_flip(v[k], t[k] & 0x80000000u));
+          if (in(i0 + k)) T[(i0 + k) * NMOV * MP_TS] = empty;  // only this warp reads the row
+          if (inb && (t[k] & MP_LINK))
+            rr_red(reinterpret_cast<double*>(orow + (t[k] & MP_OFF)), rr_flip(v[k], t[k] & 0x80000000u));
           if (ina && a[k].y) rr_red(&ocol[a[k].x], rr_flip(v[k], a[k].y & 0x80000000u));
         }
       }
@@ -364,13 +363,12 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
   return ok;
 }
 
-template <int KS, int PT, int TAIL, bool BATCH>
-__global__ void __launch_bounds__(MPLayout<KS, PT, TAIL, BATCH>::NTH, 1) k_sigma_mp(const __grid_constant__ MPArgs g) {
-  using L = MPLayout<KS, PT, TAIL, BATCH>;
-  constexpr int NTH = L::NTH;
+template <int NORB, int PT, int TAIL, bool BATCH>
+__global__ void __launch_bounds__(MPLayout<NORB, PT, TAIL, BATCH>::NTH, 1) k_sigma_mp(const __grid_constant__ MPArgs g) {
+  using L = MPLayout<NORB, PT, TAIL, BATCH>;
+  constexpr int NTH = L::NTH, KS = L::KS, npair = L::NP;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int npair = g.npair;
   MPShared S;
   S.D = (double*)smraw;
   S.V = (double*)(smraw + g.off_v);
@@ -381,12 +379,11 @@ __global__ void __launch_bounds__(MPLayout<KS, PT, TAIL, BATCH>::NTH, 1) k_sigma
   S.al = (uint2*)(smraw + g.off_al);
   S.job = (MPJob*)(smraw + g.off_job);
   S.bar = (unsigned long long*)(smraw + g.off_bar);
-  constexpr int DR = L::ROWS > 4 * KS ? L::ROWS : 4 * KS;
-  constexpr int dsz = DR * MP_DD, vsz = L::ROWS * MP_DV;
   __shared__ long long total_s;
   __shared__ int bad_s;
-  for (int i = tid; i < 2 * dsz; i += NTH) S.D[i] = 0.0;  // rows past npair stay zero
-  for (int i = tid; i < 3 * npair * MP_TS; i += NTH) S.T[i] = 0u;
+  for (int i = tid; i < 2 * L::DSZ; i += NTH) S.D[i] = 0.0;  // rows past npair stay zero
+  for (int i = tid; i < 3 * L::TSZ; i += NTH) S.T[i] = (unsigned)(g.crow_ld - 1) * 8u;
+  if (tid < 2) S.crow[tid * g.crow_ld + g.crow_ld - 1] = 0.0;
   if (tid == 0) {
     total_s = 0;
     bad_s = 0;
@@ -457,7 +454,7 @@ __global__ void __launch_bounds__(MPLayout<KS, PT, TAIL, BATCH>::NTH, 1) k_sigma
           const int s = it & 1;
           const unsigned ph = (it >> 1) & 1;
           if (ok) ok = mp_wait(&S.bar[s], ph);
-          const double* Db = S.D + s * dsz + tq * MP_DD + gq + c0;
+          const double* Db = S.D + s * L::DSZ + tq * MP_DD + gq + c0;
           double acc[2][4];
 #pragma unroll
           for (int t = 0; t < 2; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0;
@@ -487,7 +484,7 @@ __global__ void __launch_bounds__(MPLayout<KS, PT, TAIL, BATCH>::NTH, 1) k_sigma
           __syncwarp();
           if (lane == 0) mp_arrive(&S.bar[2 + s]);  // this warp has read D
           if (it >= 2 && ok) ok = mp_wait(&S.bar[6 + s], ph ^ 1);  // V of tile it-2 is scattered
-          double* const V = S.V + s * vsz + c0 + 2 * tq;
+          double* const V = S.V + s * L::VSZ + c0 + 2 * tq;
           *reinterpret_cast<double2*>(&V[r0 * MP_DV]) = make_double2(acc[0][0], acc[0][1]);
           if (pair || TAIL == 1) *reinterpret_cast<double2*>(&V[r1 * MP_DV]) = make_double2(acc[0][2], acc[0][3]);
           if (pair) {
@@ -512,7 +509,7 @@ __global__ void __launch_bounds__(MPLayout<KS, PT, TAIL, BATCH>::NTH, 1) k_sigma
       for (int jb = mp_find<BATCH>(g, lane, &t0); it < n; ++jb) {
         const csffci_sigma_job_t& Q = BATCH ? g.jobs[jb] : g.job0;
         const int m = BATCH ? (int)min((long long)(n - it), mp_job_tiles(Q) - t0) : n - it;
-        if (m > 0 && !mp_movers<KS, PT, TAIL, BATCH>(g, S, Q, t0, it, m, mw * 32 + lane, lane, mw)) bad_s = 1;
+        if (m > 0 && !mp_movers<NORB, PT, TAIL, BATCH>(g, S, Q, t0, it, m, mw * 32 + lane, lane, mw)) bad_s = 1;
         t0 = 0;
         it += m;
       }
@@ -535,33 +532,32 @@ long long sigma_mp_tiles(const csffci_sigma_job_t& J) {
 
 bool sigma_mp_supported(int norb) { return norb >= 4 && norb <= 13; }
 
-template <int KS, int PT, int TAIL, bool BATCH>
+template <int NORB, int PT, int TAIL, bool BATCH>
 static int mp_launch_as(int norb, MPArgs& g, long long max_nb, int max_nlb, long long max_tiles,
                      long long nelem, cudaStream_t stream) {
-  using L = MPLayout<KS, PT, TAIL, BATCH>;
-  constexpr int DR = L::ROWS > 4 * KS ? L::ROWS : 4 * KS;
+  using L = MPLayout<NORB, PT, TAIL, BATCH>;
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
     off += (bytes + 15) & ~(size_t)15;
     return (unsigned)o;
   };
-  take((size_t)2 * DR * MP_DD * sizeof(double));
-  g.off_v = take((size_t)2 * L::ROWS * MP_DV * sizeof(double));
+  take((size_t)2 * L::DSZ * sizeof(double));
+  g.off_v = take((size_t)2 * L::VSZ * sizeof(double));
   g.off_a = take((size_t)L::AT * sizeof(double));
-  g.off_t = take((size_t)3 * g.npair * MP_TS * sizeof(unsigned));
+  g.off_t = take((size_t)3 * L::TSZ * sizeof(unsigned));
   g.lk_ld = MP_NB * max_nlb;
   g.off_lk = take((size_t)2 * g.lk_ld * sizeof(uint2));
-  g.crow_ld = (int)((max_nb + 1) & ~1ll);
+  g.crow_ld = (int)((max_nb + 2) & ~1ll);  // and a zero behind the row
   g.off_crow = take((size_t)2 * g.crow_ld * sizeof(double));
-  g.off_al = take((size_t)2 * g.npair * sizeof(uint2));
+  g.off_al = take((size_t)2 * L::NP * sizeof(uint2));
   g.off_job = take(sizeof(MPJob));
   g.off_bar = take(8 * sizeof(unsigned long long));
   if (off > 227 * 1024 - 256) {
     set_error("sigma: row-pair tiles exceed shared memory (%zu)", off);
     return CSFFCI_ERR_INVALID;
   }
-  auto kern = k_sigma_mp<KS, PT, TAIL, BATCH>;
+  auto kern = k_sigma_mp<NORB, PT, TAIL, BATCH>;
   if (L::SPLIT) {
     // setmaxnreg re-splits the registers of the launch; with fewer the raise
     // would wait forever
@@ -573,9 +569,7 @@ static int mp_launch_as(int norb, MPArgs& g, long long max_nb, int max_nlb, long
     }
   }
   CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)off));
-  // one CTA per SM; more of them where a share would outgrow the table tags
-  const long long need = (max_tiles + MP_MAX_TILES - 1) / MP_MAX_TILES;
-  const int grid = (int)(max_tiles < 148 ? (max_tiles > 0 ? max_tiles : 1) : need > 148 ? need : 148);
+  const int grid = (int)(max_tiles < 148 ? (max_tiles > 0 ? max_tiles : 1) : 148);  // one CTA per SM
   g.rounds = (int)(nelem * 16 / MP_ROUND + 1);
   if (g.rounds > 256) g.rounds = 256;
   static const char* names[10] = {"k_sigma_mp_n4", "k_sigma_mp_n5", "k_sigma_mp_n6",  "k_sigma_mp_n7",  "k_sigma_mp_n8",
@@ -585,11 +579,11 @@ static int mp_launch_as(int norb, MPArgs& g, long long max_nb, int max_nlb, long
   return check_launch("sigma (pair rows)");
 }
 
-template <int KS, int PT, int TAIL>
+template <int NORB, int PT, int TAIL>
 static int mp_launch(int norb, MPArgs& g, long long max_nb, int max_nlb, long long max_tiles, long long nelem,
                      cudaStream_t stream) {
-  return g.jobs ? mp_launch_as<KS, PT, TAIL, true>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream)
-                : mp_launch_as<KS, PT, TAIL, false>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+  return g.jobs ? mp_launch_as<NORB, PT, TAIL, true>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream)
+                : mp_launch_as<NORB, PT, TAIL, false>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
 }
 
 // max_tiles: tiles of all jobs when every one is live
@@ -601,18 +595,17 @@ int sigma_mp_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, con
   g.jobs = jobs_dev;
   g.job0 = job0;
   g.njobs = jobs_dev ? njobs : 1;
-  g.npair = norb * (norb + 1) / 2;
-  switch (norb) {  // KS = ceil(npair / 4); 10, 15, 21, 28, 36, 45, 55, 66, 78, 91 pair rows
-    case 4: return mp_launch<3, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 5: return mp_launch<4, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+  switch (norb) {  // 10, 15, 21, 28, 36, 45, 55, 66, 78, 91 pair rows
+    case 4: return mp_launch<4, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 5: return mp_launch<5, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
     case 6: return mp_launch<6, 2, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
     case 7: return mp_launch<7, 2, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 8: return mp_launch<9, 2, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 9: return mp_launch<12, 2, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 10: return mp_launch<14, 4, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 11: return mp_launch<17, 4, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 12: return mp_launch<20, 4, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 13: return mp_launch<23, 6, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 8: return mp_launch<8, 2, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 9: return mp_launch<9, 2, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 10: return mp_launch<10, 4, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 11: return mp_launch<11, 4, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 12: return mp_launch<12, 4, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 13: return mp_launch<13, 6, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
     default: break;
   }
   set_error("sigma: no row-pair kernel for norb %d", norb);
