@@ -47,6 +47,7 @@ constexpr int MP_DD = 36;    // row stride of D: = 4 (mod 16), conflict-free B f
 constexpr int MP_DV = 40;    // row stride of V: = 8 (mod 16), conflict-free 16-byte stores
 constexpr int MP_TS = 33;    // row stride of the link table
 constexpr unsigned MP_LINK = 0x40000000u, MP_OFF = 0x1ffffu;  // table: a link is there; byte offset of its target
+constexpr int MP_AL = 8;     // slots of the ring of alpha entries (five are in use)
 constexpr int MP_POLLS = 1 << 22;
 constexpr long long MP_ROUND = 48ll << 20;  // bytes of c and sigma that a round goes through
 
@@ -59,8 +60,8 @@ struct MPArgs {
   // table's vectors (20 problems of 12 orbitals: 270 MB) would be in use at
   // once, their random adds past the L2 cache.
   int rounds;
-  unsigned off_v, off_a, off_t, off_lk, off_crow, off_al, off_job, off_bar;
-  int crow_ld, lk_ld;  // elements between the two row and link buffers
+  unsigned off_v, off_a, off_t, off_crow, off_al, off_job, off_bar;
+  int crow_ld;  // elements between the two row buffers
 };
 
 // PT row tiles in pairs of column tiles, TAIL: 0 none, 1 a 16-row tile, 2 an
@@ -112,17 +113,12 @@ __device__ __forceinline__ long long mp_job_tiles(const csffci_sigma_job_t& J) {
   return J.sym ? mp_tri(J.Na) : J.Na * ((J.Nb + MP_NB - 1) / MP_NB);
 }
 
-// a tile of a job
-struct MPPos {
-  int ja;
-  int ct, nct;  // column tile, column tiles of the row
-};
-
 // what the movers read of a job of a table
 struct MPJob {
   const double* ci;
   double* out;
   const csffci_link_t *link_a, *link_b;
+  int nla, nlb;
 };
 
 struct MPShared {
@@ -130,7 +126,6 @@ struct MPShared {
   double* V;
   double* A;  // k-steps from KR on: [step][row tile][row][4]
   unsigned* T;
-  uint2* lk;  // raw links, two tiles
   double* crow;
   uint2* al;
   MPJob* job;
@@ -163,39 +158,25 @@ __device__ __forceinline__ int mp_find(const MPArgs& g, int lane, long long* t) 
   return 0;
 }
 
-__device__ __forceinline__ int mp_nct(int ja, int Nb, int sym) { return ((sym ? ja + 1 : Nb) + MP_NB - 1) / MP_NB; }
-
-__device__ __forceinline__ MPPos mp_pos(long long t, int Nb, int sym) {
-  MPPos p;
-  if (sym) {
-    long long m = (long long)((sqrt(1.0 + 0.25 * (double)t) - 1.0) * 0.5);
-    while ((MP_NB / 2) * m * (m + 1) > t) --m;
-    while ((MP_NB / 2) * (m + 1) * (m + 2) <= t) ++m;
-    const long long rem = t - (MP_NB / 2) * m * (m + 1);
-    p.ja = (int)(MP_NB * m + rem / (m + 1));
-    p.ct = (int)(rem % (m + 1));
+// Tile *t of a job, whose tiles are listed column tile by column tile: its
+// column tile; *t becomes its row
+__device__ __forceinline__ int mp_column(const csffci_sigma_job_t& Q, long long* t) {
+  int ct = 0;
+  if (Q.sym) {
+    while (*t >= Q.Na - (long long)ct * MP_NB) *t -= Q.Na - (long long)(ct++) * MP_NB;
+    *t += (long long)ct * MP_NB;
   } else {
-    const int nct = (Nb + MP_NB - 1) / MP_NB;
-    p.ja = (int)(t / nct);
-    p.ct = (int)(t - (long long)p.ja * nct);
+    ct = (int)(*t / Q.Na);
+    *t -= ct * Q.Na;
   }
-  p.nct = mp_nct(p.ja, Nb, sym);
-  return p;
+  return ct;
 }
 
-// the next tile of the job; 1 on a new row
-__device__ __forceinline__ int mp_next(MPPos* p, int Nb, int sym) {
-  if (++p->ct < p->nct) return 0;
-  p->ct = 0;
-  ++p->ja;
-  p->nct = mp_nct(p->ja, Nb, sym);
-  return 1;
-}
-
-// Tiles it0 .. it0 + n - 1 of the CTA: those from tile t0 on of job Q.
+// Tiles it0 .. it0 + n - 1 of the CTA: rows ja0, ja0 + 1, ... of column tile ct
+// of job Q.
 template <int NORB, int PT, int TAIL, bool BATCH>
-__device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, const csffci_sigma_job_t& Q, long long t0,
-                                          int it0, int n, int mtid, int lane, int mw) {
+__device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, const csffci_sigma_job_t& Q, int ct,
+                                          int ja0, int it0, int n, int mtid, int lane, int mw) {
   using L = MPLayout<NORB, PT, TAIL, BATCH>;
   constexpr int NMOV = L::NMOV, MTH = NMOV * 32, RPM = L::RPM, NP = L::NP;
   constexpr int RB = 4, RS = BATCH ? 2 : 4;  // pair rows gathered and scattered together
@@ -203,162 +184,127 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
   // row i of this warp is pair row mw + i NMOV
   auto in = [&](int i) { return i < RPM && (i * NMOV + NMOV <= NP || mw + i * NMOV < NP); };
   const unsigned empty = (unsigned)(g.crow_ld - 1) * 8u;  // no link: the zero behind row Ja of c
-  const int Nb = (int)Q.Nb, sym = Q.sym, nlb = Q.nlb, end = it0 + n;
+  const int Nb = (int)Q.Nb, sym = Q.sym, end = it0 + n, first = ja0 - it0;
   // what one problem has in constant memory is for a job table kept in shared
   // memory: held in registers it would make the movers spill
-  if (BATCH) {
-    if (mtid == 0) *S.job = MPJob{Q.ci, sym ? Q.scratch : Q.sigma, Q.link_a, Q.link_b};
-    ws_bar_sync(5, MTH);
-  }
+  if (BATCH && mtid == 0) *S.job = MPJob{Q.ci, sym ? Q.scratch : Q.sigma, Q.link_a, Q.link_b, Q.nla, Q.nlb};
+  for (int i = mtid; i < L::TSZ; i += MTH) S.T[i] = empty;
+  for (int i = mtid; i < MP_AL * NP; i += MTH) S.al[i] = make_uint2(0u, 0u);
+  ws_bar_sync(5, MTH);
   auto ci = [&]() { return BATCH ? S.job->ci : Q.ci; };
   auto out = [&]() { return BATCH ? S.job->out : sym ? Q.scratch : Q.sigma; };
   auto link_a = [&]() { return BATCH ? S.job->link_a : Q.link_a; };
-  auto link_b = [&]() { return BATCH ? S.job->link_b : Q.link_b; };
-  MPPos cur = mp_pos(t0, Nb, sym);
-  // the raw links of the next tile, copied asynchronously: entry e of its
-  // contiguous columns is link e % nlb of column e / nlb
-  MPPos ahead = cur;
-  auto load_links = [&](int it) {
-    const int ne = min(MP_NB, Nb - ahead.ct * MP_NB) * nlb;
-    const csffci_link_t* src = link_b() + ahead.ct * MP_NB * nlb;
-    uint2* const dst = S.lk + (it & 1) * g.lk_ld;
-#pragma unroll 1
-    for (int e = mtid; e < ne; e += MTH) cp_async8(&dst[e], &src[e]);
+  auto nla = [&]() { return BATCH ? S.job->nla : Q.nla; };
+  // row Ja of c of tile it
+  auto load_row = [&](int it) {
+    double* const cr = S.crow + (it & 1) * g.crow_ld;
+    const double* const row = ci() + (first + it) * Nb;
+    for (int i = mtid; i < Nb; i += MTH) cp_async8(&cr[i], &row[i]);
     cp_async_commit();
   };
-  // the table of tile it (each thread takes the entries that it copied)
-  auto build = [&](int it) {
-    const int ne = min(MP_NB, Nb - ahead.ct * MP_NB) * nlb;
+  // the alpha links of tile it: link (if any) of this thread, and its entry
+  // (byte offset of row Ka, sign) by pair row; the ring's slot is empty
+  auto alpha_link = [&](int it) { return rr_link(&link_a()[(first + it) * nla() + mtid]); };
+  auto put_alpha = [&](int it, uint2 e) {
+    S.al[(it & (MP_AL - 1)) * NP + rr_lpair(e)] = make_uint2(e.x * (unsigned)Nb * 8u, 1u | rr_lneg(e));
+  };
+  load_row(it0);
+  for (int i = it0; i < it0 + 2 && i < end; ++i)
+    if (mtid < nla()) put_alpha(i, alpha_link(i));
+  {
+    // the beta links of the column tile: link e % nlb of column e / nlb
+    const int nlb = BATCH ? S.job->nlb : Q.nlb;
+    const int ne = min(MP_NB, Nb - ct * MP_NB) * nlb;
+    const csffci_link_t* const src = (BATCH ? S.job->link_b : Q.link_b) + ct * MP_NB * nlb;
     const unsigned inv = (1u << 20) / (unsigned)max(nlb, 1) + 1u;
-    unsigned* const T = S.T + it % 3 * L::TSZ;
-    const uint2* const src = S.lk + (it & 1) * g.lk_ld;
-    cp_async_wait_all();
-#pragma unroll 4
     for (int e = mtid; e < ne; e += MTH) {
-      const uint2 l = src[e];
-      T[rr_lpair(l) * MP_TS + (int)(((unsigned)e * inv) >> 20)] = l.x * 8u | MP_LINK | rr_lneg(l);
+      const uint2 l = rr_link(&src[e]);
+      S.T[rr_lpair(l) * MP_TS + (int)(((unsigned)e * inv) >> 20)] = l.x * 8u | MP_LINK | rr_lneg(l);
+    }
+  }
+  cp_async_wait_all();
+  ws_bar_sync(5, MTH);
+  unsigned t[RPM];
+#pragma unroll
+  for (int i = 0; i < RPM; ++i) t[i] = in(i) ? S.T[(mw + i * NMOV) * MP_TS + lane] : empty;
+  const int j = ct * MP_NB + lane;
+  double va[RPM];  // alpha values of the next tile
+  unsigned sa;     // their signs
+  auto load_alpha = [&](int it) {
+    const uint2* const al = S.al + (it & (MP_AL - 1)) * NP + mw;
+    const char* const src = reinterpret_cast<const char*>(ci() + j);
+    const bool inj = j < (sym ? first + it + 1 : Nb);
+    sa = 0u;
+#pragma unroll
+    for (int i = 0; i < RPM; ++i) {
+      const uint2 a = in(i) ? al[i * NMOV] : make_uint2(0u, 0u);
+      va[i] = (a.y && inj) ? __ldg(reinterpret_cast<const double*>(src + a.x)) : 0.0;
+      sa |= (a.y >> 31) << i;
     }
   };
-  double va[RPM];      // alpha values of the next tile
-  unsigned sa = 0u;    // their signs
-  int par = 1;
-  int pja = 0, pct = 0, ppar = 0;  // the previous tile, whose V is scattered
-  load_links(it0);
-  build(it0);
-  if (it0 + 1 < end) {
-    mp_next(&ahead, Nb, sym);
-    load_links(it0 + 1);
-  }
-  int fresh = 1;  // a new row starts at the next tile
+  load_alpha(it0);
   for (int it = it0; it <= end; ++it) {
+    uint2 next = make_uint2(0u, 0u);
+    const bool more = it + 2 < end && mtid < nla();
     if (it < end) {
       const int s = it & 1;
-      if (fresh) {
-        par ^= 1;
-        uint2* const al = S.al + par * NP;
-        double* const cr = S.crow + par * g.crow_ld;
-#pragma unroll 1
-        for (int r = mtid; r < NP; r += MTH) al[r] = make_uint2(0u, 0u);
-        const double* const row = ci() + cur.ja * Nb;
-#pragma unroll 1
-        for (int i = mtid; i < Nb; i += MTH) cp_async8(&cr[i], &row[i]);
-        cp_async_commit();
-        ws_bar_sync(5, MTH);
-#pragma unroll 1
-        for (int l = mtid; l < Q.nla; l += MTH) {
-          const uint2 e = rr_link(&link_a()[cur.ja * Q.nla + l]);
-          al[rr_lpair(e)] = make_uint2(e.x * (unsigned)Nb, 1u | rr_lneg(e));
-        }
-        cp_async_wait_all();
-        ws_bar_sync(5, MTH);  // also: the table of this tile is complete
-      }
-      const uint2* const al = S.al + par * NP + mw;
-      const int jend = sym ? cur.ja + 1 : Nb;
-      auto load_alpha = [&](int ct) {
-        const int j = ct * MP_NB + lane;
-        const double* const src = ci() + j;
-        sa = 0u;
-#pragma unroll
-        for (int i = 0; i < RPM; ++i) {
-          const uint2 a = in(i) ? al[i * NMOV] : make_uint2(0u, 0u);
-          va[i] = (a.y && j < jend) ? __ldg(&src[a.x]) : 0.0;
-          sa |= (a.y >> 31) << i;
-        }
-      };
-      if (fresh) load_alpha(cur.ct);
+      if (it + 1 < end) load_row(it + 1);
+      if (more) next = alpha_link(it + 2);
+      for (int r = mtid; r < NP; r += MTH) S.al[((it + 3) & (MP_AL - 1)) * NP + r] = make_uint2(0u, 0u);
       if (it >= 2 && ok) ok = mp_wait(&S.bar[2 + s], ((it >> 1) & 1) ^ 1);  // D of tile it-2 is consumed
-      const unsigned* const T = S.T + it % 3 * L::TSZ + mw * MP_TS + lane;
-      const char* const cr = reinterpret_cast<const char*>(S.crow + par * g.crow_ld);
+      const char* const cr = reinterpret_cast<const char*>(S.crow + s * g.crow_ld);
       double* const D = S.D + s * L::DSZ + mw * MP_DD + lane;
 #pragma unroll
       for (int i0 = 0; i0 < RPM; i0 += RB) {
-        unsigned t[RB];
         double vb[RB];
 #pragma unroll
-        for (int k = 0; k < RB; ++k) t[k] = in(i0 + k) ? T[(i0 + k) * NMOV * MP_TS] : empty;
+        for (int k = 0; k < RB; ++k)
+          vb[k] = i0 + k < RPM ? *reinterpret_cast<const double*>(cr + (t[i0 + k < RPM ? i0 + k : 0] & MP_OFF)) : 0.0;
 #pragma unroll
         for (int k = 0; k < RB; ++k)
-          vb[k] = i0 + k < RPM ? *reinterpret_cast<const double*>(cr + (t[k] & MP_OFF)) : 0.0;
-#pragma unroll
-        for (int k = 0; k < RB; ++k)
-          if (in(i0 + k))
-            D[(i0 + k) * NMOV * MP_DD] =
-                rr_flip(va[i0 + k < RPM ? i0 + k : 0], (sa << (31 - i0 - k)) & 0x80000000u) +
-                rr_flip(vb[k], t[k] & 0x80000000u);
+          if (in(i0 + k)) {
+            const int i = i0 + k < RPM ? i0 + k : 0;
+            D[i * NMOV * MP_DD] =
+                rr_flip(va[i], (sa << (31 - i)) & 0x80000000u) + rr_flip(vb[k], t[i] & 0x80000000u);
+          }
       }
       __syncwarp();
       if (lane == 0) mp_arrive(&S.bar[s]);  // this warp's rows of D are there
-      // the next tile's alpha values (same row), table and links
-      if (it + 1 < end) {
-        if (cur.ct + 1 < cur.nct) load_alpha(cur.ct + 1);
-        build(it + 1);
-        if (it + 2 < end) {
-          mp_next(&ahead, Nb, sym);
-          load_links(it + 2);
-        }
-      }
+      if (it + 1 < end) load_alpha(it + 1);
     }
     if (it > it0) {
       // scatter V of the previous tile
-      const int s = (it - 1) & 1;
+      const int s = (it - 1) & 1, pja = first + it - 1;
       if (ok) ok = mp_wait(&S.bar[4 + s], ((it - 1) >> 1) & 1);
-      const uint2* const al = S.al + ppar * NP + mw;
-      unsigned* const T = S.T + (it - 1) % 3 * L::TSZ + mw * MP_TS + lane;
+      const uint2* const al = S.al + ((it - 1) & (MP_AL - 1)) * NP + mw;
       const double* const V = S.V + s * L::VSZ + mw * MP_DV + lane;
       char* const orow = reinterpret_cast<char*>(out() + pja * Nb);
-      const int j = pct * MP_NB + lane;
+      char* const ocol = reinterpret_cast<char*>(out() + j);
       const bool inb = j < (sym ? pja + 1 : Nb), ina = sym ? j < pja : inb;
-      double* const ocol = out() + j;
 #pragma unroll
       for (int i0 = 0; i0 < RPM; i0 += RS) {
-        unsigned t[RS];
         uint2 a[RS];
         double v[RS];
 #pragma unroll
         for (int k = 0; k < RS; ++k) {
-          const bool is = in(i0 + k);
-          t[k] = is ? T[(i0 + k) * NMOV * MP_TS] : 0u;
-          a[k] = is ? al[(i0 + k) * NMOV] : make_uint2(0u, 0u);
-          v[k] = is ? V[(i0 + k) * NMOV * MP_DV] : 0.0;
+          a[k] = in(i0 + k) ? al[(i0 + k) * NMOV] : make_uint2(0u, 0u);
+          v[k] = in(i0 + k) ? V[(i0 + k) * NMOV * MP_DV] : 0.0;
         }
 #pragma unroll
-        for (int k = 0; k < RS; ++k) {
-          if (in(i0 + k)) T[(i0 + k) * NMOV * MP_TS] = empty;  // only this warp reads the row
-          if (inb && (t[k] & MP_LINK))
-            rr_red(reinterpret_cast<double*>(orow + (t[k] & MP_OFF)), rr_flip(v[k], t[k] & 0x80000000u));
-          if (ina && a[k].y) rr_red(&ocol[a[k].x], rr_flip(v[k], a[k].y & 0x80000000u));
-        }
+        for (int k = 0; k < RS; ++k)
+          if (in(i0 + k)) {
+            const unsigned tt = t[i0 + k < RPM ? i0 + k : 0];
+            if (inb && (tt & MP_LINK))
+              rr_red(reinterpret_cast<double*>(orow + (tt & MP_OFF)), rr_flip(v[k], tt & 0x80000000u));
+            if (ina && a[k].y) rr_red(reinterpret_cast<double*>(ocol + a[k].x), rr_flip(v[k], a[k].y & 0x80000000u));
+          }
       }
       __syncwarp();
       if (lane == 0) mp_arrive(&S.bar[6 + s]);  // V of the previous tile is consumed
     }
-    if (it < end) {
-      pja = cur.ja;
-      pct = cur.ct;
-      ppar = par;
-      fresh = mp_next(&cur, Nb, sym);
-    }
-    ws_bar_sync(5, MTH);  // the table of tile it+1 is complete, that of it-1 is free
+    if (more) put_alpha(it + 2, next);
+    cp_async_wait_all();
+    ws_bar_sync(5, MTH);  // row Ja of tile it+1 and the alpha entries of tile it+2 are there
   }
   return ok;
 }
@@ -374,7 +320,6 @@ __global__ void __launch_bounds__(MPLayout<NORB, PT, TAIL, BATCH>::NTH, 1) k_sig
   S.V = (double*)(smraw + g.off_v);
   S.A = (double*)(smraw + g.off_a);
   S.T = (unsigned*)(smraw + g.off_t);
-  S.lk = (uint2*)(smraw + g.off_lk);
   S.crow = (double*)(smraw + g.off_crow);
   S.al = (uint2*)(smraw + g.off_al);
   S.job = (MPJob*)(smraw + g.off_job);
@@ -382,7 +327,6 @@ __global__ void __launch_bounds__(MPLayout<NORB, PT, TAIL, BATCH>::NTH, 1) k_sig
   __shared__ long long total_s;
   __shared__ int bad_s;
   for (int i = tid; i < 2 * L::DSZ; i += NTH) S.D[i] = 0.0;  // rows past npair stay zero
-  for (int i = tid; i < 3 * L::TSZ; i += NTH) S.T[i] = (unsigned)(g.crow_ld - 1) * 8u;
   if (tid < 2) S.crow[tid * g.crow_ld + g.crow_ld - 1] = 0.0;
   if (tid == 0) {
     total_s = 0;
@@ -508,10 +452,16 @@ __global__ void __launch_bounds__(MPLayout<NORB, PT, TAIL, BATCH>::NTH, 1) k_sig
       if (it == n) continue;
       for (int jb = mp_find<BATCH>(g, lane, &t0); it < n; ++jb) {
         const csffci_sigma_job_t& Q = BATCH ? g.jobs[jb] : g.job0;
-        const int m = BATCH ? (int)min((long long)(n - it), mp_job_tiles(Q) - t0) : n - it;
-        if (m > 0 && !mp_movers<NORB, PT, TAIL, BATCH>(g, S, Q, t0, it, m, mw * 32 + lane, lane, mw)) bad_s = 1;
+        const int end = BATCH ? it + (int)min((long long)(n - it), mp_job_tiles(Q) - t0) : n;
+        if (it == end) continue;
+        int ct = mp_column(Q, &t0);
+        for (; it < end; ++ct) {
+          const int m = min(end - it, (int)(Q.Na - t0));
+          if (!mp_movers<NORB, PT, TAIL, BATCH>(g, S, Q, ct, (int)t0, it, m, mw * 32 + lane, lane, mw)) bad_s = 1;
+          it += m;
+          t0 = Q.sym ? (long long)(ct + 1) * MP_NB : 0;
+        }
         t0 = 0;
-        it += m;
       }
     }
   }
@@ -533,7 +483,7 @@ long long sigma_mp_tiles(const csffci_sigma_job_t& J) {
 bool sigma_mp_supported(int norb) { return norb >= 4 && norb <= 13; }
 
 template <int NORB, int PT, int TAIL, bool BATCH>
-static int mp_launch_as(int norb, MPArgs& g, long long max_nb, int max_nlb, long long max_tiles,
+static int mp_launch_as(int norb, MPArgs& g, long long max_nb, long long max_tiles,
                      long long nelem, cudaStream_t stream) {
   using L = MPLayout<NORB, PT, TAIL, BATCH>;
   size_t off = 0;
@@ -545,12 +495,10 @@ static int mp_launch_as(int norb, MPArgs& g, long long max_nb, int max_nlb, long
   take((size_t)2 * L::DSZ * sizeof(double));
   g.off_v = take((size_t)2 * L::VSZ * sizeof(double));
   g.off_a = take((size_t)L::AT * sizeof(double));
-  g.off_t = take((size_t)3 * L::TSZ * sizeof(unsigned));
-  g.lk_ld = MP_NB * max_nlb;
-  g.off_lk = take((size_t)2 * g.lk_ld * sizeof(uint2));
+  g.off_t = take((size_t)L::TSZ * sizeof(unsigned));
   g.crow_ld = (int)((max_nb + 2) & ~1ll);  // and a zero behind the row
   g.off_crow = take((size_t)2 * g.crow_ld * sizeof(double));
-  g.off_al = take((size_t)2 * L::NP * sizeof(uint2));
+  g.off_al = take((size_t)MP_AL * L::NP * sizeof(uint2));
   g.off_job = take(sizeof(MPJob));
   g.off_bar = take(8 * sizeof(unsigned long long));
   if (off > 227 * 1024 - 256) {
@@ -580,15 +528,15 @@ static int mp_launch_as(int norb, MPArgs& g, long long max_nb, int max_nlb, long
 }
 
 template <int NORB, int PT, int TAIL>
-static int mp_launch(int norb, MPArgs& g, long long max_nb, int max_nlb, long long max_tiles, long long nelem,
+static int mp_launch(int norb, MPArgs& g, long long max_nb, long long max_tiles, long long nelem,
                      cudaStream_t stream) {
-  return g.jobs ? mp_launch_as<NORB, PT, TAIL, true>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream)
-                : mp_launch_as<NORB, PT, TAIL, false>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+  return g.jobs ? mp_launch_as<NORB, PT, TAIL, true>(norb, g, max_nb, max_tiles, nelem, stream)
+                : mp_launch_as<NORB, PT, TAIL, false>(norb, g, max_nb, max_tiles, nelem, stream);
 }
 
 // max_tiles: tiles of all jobs when every one is live
 int sigma_mp_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, const csffci_sigma_job_t& job0,
-                    long long max_nb, int max_nlb, long long max_tiles,
+                    long long max_nb, long long max_tiles,
                      long long nelem, cudaStream_t stream) {
   MPArgs g;
   memset(&g, 0, sizeof(g));
@@ -596,16 +544,16 @@ int sigma_mp_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, con
   g.job0 = job0;
   g.njobs = jobs_dev ? njobs : 1;
   switch (norb) {  // 10, 15, 21, 28, 36, 45, 55, 66, 78, 91 pair rows
-    case 4: return mp_launch<4, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 5: return mp_launch<5, 0, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 6: return mp_launch<6, 2, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 7: return mp_launch<7, 2, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 8: return mp_launch<8, 2, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 9: return mp_launch<9, 2, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 10: return mp_launch<10, 4, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 11: return mp_launch<11, 4, 2>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 12: return mp_launch<12, 4, 1>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
-    case 13: return mp_launch<13, 6, 0>(norb, g, max_nb, max_nlb, max_tiles, nelem, stream);
+    case 4: return mp_launch<4, 0, 1>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 5: return mp_launch<5, 0, 1>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 6: return mp_launch<6, 2, 0>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 7: return mp_launch<7, 2, 0>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 8: return mp_launch<8, 2, 2>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 9: return mp_launch<9, 2, 1>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 10: return mp_launch<10, 4, 0>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 11: return mp_launch<11, 4, 2>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 12: return mp_launch<12, 4, 1>(norb, g, max_nb, max_tiles, nelem, stream);
+    case 13: return mp_launch<13, 6, 0>(norb, g, max_nb, max_tiles, nelem, stream);
     default: break;
   }
   set_error("sigma: no row-pair kernel for norb %d", norb);

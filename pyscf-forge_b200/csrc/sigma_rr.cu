@@ -129,7 +129,7 @@ int sigma_rr_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev,
   if (variant < 0 && !jobs_dev) variant = sigma_rr_single_variant(norb);
   if (variant < 0) variant = rr_default_variant(norb);
   if (variant == RR_VARIANT_WS && sigma_mp_supported(norb))  // the deterministic scatter went above
-    return sigma_mp_launch(norb, njobs, jobs_dev, job0, max_nb, max_nlb,
+    return sigma_mp_launch(norb, njobs, jobs_dev, job0, max_nb,
                            jobs_dev ? mp_tiles : sigma_mp_tiles(job0), nelem, stream);
   if (variant == RR_VARIANT_WS || variant == RR_VARIANT_WS16)
     return sigma_ws_launch(norb, njobs, jobs_dev, job0, total_units, max_nb, max_nla, max_nlb, stream,

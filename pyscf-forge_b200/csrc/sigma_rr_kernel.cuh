@@ -476,7 +476,7 @@ int sigma_wsr_launch(int norb, const csffci_sigma_job_t& job0, long long total_u
 // variant 4 without the deterministic scatter at 4..13 orbitals (sigma_mp.cu)
 bool sigma_mp_supported(int norb);
 int sigma_mp_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, const csffci_sigma_job_t& job0,
-                    long long max_nb, int max_nlb, long long max_tiles, long long nelem, cudaStream_t stream);
+                    long long max_nb, long long max_tiles, long long nelem, cudaStream_t stream);
 long long sigma_mp_tiles(const csffci_sigma_job_t& J);  // host: tiles of a prepared job
 bool rr_variant_valid(int norb, int v);
 // the variants a job table may run: the tile shapes and the warp-specialised kernel
