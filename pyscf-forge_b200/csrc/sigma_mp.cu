@@ -12,26 +12,28 @@
 //     them share a row tile), four more the last 16 (or 8) rows x 8 columns
 //     each, so that every scheduler carries the same number of MMAs.
 //   - The movers work by pair rows, lanes over the 32 columns.  The beta links
-//     of a tile are turned into a table [pair row][column] -> (target, sign)
-//     in shared memory (a column has at most one link per pair row), so that a
-//     row of D = +-c[Ka][J] +- c[Ja][K] is made in registers and stored once:
-//     no zero rows, no read-modify-write, no order between alpha and beta, and
-//     every access of D, V and the table is a row.  k_sigma_ws went link by
-//     link: random rows, four shared accesses a link with bank conflicts.
-//   - The alpha values of the next tile are loaded into registers and its beta
-//     links copied to shared memory a tile ahead; row Ja of c and the alpha
-//     rows' addresses are double-buffered, so that the scatter of the last row
-//     runs behind the gather of the next.
+//     of a column tile become a table [pair row][column] -> (target, sign) (a
+//     column has at most one link per pair row), so that a row of D =
+//     +-c[Ka][J] +- c[Ja][K] is made in registers and stored once: no zero
+//     rows, no read-modify-write, no order between alpha and beta, and every
+//     access of D and V is a row.  k_sigma_ws went link by link: random rows,
+//     four shared accesses a link with bank conflicts.
+//   - The tiles are listed column tile by column tile, so the table is made
+//     once for many rows Ja and each mover keeps its pair rows' entries in
+//     registers.  Row by row it was made for every tile (12 orbitals (6,6)
+//     singlet 265 us a call, now 249; 20 problems of 10 orbitals 0.36 ms, now
+//     0.27).  What a tile brings is row Ja of c, its alpha entries (two tiles
+//     ahead) and its alpha values (in registers, one ahead).
 //   - The shares of the CTAs are tiles, not rows: the small spaces have fewer
 //     rows than the GPU has SMs.
 //
-// What bounds it: a mover's shared-memory accesses depend on one another and
-// take 200 to 400 cycles under the MMA warps' load, so there are 12 movers (4:
-// 478 us at 12 orbitals, 12: 300 us).  12 orbitals (6,6): 470 us, 280 us of it
-// FP64 MMAs at the 37.1 TFLOP/s peak (60%); without its MMAs or without its
-// adds the kernel would still take 90% of that.  Against the fastest kernel
-// before it: 8 orbitals (4,4) singlet 12.4 -> 5.2 us, 12 (6,6) 580 -> 470 us,
-// 13 (7,6) 2595 -> 2020 us.
+// What bounds it: the movers.  Their shared-memory accesses depend on one
+// another and take 200 to 400 cycles under the MMA warps' load, so there are
+// 12 of them (4: 478 us a call at 12 orbitals, 12: 298 us), and after that their
+// issue slots (65% of all in use with a table whose entries carried a tag, now
+// 53%).  12 orbitals (6,6) singlet, kernel: 226 us, the DMMA pipe 74% active
+// (k_sigma_ws 340 us, 46%); 8 orbitals (4,4) singlet 12.4 -> 5 us, 13 (7,6) 2580
+// (k_sigma_rr) -> 1815 us a call.
 //
 // The CTAs (one per SM) take equal, contiguous shares of the tiles of all rows
 // of all live jobs, in rounds (see MPArgs::rounds).
@@ -78,8 +80,8 @@ struct MPLayout {
   // Registers.  With 12 MMA warps the launch has 80 a thread, split again by
   // setmaxnreg; the k-steps from KR on are then read from shared memory.  The
   // movers of a job table hold what for one problem is in constant memory or
-  // in uniform registers: 56 would spill (20 problems of 12 orbitals 8.28 ms),
-  // 72 do not (6.83 ms).  At 13 orbitals shared memory has no room for more.
+  // in uniform registers: 56 spilled (20 problems of 12 orbitals 8.28 ms, in an
+  // earlier form), 72 do not (6.83 ms).  At 13 orbitals shared memory has no room for more.
   static constexpr bool SPLIT = NMMA == 12;
   static constexpr int KR = KS <= 14 ? KS : KS > 20 ? 17 : BATCH ? 12 : 17;
   static constexpr int AT = (KS - KR) * (PT + (TAIL ? 1 : 0)) * 64;  // elements of that part of h2e

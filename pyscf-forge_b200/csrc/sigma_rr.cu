@@ -45,8 +45,7 @@ static bool rr_aligned8(const void* p) { return ((uintptr_t)p & 7u) == 0; }
 // registers, so those sizes have no (16, 4) instance.  The warp-specialised
 // kernels are the default from 4 orbitals on (rr_default_variant);
 // CSFFCI_SIGMA_VARIANT overrides the choice and the batched solver's
-// autotuner picks per orbital count (many small problems of 6, 7 or 10
-// orbitals run a few percent faster with a tile shape or variant 7).
+// autotuner picks per orbital count.
 static const int kVariantShape[RR_NVARIANT][2] = {{16, 4}, {8, 4}, {16, 2}, {8, 2}};
 
 bool rr_variant_valid(int norb, int v) { return v >= 0 && v < RR_NVARIANT && !(v == 0 && norb >= 15); }
@@ -74,12 +73,11 @@ int sigma_rr_single_variant(int norb) {
 
 // Job tables and one problem below 16 orbitals: variant 4 from 4 orbitals on,
 // up to 13 k_sigma_mp, then k_sigma_ws.  Measured on B200, the best of the
-// other kernels -> k_sigma_mp (kernel time, us), one problem: 6 orbitals
-// (3,3) singlet 7.6 -> 4.5, 8 (4,4) singlet 12.4 -> 5.2, 9 (4,4) singlet
-// 17.2 -> 9.1, 11 (6,5) 159 -> 117, 12 (6,6) singlet 340 -> 278, 13 (7,6)
-// 2595 -> 2020; tables of 20 large problems: 10 orbitals 383 -> 403, 11
-// 1650 -> 1435, 12 7440 -> 6830; of 30 small ones: 8 orbitals 25 -> 22, 10
-// 68 -> 62, 12 198 -> 172.  k_sigma_ws against the best tile shape: 14
+// other kernels -> k_sigma_mp (us), one problem, kernel: 6 orbitals (3,3)
+// singlet 7.6 -> 4.5, 8 (4,4) singlet 12.4 -> 5; call: 11 (6,5) 199 -> 121, 12
+// (6,6) singlet 368 -> 249, 13 (7,6) 2600 -> 1840; tables of 20 large problems,
+// kernel: 8 orbitals 38 -> 26, 10 388 -> 271, 11 1695 -> 1083, 12 7430 ->
+// 5280; of 30 small ones: 8 orbitals 25 -> 17, 10 68 -> 45, 12 198 -> 146.  k_sigma_ws against the best tile shape: 14
 // orbitals singlet 7.61 -> 6.31 ms, 15: 31.1 -> 25.8 ms.  The batched
 // solver's autotuner times every variant on its own job tables.
 int rr_default_variant(int norb) {
