@@ -127,8 +127,15 @@ static size_t gram_skinny_workspace(int nx, int ny, int64_t n) {
   return (size_t)gram_skinny_blocks(n) * nx * gram_skinny_ystride(ny) * sizeof(double);
 }
 
+// with one or two narrow vectors half the blocks will do: a workspace of that
+// size is taken too, every block then going over two chunks
+static size_t gram_skinny_least(int nx, int ny, int64_t n) {
+  const int narrow = ny <= GS_MAXY && nx <= GS_MAXX ? ny : nx;
+  return gram_skinny_workspace(nx, ny, narrow <= 2 ? (n + 1) / 2 : n);
+}
+
 static int gram_skinny_run(int nx, const double* x, int64_t ldx, int ny, const double* y, int64_t ldy, int64_t n,
-                           double* out, double* part, cudaStream_t stream) {
+                           double* out, double* part, size_t work_bytes, cudaStream_t stream) {
   int transposed = 0;
   if (!(ny <= GS_MAXY && nx <= GS_MAXX)) {
     std::swap(nx, ny);
@@ -136,8 +143,8 @@ static int gram_skinny_run(int nx, const double* x, int64_t ldx, int ny, const d
     std::swap(ldx, ldy);
     transposed = 1;
   }
-  const int nblk = gram_skinny_blocks(n);
   const int ys = gram_skinny_ystride(ny);
+  const int nblk = (int)std::min<size_t>(gram_skinny_blocks(n), work_bytes / ((size_t)nx * ys * sizeof(double)));
   // the rows are split until there are 4 blocks a SM, not below 4 rows (the
   // narrow side is read again by every group)
   int groups = (148 * 4 + nblk - 1) / nblk;
@@ -576,12 +583,13 @@ int csffci_gram(int nx, const double* x, int64_t ldx, int ny, const double* y, i
                 int64_t n, double* out, void* work, size_t work_bytes, cudaStream_t stream) {
   CSF_REQUIRE(nx >= 0 && ny >= 0 && n >= 0, "gram: bad sizes");
   if (nx == 0 || ny == 0) return CSFFCI_OK;
-  size_t need = csffci_gram_workspace(nx, ny, n);
+  const bool skinny = gram_skinny_fits(nx, ny);
+  size_t need = skinny ? gram_skinny_least(nx, ny, n) : csffci_gram_workspace(nx, ny, n);
   if (work == nullptr || work_bytes < need) {
     set_error("gram: workspace of %zu bytes < %zu required", work_bytes, need);
     return CSFFCI_ERR_MEMORY;
   }
-  if (gram_skinny_fits(nx, ny)) return gram_skinny_run(nx, x, ldx, ny, y, ldy, n, out, (double*)work, stream);
+  if (skinny) return gram_skinny_run(nx, x, ldx, ny, y, ldy, n, out, (double*)work, work_bytes, stream);
   return gram_run(nx, x, ldx, ny, y, ldy, n, out, 0, (double*)work, stream);
 }
 

@@ -32,3 +32,21 @@ def test_combine(n, nx, ny, beta):
     x, y, c = _draw(nx, n + 1)[:, :n], _draw(ny, n), _draw(ny, nx)
     ref, bound = beta * y + c @ x, 2 * (nx + 2) * 2.0 ** -53 * (abs(beta) * y.abs() + c.abs() @ x.abs())
     assert bool(((combine(y.clone(), x, c, beta=beta) - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n", [4097, 70001])
+@pytest.mark.parametrize("nx,ny", [(7, 1), (2, 9)])
+def test_gram_in_half_the_workspace(n, nx, ny):
+    """One or two narrow vectors: half the blocks' worth of workspace is
+    enough, less is refused."""
+    from pyscf_forge_b200 import _capi
+    from pyscf_forge_b200._runtime import ptr, stream
+    x, y = _draw(nx, n), _draw(ny, n)
+    out = torch.empty((nx, ny), dtype=torch.float64, device="cuda")
+    least = -(-n // 4096) * nx * ny * 8
+    work = torch.empty(least, dtype=torch.uint8, device="cuda")
+    args = (nx, ptr(x), n, ny, ptr(y), n, n, ptr(out), ptr(work))
+    _capi.call("csffci_gram", *args, least, stream())
+    assert bool(((out - x @ y.T).abs() <= 2 * n * 2.0 ** -53 * (x.abs() @ y.abs().T)).all())
+    with pytest.raises(_capi.CSFFCIError):
+        _capi.call("csffci_gram", *args, least - 8, stream())
