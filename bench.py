@@ -341,7 +341,13 @@ def run_ours(args, rank_env):
                                       "(register-only m8n8k4 loop, csffci_fp64_peak)",
                          "peak_note": "hbm_gbs %s (MEASURED_PEAKS.json)" % src},
             "clocks": clk.summary()}
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    with_ref = not args.no_cpu_baseline
+    if rank == 0 and world == 1 and with_ref:
+        import gasref
+        if not gasref.available():
+            with_ref = False
+            line["cpu_baseline"] = {"unavailable": "the reference's CPU library (oracle/_ref) is not built here"}
+    if rank == 0 and world == 1 and with_ref:
         # one full reference sigma on the host, on the very vector the timed
         # loop used: the measured CPU baseline, and the check of the timed
         # output against the reference
@@ -368,7 +374,7 @@ def run_ours(args, rank_env):
         line["batched"]["transforms"] = run_batch_transforms()
         line["solves"] = run_solves()
     if rank == 0 and world == 1 and not args.no_c4:
-        line["c4"] = run_c4(ref_check=not args.no_cpu_baseline)
+        line["c4"] = run_c4(ref_check=with_ref)
     if rank == 0 and world == 1 and not args.no_rdm:
         line["transforms"] = run_transforms()
     if rank == 0:
