@@ -48,5 +48,5 @@ def test_gram_in_half_the_workspace(n, nx, ny):
     args = (nx, ptr(x), n, ny, ptr(y), n, n, ptr(out), ptr(work))
     _capi.call("csffci_gram", *args, least, stream())
     assert bool(((out - x @ y.T).abs() <= 2 * n * 2.0 ** -53 * (x.abs() @ y.abs().T)).all())
-    with pytest.raises(_capi.CSFFCIError):
+    with pytest.raises(MemoryError):
         _capi.call("csffci_gram", *args, least - 8, stream())
