@@ -390,19 +390,19 @@ class CSFTransformer:
     # ---- reference-shaped API ------------------------------------------
     def vec_det2csf(self, civec, order='C', normalize=True, return_norm=False):
         """csfstring.py:45-52 / transform_civec_det2csf 341-414."""
-        civec, norm = self._transform(civec, order, normalize, reverse=False)
+        civec, norm = self._transform(civec, order, normalize, reverse=False, want_norm=return_norm)
         if return_norm:
             return civec, norm
         return civec
 
     def vec_csf2det(self, civec, order='C', normalize=True, return_norm=False):
         """csfstring.py:54-60 / transform_civec_csf2det 416-487."""
-        civec, norm = self._transform(civec, order, normalize, reverse=True)
+        civec, norm = self._transform(civec, order, normalize, reverse=True, want_norm=return_norm)
         if return_norm:
             return civec, norm
         return civec
 
-    def _transform(self, arr, order, normalize, reverse):
+    def _transform(self, arr, order, normalize, reverse, want_norm=True):
         vec_on_cols = order.upper() == 'F'
         is_torch = isinstance(arr, torch.Tensor)
         is_list = isinstance(arr, list)
@@ -429,7 +429,9 @@ class CSFTransformer:
         else:
             x = x.reshape(nvec, ncol_in)
         y = self.dev_csf2det(x) if reverse else self.dev_det2csf(x)
-        norm = torch.linalg.norm(y, dim=1)
+        # the norms are a pass over the vectors of their own (29 us each at 14
+        # orbitals, of 300): only for those who use them
+        norm = torch.linalg.norm(y, dim=1) if normalize or want_norm else None
         if normalize:
             if reverse:
                 y = y / norm[:, None]
@@ -440,14 +442,14 @@ class CSFTransformer:
             y = y.T.contiguous()
         if not is_torch:
             y = y.cpu().numpy()
-            norm = norm.cpu().numpy()
+            norm = norm.cpu().numpy() if norm is not None else None
         if is_flat:
             y = y.reshape(-1)
         elif is_list:
             y = list(y)
         elif is_tuple:
             y = tuple(y)
-        if norm.shape[0] == 1:
+        if norm is not None and norm.shape[0] == 1:
             norm = norm[0] if not is_torch else norm[0]
             norm = float(norm)
         return y, norm
