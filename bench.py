@@ -414,11 +414,12 @@ def run_rdm(dmma_peak, cases=None):
         flops = nroots * 2.0 * n * norb ** 4
         out[tag] = {"ms": ms, "determinants": n, "roots": nroots,
                     "gram_tflops": flops / (ms * 1e-3) / 1e12,
-                    "frac_dmma": flops / (ms * 1e-3) / 1e12 / dmma_peak,
+                    "frac_dmma": flops / 4 / (ms * 1e-3) / 1e12 / dmma_peak,
                     "trace_dm1": float(torch.trace(dm1))}
-    out["note"] = ("adjoint = transition-density / RDM kernel: T slabs <J|E_pq|c> built in shared memory, "
-                   "Gram on FP64 DMMA (bra == ket: symmetric half), 1-RDM from the Gram; flops counted "
-                   "as the dense 2*ndet*norb^4")
+    out["note"] = ("adjoint = transition-density / RDM kernel: excitation rows <J|E_pq|c> built and contracted "
+                   "in shared memory on FP64 DMMA, as the symmetric and antisymmetric halves of the pairs "
+                   "and (bra == ket) the upper tiles only: a quarter of the dense 2*ndet*norb^4 that "
+                   "gram_tflops counts; frac_dmma counts the quarter")
     return out
 
 
