@@ -69,6 +69,14 @@ struct RFArgs {
   unsigned char ta[RF_MAXT], tb[RF_MAXT];  // row blocks (ta, ta + 1) x tb
 };
 
+// A link (target; creation and annihilation orbital, sign) by its documented
+// fields alone and in 4-byte loads: csffci_rdm12 takes tables that are aligned
+// like csffci_link_t and whose padding byte holds anything.
+__device__ __forceinline__ uint2 rf_link(const csffci_link_t* p) {
+  const unsigned* const w = reinterpret_cast<const unsigned*>(p);
+  return make_uint2(__ldg(w), __ldg(w + 1));
+}
+
 // A link as the movers use it.  x: offset in crow (bytes) of a beta link, or
 // Ka * Nb of an alpha link; y: offsets of the S (or T) row in bits 0-13 and
 // of the A row in bits 14-27 (elements of a set; the spare row behind the
@@ -79,7 +87,7 @@ __device__ __forceinline__ unsigned rf_pack_rows(const RFArgs& g, uint2 e) {
   unsigned neg = rr_lneg(e);
   int rs, ra = g.rows_e;
   if (g.sa) {
-    rs = rr_lpair(e);
+    rs = pair_index(a, i);
     if (a != i) ra = g.rows_s + rs - max(a, i);
   } else {
     rs = i * g.norb + a;
@@ -100,7 +108,7 @@ __global__ void k_rdm_pack_links(const __grid_constant__ RFArgs g) {
     const long long J = t / ((long long)RF_NB * g.nlb) * RF_NB + jl;
     uint2 p = make_uint2(0u, 0u);  // past the last column: never used
     if (J < g.Nb) {
-      const uint2 e = rr_link(&g.lb[J * g.nlb + m]);
+      const uint2 e = rf_link(&g.lb[J * g.nlb + m]);
       p = make_uint2(e.x * (unsigned)sizeof(double), rf_pack_rows(g, e));
     }
     g.pack[t] = p;
@@ -234,7 +242,7 @@ __device__ __forceinline__ bool rf_movers(const RFArgs& g, unsigned char* smraw,
     cp_async_commit();
     ws_bar_sync(5, MTH);
     for (int l = mtid; l < nla; l += MTH) {
-      const uint2 e = rr_link(&g.la[ja * nla + l]);
+      const uint2 e = rf_link(&g.la[ja * nla + l]);
       const unsigned y = rf_pack_rows(g, e);
       rf[rf_srow(y) / RF_DS] = 1;
       if (rf_arow(y) < g.rows_e * RF_DS) rf[rf_arow(y) / RF_DS] = 1;
