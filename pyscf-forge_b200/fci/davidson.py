@@ -230,7 +230,9 @@ def davidson(aop, x0, precond, tol=1e-10, max_cycle=100, max_space=12, lindep=1e
         if type(precond) is DiagPrecond:
             t = precond.block([R[i] for i in act], e[act], [X[i] for i in act])
         else:
-            t = torch.cat([precond(R[i], e[i], X[i]).reshape(1, -1) for i in act])
+            t = torch.empty((len(act), n), dtype=torch.float64, device=dev)
+            for row, i in enumerate(act):  # each taken at once: the next call may reuse its buffer
+                t[row] = precond(R[i], e[i], X[i]).reshape(n)
         nt = np.sqrt(np.maximum(np.diag(gram(t, t).cpu().numpy()), 0.0))
         keep = np.flatnonzero(nt > 0.0)
         if len(keep) < len(act):
