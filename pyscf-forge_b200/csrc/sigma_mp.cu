@@ -175,14 +175,14 @@ __device__ __forceinline__ int mp_column(const csffci_sigma_job_t& Q, long long*
 }
 
 // Tiles it0 .. it0 + n - 1 of the CTA: rows ja0, ja0 + 1, ... of column tile ct
-// of job Q.
+// of job Q.  ok: false once a wait of this warp has run out (it then waits no
+// more, in later calls either).
 template <int NORB, int PT, int TAIL, bool BATCH>
-__device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, const csffci_sigma_job_t& Q, int ct,
-                                          int ja0, int it0, int n, int mtid, int lane, int mw) {
+__device__ __forceinline__ void mp_movers(const MPArgs& g, const MPShared& S, const csffci_sigma_job_t& Q, int ct,
+                                          int ja0, int it0, int n, int mtid, int lane, int mw, bool& ok) {
   using L = MPLayout<NORB, PT, TAIL, BATCH>;
   constexpr int NMOV = L::NMOV, MTH = NMOV * 32, RPM = L::RPM, NP = L::NP;
   constexpr int RB = 4, RS = BATCH ? 2 : 4;  // pair rows gathered and scattered together
-  bool ok = true;
   // row i of this warp is pair row mw + i NMOV
   auto in = [&](int i) { return i < RPM && (i * NMOV + NMOV <= NP || mw + i * NMOV < NP); };
   const unsigned empty = (unsigned)(g.crow_ld - 1) * 8u;  // no link: the zero behind row Ja of c
@@ -308,7 +308,26 @@ __device__ __forceinline__ bool mp_movers(const MPArgs& g, const MPShared& S, co
     cp_async_wait_all();
     ws_bar_sync(5, MTH);  // row Ja of tile it+1 and the alpha entries of tile it+2 are there
   }
-  return ok;
+}
+
+// A hand-over that never came shows as NaN in every job that this CTA has had
+// tiles of: with two stages in flight the values lost may be those of an
+// earlier job than the one at hand when a wait ran out.  By one warp.
+template <bool BATCH>
+__device__ __forceinline__ void mp_poison(const MPArgs& g, long long total, int lane) {
+  const long long shares = (long long)gridDim.x * g.rounds;
+  for (int r = 0; r < g.rounds; ++r) {
+    const long long q = (long long)r * gridDim.x + blockIdx.x;
+    long long t0 = total * q / shares, n = total * (q + 1) / shares - t0;
+    if (n == 0) continue;
+    for (int jb = mp_find<BATCH>(g, lane, &t0); n > 0; ++jb) {
+      const csffci_sigma_job_t& Q = BATCH ? g.jobs[jb] : g.job0;
+      const long long m = BATCH ? min(n, mp_job_tiles(Q) - t0) : n;
+      if (m > 0 && lane == 0) rr_red(Q.sym ? Q.scratch : Q.sigma, __longlong_as_double(0x7ff8000000000000ll));
+      n -= m;
+      t0 = 0;
+    }
+  }
 }
 
 template <int NORB, int PT, int TAIL, bool BATCH>
@@ -446,6 +465,7 @@ __global__ void __launch_bounds__(MPLayout<NORB, PT, TAIL, BATCH>::NTH, 1) k_sig
   } else {
     if constexpr (L::SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(L::REG_MOV));
     const int mw = warp - L::NMMA;
+    bool ok = true;
     int it = 0;
     for (int r = 0; r < g.rounds; ++r) {
       const long long q = (long long)r * gridDim.x + blockIdx.x;
@@ -459,22 +479,17 @@ __global__ void __launch_bounds__(MPLayout<NORB, PT, TAIL, BATCH>::NTH, 1) k_sig
         int ct = mp_column(Q, &t0);
         for (; it < end; ++ct) {
           const int m = min(end - it, (int)(Q.Na - t0));
-          if (!mp_movers<NORB, PT, TAIL, BATCH>(g, S, Q, ct, (int)t0, it, m, mw * 32 + lane, lane, mw)) bad_s = 1;
+          mp_movers<NORB, PT, TAIL, BATCH>(g, S, Q, ct, (int)t0, it, m, mw * 32 + lane, lane, mw, ok);
           it += m;
           t0 = Q.sym ? (long long)(ct + 1) * MP_NB : 0;
         }
         t0 = 0;
       }
     }
+    if (!ok) bad_s = 1;
   }
   __syncthreads();
-  // a hand-over that never came shows as NaN
-  if (bad_s && warp == 0) {
-    long long t = total * blockIdx.x / shares;
-    const int jb = mp_find<BATCH>(g, lane, &t);
-    const csffci_sigma_job_t& J = BATCH ? g.jobs[jb] : g.job0;
-    if (lane == 0) atomicAdd(J.sym ? J.scratch : J.sigma, __longlong_as_double(0x7ff8000000000000ll));
-  }
+  if (bad_s && warp == 0) mp_poison<BATCH>(g, total, lane);
 }
 
 long long sigma_mp_tiles(const csffci_sigma_job_t& J) {
