@@ -327,6 +327,8 @@ int csffci_spin_ladder(int norb, int neleca, int nelecb, int op, const double* c
  *      csf.py:557; reference twin fci_rdm_gas_plan_make_rdm12s,
  *      fci_rdm_gas.c:2207-2243, assembled as fci_gas.py:724-733) --------- */
 
+/* The size that lets a call take its fastest form.  Small spaces run in less
+ * (the slab form, whose minimum is what is refused below). */
 size_t csffci_rdm12_workspace(int norb, int neleca, int nelecb);
 /* dm1[p][q] = <bra|q+ p|ket>, dm2[p][q][r][s] = <bra|p+ r+ s q|ket>
  * (fci_gas.h:260-268).  dm2 may be NULL (1-RDM only). */

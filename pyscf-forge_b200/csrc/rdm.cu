@@ -8,6 +8,7 @@
 // (conventions of pyscf/lib/mcscf/fci_gas.h:260-268).  The determinant
 // space is processed in slabs that fit the caller's workspace, so D(pq,J)
 // is never materialised for the whole space.
+#include <algorithm>
 #include <utility>
 
 #include "common.cuh"
@@ -597,7 +598,9 @@ size_t csffci_gram_workspace(int nx, int ny, int64_t n) {
   return gram_skinny_fits(nx, ny) ? gram_skinny_workspace(nx, ny, n) : gram_workspace(nx, ny, n);
 }
 
-size_t csffci_rdm12_workspace(int norb, int neleca, int nelecb) {
+// what the slab form needs; every call may come with that much, and takes the
+// fused form only with a workspace that holds it
+static size_t rdm12_slab_workspace(int norb, int neleca, int nelecb) {
   long long ndet = (long long)(host_binom(norb, neleca) * host_binom(norb, nelecb));
   long long n2 = (long long)norb * norb;
   long long S = ndet < (1ll << 18) ? ndet : (1ll << 18);
@@ -608,9 +611,15 @@ size_t csffci_rdm12_workspace(int norb, int neleca, int nelecb) {
   size_t partd = gram_dmma_workspace((int)n2, (int)n2, S);
   size_t part1 = gram_workspace(1, (int)n2, S);
   if (partd > part) part = partd;
-  const size_t slab = t + g + (part > part1 ? part : part1) + 1024;
-  const size_t fused = rdm_fused_workspace(norb, (long long)host_binom(norb, nelecb), nelecb * (norb - nelecb + 1));
-  return slab > fused ? slab : fused;
+  return t + g + (part > part1 ? part : part1) + 1024;
+}
+
+static size_t rdm_fused_bytes(int norb, int nelecb) {
+  return rdm_fused_workspace(norb, (long long)host_binom(norb, nelecb), nelecb * (norb - nelecb + 1));
+}
+
+size_t csffci_rdm12_workspace(int norb, int neleca, int nelecb) {
+  return std::max(rdm12_slab_workspace(norb, neleca, nelecb), rdm_fused_bytes(norb, nelecb));
 }
 
 int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
@@ -621,7 +630,7 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   long long ndet = Na * Nb;
   int n2 = norb * norb;
   int nla = neleca * (norb - neleca + 1), nlb = nelecb * (norb - nelecb + 1);
-  size_t need = csffci_rdm12_workspace(norb, neleca, nelecb);
+  const size_t need = rdm12_slab_workspace(norb, neleca, nelecb);
   if (work == nullptr || work_bytes < need) {
     set_error("rdm12: workspace of %zu bytes < %zu required", work_bytes, need);
     return CSFFCI_ERR_MEMORY;
@@ -629,7 +638,7 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   const bool same = (bra == ket);
   int st;
   RdmFusedJob J = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 3, 3);
-  if (dm2 && ndet > 0 && rdm_fused_fits(J)) {
+  if (dm2 && ndet > 0 && work_bytes >= rdm_fused_bytes(norb, nelecb) && rdm_fused_fits(J)) {
     double* M = rdm_fused_m(work);
     const int ld = rdm_fused_ld(J);
     const int ne = neleca + nelecb;
@@ -693,7 +702,7 @@ static long long rdm12s_slab(long long ndet) {
   return S < 1 ? 1 : S;
 }
 
-size_t csffci_rdm12s_workspace(int norb, int neleca, int nelecb) {
+static size_t rdm12s_slab_workspace(int norb, int neleca, int nelecb) {
   long long ndet = (long long)(host_binom(norb, neleca) * host_binom(norb, nelecb));
   long long n2 = (long long)norb * norb;
   long long S = rdm12s_slab(ndet);
@@ -703,9 +712,11 @@ size_t csffci_rdm12s_workspace(int norb, int neleca, int nelecb) {
   size_t partd = gram_dmma_workspace((int)n2, (int)n2, S);
   size_t part1 = gram_workspace(1, (int)n2, S);
   if (partd > part) part = partd;
-  const size_t slab = t + g + (part > part1 ? part : part1) + 1024;
-  const size_t fused = rdm_fused_workspace(norb, (long long)host_binom(norb, nelecb), nelecb * (norb - nelecb + 1));
-  return slab > fused ? slab : fused;
+  return t + g + (part > part1 ? part : part1) + 1024;
+}
+
+size_t csffci_rdm12s_workspace(int norb, int neleca, int nelecb) {
+  return std::max(rdm12s_slab_workspace(norb, neleca, nelecb), rdm_fused_bytes(norb, nelecb));
 }
 
 int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
@@ -720,7 +731,7 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   long long ndet = Na * Nb;
   int n2 = norb * norb;
   int nla = neleca * (norb - neleca + 1), nlb = nelecb * (norb - nelecb + 1);
-  size_t need = csffci_rdm12s_workspace(norb, neleca, nelecb);
+  const size_t need = rdm12s_slab_workspace(norb, neleca, nelecb);
   if (work == nullptr || work_bytes < need) {
     set_error("rdm12s: workspace of %zu bytes < %zu required", work_bytes, need);
     return CSFFCI_ERR_MEMORY;
@@ -728,7 +739,7 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   const bool same = (bra == ket);
   const bool two = dm2aa != nullptr;
   int st;
-  if (two && ndet > 0) {
+  if (two && ndet > 0 && work_bytes >= rdm_fused_bytes(norb, nelecb)) {
     RdmFusedJob Jaa = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 1, 1);
     RdmFusedJob Jbb = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 2, 2);
     RdmFusedJob Jab = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, false, 1, 2);

@@ -764,7 +764,7 @@ static double* rf_base(void* work) { return (double*)(((uintptr_t)work + 15) & ~
 double* rdm_fused_m(void* work) { return rf_base(work) + (size_t)RF_MAXCTA * RF_MAXT * 128; }
 
 size_t rdm_fused_workspace(int norb, long long Nb, int nlb) {
-  if (norb > 16) return 0;
+  if (norb < 2 || norb > 16) return 0;
   return (size_t)RF_MAXCTA * RF_MAXT * 128 * sizeof(double) + rf_m_bytes(norb) +
          (size_t)(Nb + RF_NB) * nlb * sizeof(uint2) + 256;
 }

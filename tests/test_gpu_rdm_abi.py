@@ -1,6 +1,7 @@
 """csffci_rdm12 and csffci_rdm12s through the C ABI with what a caller other
 than the Python layer may hand over: link tables that are aligned like their
-entries (4 bytes) and whose padding byte was never written."""
+entries (4 bytes) and whose padding byte was never written, and workspaces of the size
+that the slab form alone needs."""
 import numpy as np
 import pytest
 
@@ -57,3 +58,28 @@ def test_link_tables_by_their_documented_fields(norb, nelec, same, pad, offset):
     got = _rdms(norb, nelec, bra, ket, _table(la, pad, offset), _table(lb, pad, offset))
     for x, y in zip(got, want):
         assert np.array_equal(x, y)
+
+
+# bytes that the slab form needs: csffci_rdm12, csffci_rdm12s
+SLAB_BYTES = {(4, 2, 2): (14592, 28160), (6, 3, 3): (252736, 504448), (8, 4, 4): (5216256, 10300416),
+              (16, 1, 0): (1119232, 2237440)}
+
+
+@pytest.mark.parametrize("space", sorted(SLAB_BYTES))
+@pytest.mark.parametrize("same", [True, False])
+def test_workspace_of_the_slab_form(space, same):
+    """The slab form's workspace is taken, with the same densities to the
+    rounding of sums of at most 4900 normalised products; one byte less is
+    refused."""
+    from pyscf_forge_b200.fci import direct_spin1 as D
+    norb, na, nb = space
+    bra, ket = _vectors(norb, na, nb, same, norb + 1)
+    la, lb = (D.dev_link_table(norb, n) for n in (na, nb))
+    least = dict(zip(("csffci_rdm12", "csffci_rdm12s"), SLAB_BYTES[space]))
+    want = _rdms(norb, (na, nb), bra, ket, la, lb)
+    got = _rdms(norb, (na, nb), bra, ket, la, lb, least)
+    for x, y in zip(got, want):
+        assert np.abs(x - y).max() < 1e-12
+    for call in least:
+        with pytest.raises(MemoryError):
+            _rdms(norb, (na, nb), bra, ket, la, lb, dict(least, **{call: least[call] - 1}))
