@@ -574,6 +574,33 @@ static RdmFusedJob fused_job(int norb, int neleca, int nelecb, const csffci_link
   return J;
 }
 
+// Whether the fused kernel takes these Grams (one, or alpha-alpha, beta-beta
+// and alpha-beta), or the slab form does: the shorter of two estimates in
+// microseconds, fitted to both forms at 8 to 16 orbitals and 1 to 260 000
+// determinants (870 calls; the form taken was never more than 1.27 times the
+// other's time).  The fused kernel pays for every pass over the determinants
+// and for whole tiles of 16 columns, the slab form by the element of T and of
+// its 64 x 64 Gram tiles.  Measured, slab form against fused (us), two vectors at 16
+// orbitals: 8960 determinants 106 against 194, 12870 x 1 164 against 1544,
+// 67 200 612 against 509, 218 400 1918 against 1287; one vector at 16 orbitals,
+// 12870 x 1: 101 against 321; at 12 orbitals two vectors of 144: 42 against 53.
+static bool take_fused(const RdmFusedJob* jobs, int njob, bool same) {
+  double fused = same ? 5.0 : 12.0;
+  for (int i = 0; i < njob; ++i) {
+    if (!rdm_fused_fits(jobs[i])) return false;
+    const RdmFusedSize z = rdm_fused_size(jobs[i]);
+    fused += z.passes * ((same ? 19.0 : 24.0) + 0.7 * z.cta_rows) + 0.025 * z.out_tiles * z.cta_tiles;
+  }
+  const double n2 = (double)jobs[0].norb * jobs[0].norb, ndet = (double)jobs[0].Na * jobs[0].Nb;
+  const int t = (int)((n2 + GD_T - 1) / GD_T);
+  double tiles = same ? t * (t + 1) / 2 : t * t;
+  if (njob == 3) tiles = 2 * tiles + t * t;
+  const double more = njob == 3 ? 40.0 : 0.0;
+  const double least = std::min(32.0 + more + 0.06 * ndet * njob, njob == 3 ? 210.0 : 90.0);
+  const double slab = 40.0 + more + (3.3e-4 * tiles + 5.7e-6 * n2 * (same ? 1 : 2) * njob) * ndet;
+  return fused <= std::max(least, slab);
+}
+
 }  // namespace csffci
 
 using namespace csffci;
@@ -638,7 +665,7 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   const bool same = (bra == ket);
   int st;
   RdmFusedJob J = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 3, 3);
-  if (dm2 && ndet > 0 && work_bytes >= rdm_fused_bytes(norb, nelecb) && rdm_fused_fits(J)) {
+  if (dm2 && ndet > 0 && work_bytes >= rdm_fused_bytes(norb, nelecb) && take_fused(&J, 1, same)) {
     double* M = rdm_fused_m(work);
     const int ld = rdm_fused_ld(J);
     const int ne = neleca + nelecb;
@@ -740,11 +767,12 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   const bool two = dm2aa != nullptr;
   int st;
   if (two && ndet > 0 && work_bytes >= rdm_fused_bytes(norb, nelecb)) {
-    RdmFusedJob Jaa = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 1, 1);
-    RdmFusedJob Jbb = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 2, 2);
-    RdmFusedJob Jab = fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, false, 1, 2);
-    Jab.sa = same ? 1 : 0;
-    if (rdm_fused_fits(Jaa) && rdm_fused_fits(Jbb) && rdm_fused_fits(Jab)) {
+    RdmFusedJob J[3] = {fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 1, 1),
+                        fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, same, 2, 2),
+                        fused_job(norb, neleca, nelecb, link_a, link_b, bra, ket, false, 1, 2)};
+    const RdmFusedJob &Jaa = J[0], &Jbb = J[1], &Jab = J[2];
+    J[2].sa = same ? 1 : 0;
+    if (take_fused(J, 3, same)) {
       double* M = rdm_fused_m(work);
       if (same) {
         if ((st = rdm_fused_run(Jaa, work, stream))) return st;

@@ -751,6 +751,22 @@ static int rf_strips(RFTile* t, int n, int a0, int a1, int b0, int b1, bool tri)
 
 constexpr int RF_MAX_ALL = 1200;  // tiles of one Gram: 32 x 64 / 2 and spare
 
+// the output tiles of a Gram, after rf_layout
+static int rf_tiles(const RFArgs& g, RFTile* tiles) {
+  int n = 0;
+  const int bs = g.rows_s / 8, be = g.rows_e / 8, bw = g.setrows / 8;
+  if (g.nsrc == 1) {  // S.S and A.A (or T.T), upper triangles
+    n = rf_strips(tiles, n, 0, bs, 0, bs, true);
+    if (g.sa) n = rf_strips(tiles, n, bs, be, bs, be, true);
+  } else if (g.sa) {  // S1.S2 and A1.A2
+    n = rf_strips(tiles, n, 0, bs, bw, bw + bs, false);
+    n = rf_strips(tiles, n, bs, be, bw + bs, bw + be, false);
+  } else {
+    n = rf_strips(tiles, n, 0, be, bw, bw + be, false);
+  }
+  return n;
+}
+
 // workspace: partial sums, the matrix M with the two flags behind it, the
 // packed links
 static size_t rf_m_bytes(int norb) {
@@ -774,6 +790,18 @@ bool rdm_fused_fits(const RdmFusedJob& j) {
   if (j.norb < 2 || j.norb > 16) return false;
   RFArgs g = rf_args(j);
   return rf_layout(g) != 0;
+}
+
+RdmFusedSize rdm_fused_size(const RdmFusedJob& j) {
+  RFArgs g = rf_args(j);
+  RFTile tiles[RF_MAX_ALL];
+  rf_layout(g);
+  RdmFusedSize s;
+  s.out_tiles = rf_tiles(g, tiles);
+  s.passes = (s.out_tiles + RF_MAXT - 1) / RF_MAXT;
+  s.cta_rows = (g.Na + RF_MAXCTA - 1) / RF_MAXCTA;
+  s.cta_tiles = (g.Na * ((g.Nb + RF_NB - 1) / RF_NB) + RF_MAXCTA - 1) / RF_MAXCTA;
+  return s;
 }
 
 int rdm_fused_rows_s(const RdmFusedJob& j) {
@@ -803,17 +831,7 @@ int rdm_fused_run(const RdmFusedJob& j, void* work, cudaStream_t stream) {
     if ((st = check_launch("rdm pack links"))) return st;
   }
   RFTile tiles[RF_MAX_ALL];
-  const int bs = g.rows_s / 8, be = g.rows_e / 8, bw = g.setrows / 8;
-  int n = 0;
-  if (j.nsrc == 1) {  // S.S and A.A (or T.T), upper triangles
-    n = rf_strips(tiles, n, 0, bs, 0, bs, true);
-    if (g.sa) n = rf_strips(tiles, n, bs, be, bs, be, true);
-  } else if (g.sa) {  // S1.S2 and A1.A2
-    n = rf_strips(tiles, n, 0, bs, bw, bw + bs, false);
-    n = rf_strips(tiles, n, bs, be, bw + bs, bw + be, false);
-  } else {
-    n = rf_strips(tiles, n, 0, be, bw, bw + be, false);
-  }
+  const int n = rf_tiles(g, tiles);
   const long long all = g.Na * nct;
   const int grid = all < RF_MAXCTA ? (int)all : RF_MAXCTA;
   // equal passes of at most RF_MAXT tiles

@@ -21,6 +21,13 @@ struct RdmFusedJob {
 };
 
 bool rdm_fused_fits(const RdmFusedJob& j);
+// what its time depends on: output tiles of the Gram and passes over the
+// determinants that they take, rows Ja and 16-column tiles of a CTA
+struct RdmFusedSize {
+  int out_tiles, passes;
+  long long cta_rows, cta_tiles;
+};
+RdmFusedSize rdm_fused_size(const RdmFusedJob& j);
 // workspace: partial sums, the matrix M with the two flags of rdm_sym_check
 // behind its ld*ld elements, the packed beta links
 size_t rdm_fused_workspace(int norb, long long Nb, int nlb);
