@@ -35,7 +35,8 @@ __device__ __forceinline__ int find_job(const csffci_transform_job_t* jobs, int 
 }
 
 // One task = the CTA task of transform_tile.cuh of one job (one npair block of
-// one problem); pad holds the tile class and the column chunks.
+// one problem); pad holds the tile class, the column chunks and the vectors of
+// a tile.
 __global__ void __launch_bounds__(XF_W * 32, 2) k_transform_batch(const csffci_transform_job_t* jobs, int njobs,
                                                                   int64_t total_tiles, int reverse) {
   __shared__ double red[XF_RED];
@@ -58,10 +59,10 @@ __global__ void __launch_bounds__(XF_W * 32, 2) k_transform_batch(const csffci_t
     B.ndet = J.ndet;
     B.ncsf = J.ncsf;
     B.sign = J.sign;
-    const int cls = J.pad & 7, nchunk = J.pad >> 3;
+    const int cls = J.pad & 7, nchunk = (J.pad >> 3) & 0x3fff, vper = J.pad >> 17;
     const int64_t t = tile - J.tile_begin;
-    if (reverse) xf_run<XF_CSF2DET>(B, nullptr, cls, t, nchunk, lane, warp, red);
-    else xf_run<XF_DET2CSF>(B, nullptr, cls, t, nchunk, lane, warp, red);
+    if (reverse) xf_run<XF_CSF2DET, true>(B, nullptr, cls, t, nchunk, vper, lane, warp, red);
+    else xf_run<XF_DET2CSF, true>(B, nullptr, cls, t, nchunk, vper, lane, warp, red);
   }
 }
 
@@ -155,7 +156,7 @@ int transform_batch_prepare(int reverse, int njobs, csffci_transform_job_t* jobs
     CSF_REQUIRE(J.x && J.y && J.mask && J.umat && J.ncsf > 0 && J.ndet > 0, "transform_batch: job %d incomplete", i);
     J.tile_begin = tiles;
     const XfShape sh = xf_shape(J.nconf, J.nvec, reverse ? J.ndet : J.ncsf, reverse ? J.ncsf : J.ndet);
-    J.pad = sh.cls | sh.nchunk << 3;
+    J.pad = sh.cls | sh.nchunk << 3 | sh.vper << 17;
     tiles += sh.ntask;
   }
   *total_tiles = tiles;

@@ -30,7 +30,7 @@ struct XfBlock {
   const int32_t* sel;
   int64_t csf_off, nconf, sconf, task0;
   double sign;
-  int ndet, ncsf, nspin, npair, cls, nchunk;
+  int ndet, ncsf, nspin, npair, cls, nchunk, vper;
 };
 
 struct XfArgs {
@@ -42,7 +42,9 @@ struct XfArgs {
   XfBlock b[XF_MAXB];
 };
 
-template <int MODE>
+// DEAL: some block's vectors are dealt out (without, one vector of 16 orbitals
+// (5,4) 93 us, with 101: registers)
+template <int MODE, bool DEAL>
 __global__ void __launch_bounds__(XF_W * 32, 2) k_transform(const __grid_constant__ XfArgs g) {
   __shared__ double red[XF_RED];
   __shared__ double kx[MODE == XF_HDIAG ? 256 : 1];
@@ -81,7 +83,7 @@ __global__ void __launch_bounds__(XF_W * 32, 2) k_transform(const __grid_constan
     o.npair = b.npair;
     o.nspin = b.nspin;
     o.sconf = b.sconf;
-    xf_run<MODE>(B, &o, b.cls, task - b.task0, b.nchunk, lane, warp, red);
+    xf_run<MODE, DEAL>(B, &o, b.cls, task - b.task0, b.nchunk, b.vper, lane, warp, red);
   }
 }
 
@@ -104,6 +106,7 @@ constexpr int XF_UP_MAX = 45;     // (doubly, singly) counts of up to 8 upper or
 constexpr int XF_UP_BLOCKS = 12;  // npair blocks
 constexpr int64_t XF_UP_ELEMENTS = 8 << 20;  // 64 MiB: half of the L2
 constexpr int64_t XF_L2_BYTES = 126ll << 20;
+constexpr int64_t XF_TOGETHER = 12 << 20;    // 96 MiB of vectors in a launch
 
 struct XfUp {
   int n, low, nk;  // counts in the table; lower orbitals; blocks with shared tiles (first in XfArgs)
@@ -221,6 +224,21 @@ static int xf_norb(const csffci_block_t* blocks, int nblock) {
   return 0;
 }
 
+// whether the CSF->det launch of these blocks takes the upper-orbital order
+// (*norb: its orbitals): vectors that outgrow the L2, and row tiles for all
+// warps, since the order does not deal the vectors out (10 orbitals, 256
+// vectors: 670 us, in block order 220)
+static bool xf_upper(const csffci_block_t* blocks, int nblock, int nvec, int* norb) {
+  int64_t ndet = 0, rows = 0;
+  for (int b = 0; b < nblock; ++b) {
+    ndet += blocks[b].nconf * blocks[b].ndet;
+    rows += (blocks[b].nconf + 15) / 16;
+  }
+  if (ndet * nvec < XF_UP_ELEMENTS || nblock > XF_UP_BLOCKS || rows < XF_WARPS) return false;
+  *norb = xf_norb(blocks, nblock);
+  return *norb >= 8 && *norb <= 16;
+}
+
 // the table of a launch whose blocks nk.. are in the upper-orbital order
 static void xf_up(XfUp& up, const XfArgs& g) {
   const int nh = g.norb / 2;
@@ -269,11 +287,8 @@ static int run_blocks(int nvec, const double* x, int64_t ldx, double* y, int64_t
     bi = nblock - b0 < XF_MAXB ? nblock : b0 + XF_MAXB;
     int64_t ndet = 0;
     for (int b = b0; b < bi; ++b) ndet += blocks[b].nconf * blocks[b].ndet;
-    bool upper = false;
-    if (MODE == XF_CSF2DET && ndet * nvec >= XF_UP_ELEMENTS && bi - b0 <= XF_UP_BLOCKS) {
-      g.norb = xf_norb(blocks + b0, bi - b0);
-      upper = g.norb >= 8 && g.norb <= 16;
-    }
+    bool deal = false;
+    const bool upper = MODE == XF_CSF2DET && xf_upper(blocks + b0, bi - b0, nvec, &g.norb);
     for (int pass = 0; pass < 2; ++pass)  // tiles shared by a CTA first
       for (int b = b0; b < bi; ++b) {
         const csffci_block_t& S = blocks[b];
@@ -307,6 +322,8 @@ static int run_blocks(int nvec, const double* x, int64_t ldx, double* y, int64_t
         d.npair = S.npair;
         d.cls = sh.cls;
         d.nchunk = sh.nchunk;
+        d.vper = sh.vper;
+        deal = deal || (sh.cls < 4 && sh.vper < nvec);
         d.task0 = g.ntask;
         g.ntask += sh.ntask;
       }
@@ -323,7 +340,8 @@ static int run_blocks(int nvec, const double* x, int64_t ldx, double* y, int64_t
       k_csf2det_up<<<grid_for(tasks, 1, 148 * ctas), XF_W * 32, 0, stream>>>(g, up);
     } else {
       ProfScope ps_(name, stream);
-      k_transform<MODE><<<grid_for(g.ntask, 1, 148 * 2), XF_W * 32, 0, stream>>>(g);
+      auto kern = MODE != XF_HDIAG && deal ? k_transform<MODE, MODE != XF_HDIAG> : k_transform<MODE, false>;
+      kern<<<grid_for(g.ntask, 1, 148 * 2), XF_W * 32, 0, stream>>>(g);
     }
     const int st = check_launch("det/csf transform");
     if (st) return st;
@@ -430,18 +448,31 @@ int csffci_csf2det(int nvec, const double* x_csf, int64_t ld_csf, double* x_det,
     int st = check_launch("csf2det zero");
     if (st) return st;
   }
-  // a vector larger than the L2 at a time: with several, the sectors of one are
-  // evicted half written while the others' are (CAS(16,16), 4 vectors: 15.9 ms
-  // together, 13.5 ms one by one)
+  // How many vectors in a launch.  A sector is shared by several blocks, and one
+  // that leaves the L2 before it is complete costs a read and a second write:
+  // a vector larger than the L2 goes by itself (CAS(16,16), 4 vectors: 15.9 ms
+  // together, 13.5 ms one by one), many smaller ones in launches of 64 to 96
+  // MiB (12 orbitals (8,4), 64 vectors: 422 -> 160 us; 14 (10,4), 64: 1.68 ->
+  // 0.92 ms; 18 (15,3), 32: 0.53 -> 0.31 ms).  Up to 192 MiB in the
+  // upper-orbital order few vectors are faster together (12 (6,6), 16 vectors:
+  // 160 us against 186 in halves).
+  int64_t chunk = nvec;
+  const int64_t all = ndet * nvec;
+  int norb;
   if (ndet * (int64_t)sizeof(double) > XF_L2_BYTES) {
-    for (int v = 0; v < nvec; ++v) {
-      const int st = run_blocks<XF_CSF2DET>(1, x_csf + v * ld_csf, ld_csf, x_det + v * ld_det, ld_det, csd_mask, blocks,
-                                            nblock, stream);
-      if (st) return st;
-    }
-    return CSFFCI_OK;
+    chunk = 1;
+  } else if (ndet < XF_UP_ELEMENTS && all > XF_TOGETHER &&
+             (nvec > 32 || all > 2 * XF_TOGETHER || !xf_upper(blocks, nblock, nvec, &norb))) {
+    const int64_t most = (8 * ndet <= XF_UP_ELEMENTS ? XF_UP_ELEMENTS : XF_TOGETHER) / ndet;
+    const int64_t launches = (nvec + most - 1) / most;
+    chunk = (nvec + launches - 1) / launches;
   }
-  return run_blocks<XF_CSF2DET>(nvec, x_csf, ld_csf, x_det, ld_det, csd_mask, blocks, nblock, stream);
+  for (int64_t v = 0; v < nvec; v += chunk) {
+    const int st = run_blocks<XF_CSF2DET>((int)(nvec - v < chunk ? nvec - v : chunk), x_csf + v * ld_csf, ld_csf,
+                                          x_det + v * ld_det, ld_det, csd_mask, blocks, nblock, stream);
+    if (st) return st;
+  }
+  return CSFFCI_OK;
 }
 
 int csffci_hdiag_csf(int norb, int neleca, int nelecb, const double* hdiag_det, const double* eri,

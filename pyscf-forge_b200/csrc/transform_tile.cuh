@@ -50,6 +50,7 @@ struct XfOrb {
 // x kcols column tiles of a CTA with K split over its warps.
 struct XfShape {
   int cls, nchunk;  // class, column chunks
+  int vper;         // vectors of a warp's tile (classes below 4)
   int64_t ntask;    // CTA tasks
 };
 
@@ -58,10 +59,22 @@ __host__ __device__ inline int xf_cols(int cls) {
   return cls == 0 || cls == 4 ? 1 : cls == 1 || cls == 5 ? 2 : cls == 3 ? 8 : 4;
 }
 
+constexpr int XF_WARPS = 148 * 2 * XF_W;  // of two CTAs an SM
+constexpr int XF_VMAX = (1 << 14) - 1;  // vectors of a tile, as job tables hold it
+
+inline int xf_vper(int64_t warps, int nvec) {
+  const int64_t groups = warps > 0 && warps < XF_WARPS ? (XF_WARPS + warps - 1) / warps : 1;
+  const int64_t per = (nvec + groups - 1) / groups;
+  return (int)(per < 1 ? 1 : per > XF_VMAX ? XF_VMAX : per);
+}
+
 // nconf configurations of nvec vectors, N columns, K terms.  Up to 16 columns
 // two row tiles a warp (the gathers of 32 rows in flight hide the latency of
-// the few k-steps), else one row tile x 32 or 64 columns.  Where that gives
-// fewer than four warps per SM and K is long, a CTA shares one tile: columns
+// the few k-steps), else one row tile x 32 or 64 columns.  A tile goes over
+// the vectors one by one; where the tiles are fewer than XF_WARPS, the vectors
+// are dealt out among the warps (256 vectors of a 7-orbital space one after
+// another took 660 us, now 20).  Where the tiles make
+// fewer than four warps an SM and K is long, a CTA shares one tile: columns
 // are then cut until the tiles cover the SMs twice.
 inline XfShape xf_shape(int64_t nconf, int nvec, int N, int K) {
   XfShape s;
@@ -70,7 +83,8 @@ inline XfShape xf_shape(int64_t nconf, int nvec, int N, int K) {
   s.cls = nt <= 1 ? 0 : nt <= 2 ? 1 : nt <= 4 ? 2 : 3;
   s.nchunk = (nt + xf_cols(s.cls) - 1) / xf_cols(s.cls);
   const int64_t warps = (mt + xf_rows(s.cls) - 1) / xf_rows(s.cls) * s.nchunk;
-  s.ntask = (warps + XF_W - 1) / XF_W;
+  s.vper = xf_vper(warps, nvec);
+  s.ntask = (warps * ((nvec + s.vper - 1) / s.vper) + XF_W - 1) / XF_W;
   if (warps < 148 * 4 && K >= 64) {
     const int64_t ms = (nconf * nvec + 15) / 16;
     for (s.cls = 6; s.cls > 4 && ms * ((nt + xf_cols(s.cls) - 1) / xf_cols(s.cls)) < 2 * 148; --s.cls) {
@@ -119,30 +133,32 @@ __device__ __forceinline__ void xf_bfrag(const XfTile& B, const double* u, int n
   }
 }
 
-// One vector: acc[R][NT] += the rows' products over k in [k0, k1).  mo: offset
-// of a row in the block's mask (det->CSF), co: of its CSFs in x (CSF->det).
+// determinants of the rows at step kb (det->CSF and diagonal)
+template <int R>
+__device__ __forceinline__ void xf_load_mask(const XfTile& B, const uint32_t (&mo)[R][2], int kb, int k1, int tq,
+                                             uint32_t (&d)[R][2][4]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int k = kb + tq + 4 * j;
+        d[r][h][j] = k < k1 ? B.mask[mo[r][h] + k] : 0u;
+      }
+}
+
+// One vector: acc[R][NT] += the rows' products over k in [0, k1).  mo: offset
+// of a row in the block's mask and d: its determinants at the first step, left
+// so if more vectors follow (det->CSF), co: of its CSFs in x (CSF->det).
 template <int MODE, int R, int NT>
 __device__ __forceinline__ void xf_accumulate(const XfTile& B, const double* __restrict__ x, const uint32_t (&mo)[R][2],
-                                              const uint32_t (&co)[R][2], int n0, int k0, int k1, int lane,
-                                              double (&acc)[R][NT][4]) {
+                                              const uint32_t (&co)[R][2], int n0, int k1, bool more, int lane,
+                                              uint32_t (&d)[R][2][4], double (&acc)[R][NT][4]) {
   const int gq = lane >> 2, tq = lane & 3;
   const int N = MODE == XF_CSF2DET ? B.ndet : B.ncsf;
-  const uint32_t* __restrict__ mask = B.mask;
   const double* __restrict__ u = B.u;
-  uint32_t d[R][2][4];
-  auto load_mask = [&](int kb) {
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int k = kb + tq + 4 * j;
-          d[r][h][j] = k < k1 ? mask[mo[r][h] + k] : 0u;
-        }
-  };
-  if (MODE != XF_CSF2DET) load_mask(k0);
-  for (int kb = k0; kb < k1; kb += 16) {
+  for (int kb = 0; kb < k1; kb += 16) {
     double a[R][2][4];
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -153,7 +169,8 @@ __device__ __forceinline__ void xf_accumulate(const XfTile& B, const double* __r
           const int k = kb + tq + 4 * j;
           a[r][h][j] = k >= k1 ? 0.0 : MODE == XF_CSF2DET ? x[co[r][h] + k] : __ldcg(x + d[r][h][j]);
         }
-    if (MODE != XF_CSF2DET && kb + 16 < k1) load_mask(kb + 16);
+    if (MODE != XF_CSF2DET && k1 > 16 && (kb + 16 < k1 || more))
+      xf_load_mask<R>(B, mo, kb + 16 < k1 ? kb + 16 : 0, k1, tq, d);
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
       double b[4];
@@ -232,14 +249,17 @@ __device__ __forceinline__ void xf_rows_tile(const XfTile& B, const XfOrb* orb, 
             d[r][h][t][i] = n < N ? B.mask[mo[r][h] + n] : 0u;
           }
   }
+  uint32_t dk[R][2][4];
+  if (MODE == XF_DET2CSF) xf_load_mask<R>(B, mo, 0, K, tq, dk);
   for (int v = 0; v < B.nvec; ++v) {
+    if (MODE == XF_HDIAG) xf_load_mask<R>(B, mo, 0, K, tq, dk);  // one vector
     double acc[R][NT][4];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int t = 0; t < NT; ++t) acc[r][t][0] = acc[r][t][1] = acc[r][t][2] = acc[r][t][3] = 0.0;
     const double* const x = B.x + v * B.ldx + (MODE == XF_CSF2DET ? B.csf_off : 0);
-    xf_accumulate<MODE, R, NT>(B, x, mo, co, n0, 0, K, lane, acc);
+    xf_accumulate<MODE, R, NT>(B, x, mo, co, n0, K, MODE == XF_DET2CSF && v + 1 < B.nvec, lane, dk, acc);
     if (MODE == XF_HDIAG && orb->nspin >= 2) xf_exchange<R, NT>(B, *orb, cf, n0, lane, acc);
     double* const y = B.y + v * B.ldy + (MODE == XF_CSF2DET ? 0 : B.csf_off);
 #pragma unroll
@@ -257,6 +277,13 @@ __device__ __forceinline__ void xf_rows_tile(const XfTile& B, const XfOrb* orb, 
           }
       }
   }
+}
+
+// vectors v0 to v0 + n - 1 of a block alone
+__device__ __forceinline__ void xf_vectors(XfTile& B, int v0, int n) {
+  B.x += v0 * B.ldx;
+  B.y += v0 * B.ldy;
+  B.nvec = n;
 }
 
 // the w-th warp tile of a block in configuration order
@@ -348,10 +375,19 @@ __device__ __forceinline__ void xf_shared(const XfTile& B, const XfOrb* orb, int
   }
 }
 
-template <int MODE>
-__device__ __forceinline__ void xf_run(const XfTile& B, const XfOrb* orb, int cls, int64_t task, int nchunk, int lane,
-                                       int warp, double* red) {
-  const int64_t w = task * XF_W + warp;
+// A CTA task.  DEAL: B's vectors may be dealt out among the warps, group by
+// group (B is changed to those of the group)
+template <int MODE, bool DEAL>
+__device__ __forceinline__ void xf_run(XfTile& B, const XfOrb* orb, int cls, int64_t task, int nchunk, int vper,
+                                       int lane, int warp, double* red) {
+  int64_t w = task * XF_W + warp;
+  if (DEAL && cls < 4 && B.nvec > vper) {
+    const int rows = 16 * xf_rows(cls);
+    const int64_t n = (B.nconf + rows - 1) / rows * nchunk, q = w / n;
+    if (q * vper >= B.nvec) return;
+    w -= q * n;
+    xf_vectors(B, (int)q * vper, min(vper, B.nvec - (int)q * vper));
+  }
   switch (cls) {
     case 0: return xf_warp<MODE, 2, 1>(B, orb, w, nchunk, lane);
     case 1: return xf_warp<MODE, 2, 2>(B, orb, w, nchunk, lane);

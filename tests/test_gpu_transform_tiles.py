@@ -74,3 +74,54 @@ def test_diagonal(norb, na, nb, smult):
     sol = P.csf_solver(None, smult=smult)
     hd = sol.make_hdiag_csf(h1, eri, norb, (na, nb))
     assert np.abs(hd - R.make_hdiag_csf(h1, eri, norb, (na, nb), smult)).max() < 1e-11
+
+
+# vectors dealt out among the warps, K split over a CTA, launches of some of
+# the vectors, the upper-orbital order and blocks without CSFs
+MANY = [(6, 3, 3, 1, 256), (7, 4, 3, 4, 17), (8, 4, 4, 3, 64), (10, 5, 5, 1, 140), (11, 8, 3, 6, 33), (12, 8, 4, 9, 40),
+        (13, 7, 6, 2, 9), (12, 6, 6, 3, 15), (18, 3, 15, 17, 20)]
+
+
+@pytest.mark.parametrize("norb,na,nb,smult,nvec", MANY)
+def test_many_vectors_as_one_by_one(norb, na, nb, smult, nvec):
+    """A vector's coefficients do not depend on those beside it, to the bit."""
+    import torch
+    from pyscf_forge_b200.csf_fci.csfstring import CSFTransformer
+    t = CSFTransformer(norb, na, nb, smult)
+    g = torch.Generator(device="cuda").manual_seed(nvec)
+    x = torch.randn((nvec, t.ncsf), generator=g, dtype=torch.float64, device="cuda")
+    d = torch.randn((nvec, t.ndet), generator=g, dtype=torch.float64, device="cuda")
+    det, csf = t.dev_csf2det(x), t.dev_det2csf(d)
+    for v in range(nvec):
+        assert torch.equal(det[v], t.dev_csf2det(x[v:v + 1])[0])
+        assert torch.equal(csf[v], t.dev_det2csf(d[v:v + 1])[0])
+
+
+def _us(call):
+    """Device time of one call, microseconds (the least of five)."""
+    import torch
+    call()
+    best = float("inf")
+    for _ in range(5):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        torch.cuda.synchronize()
+        e[0].record()
+        for _ in range(10):
+            call()
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]) * 100)
+    return best
+
+
+@pytest.mark.parametrize("norb,na,nb,smult", [(6, 3, 3, 3), (7, 4, 3, 4), (10, 3, 3, 3)])
+def test_many_vectors_fill_the_gpu(norb, na, nb, smult):
+    """256 vectors of a space far too small for the GPU cost a few times one,
+    not the vectors one after another (25 to 30 times)."""
+    import torch
+    from pyscf_forge_b200.csf_fci.csfstring import CSFTransformer
+    t = CSFTransformer(norb, na, nb, smult)
+    x = torch.zeros((256, t.ncsf), dtype=torch.float64, device="cuda")
+    d = torch.zeros((256, t.ndet), dtype=torch.float64, device="cuda")
+    assert _us(lambda: t.dev_csf2det(x)) < 8 * _us(lambda: t.dev_csf2det(x[:1]))
+    assert _us(lambda: t.dev_det2csf(d)) < 8 * _us(lambda: t.dev_det2csf(d[:1]))
