@@ -270,7 +270,7 @@ static void xf_up(XfUp& up, const XfArgs& g) {
 
 template <int MODE>
 static int run_blocks(int nvec, const double* x, int64_t ldx, double* y, int64_t ldy, const uint32_t* mask,
-                      const csffci_block_t* blocks, int nblock, cudaStream_t stream, int norb = 0,
+                      const csffci_block_t* blocks, int nblock, cudaStream_t stream, bool zeroed, int norb = 0,
                       const double* eri = nullptr) {
   int bi = 0;
   while (bi < nblock) {  // one launch unless a caller lists more than XF_MAXB blocks
@@ -293,9 +293,9 @@ static int run_blocks(int nvec, const double* x, int64_t ldx, double* y, int64_t
       for (int b = b0; b < bi; ++b) {
         const csffci_block_t& S = blocks[b];
         if (S.nconf == 0 || S.ndet == 0) continue;
-        // CSF -> det writes the zeros of a block without CSFs as well, but
-        // where a selection is in force the caller has zeroed everything
-        if (S.ncsf == 0 && (MODE != XF_CSF2DET || S.conf_sel != nullptr)) continue;
+        // CSF -> det writes the zeros of a block without CSFs as well, unless
+        // everything has been zeroed
+        if (S.ncsf == 0 && (MODE != XF_CSF2DET || zeroed)) continue;
         CSF_REQUIRE(S.umat != nullptr || S.ncsf == 0, "transform: block %d has no umat", b);
         CSF_REQUIRE(MODE != XF_HDIAG || S.nspin < 2 || S.zmat != nullptr, "hdiag_csf: block %d has no zmat", b);
         XfShape sh = xf_shape(S.nconf, nvec, MODE == XF_CSF2DET ? S.ndet : S.ncsf,
@@ -425,7 +425,7 @@ int csffci_det2csf(int nvec, const double* x_det, int64_t ld_det, double* x_csf,
   CSF_REQUIRE(nvec >= 0 && blocks != nullptr && nblock >= 0, "det2csf: bad arguments");
   if (nvec == 0) return CSFFCI_OK;
   return run_blocks<XF_DET2CSF>(nvec, x_det, ld_det, x_csf, ld_csf, csd_mask, blocks, nblock,
-                                  stream);
+                                  stream, false);
 }
 
 int csffci_csf2det(int nvec, const double* x_csf, int64_t ld_csf, double* x_det, int64_t ld_det,
@@ -433,13 +433,20 @@ int csffci_csf2det(int nvec, const double* x_csf, int64_t ld_csf, double* x_det,
                    int nblock, cudaStream_t stream) {
   CSF_REQUIRE(nvec >= 0 && blocks != nullptr && nblock >= 0, "csf2det: bad arguments");
   if (nvec == 0) return CSFFCI_OK;
-  // determinants outside a selection start from zero; those of a block
-  // without CSFs are written as zeros by its own tasks
-  bool full = true;
-  for (int b = 0; b < nblock; ++b)
+  // Determinants outside a selection start from zero.  Those of blocks without
+  // CSFs are written as zeros by the blocks' own tasks, one sector each, unless
+  // they are many and a fourth of all: a pass over the vector writes eight in
+  // the time of one (18 orbitals (15,3) 2S+1 = 17, where they are 94 %, 16
+  // vectors: 80 us, with the pass 37).
+  bool zeroed = false;
+  int64_t without = 0;
+  for (int b = 0; b < nblock; ++b) {
     if (blocks[b].conf_sel != nullptr || (blocks[b].ncsf == 0 && blocks[b].nconf > 0 && blocks[b].ndet == 0))
-      full = false;
-  if (!full) {
+      zeroed = true;
+    if (blocks[b].ncsf == 0) without += blocks[b].nconf * blocks[b].ndet;
+  }
+  if (4 * without >= ndet && without * nvec >= 1 << 18) zeroed = true;
+  if (zeroed) {
     {
       ProfScope ps_("k_zero_rows", stream);
       k_zero_rows<<<grid_for((int64_t)nvec * ndet, 256, 148 * 16), 256, 0, stream>>>(x_det, ld_det,
@@ -469,7 +476,7 @@ int csffci_csf2det(int nvec, const double* x_csf, int64_t ld_csf, double* x_det,
   }
   for (int64_t v = 0; v < nvec; v += chunk) {
     const int st = run_blocks<XF_CSF2DET>((int)(nvec - v < chunk ? nvec - v : chunk), x_csf + v * ld_csf, ld_csf,
-                                          x_det + v * ld_det, ld_det, csd_mask, blocks, nblock, stream);
+                                          x_det + v * ld_det, ld_det, csd_mask, blocks, nblock, stream, zeroed);
     if (st) return st;
   }
   return CSFFCI_OK;
@@ -480,7 +487,7 @@ int csffci_hdiag_csf(int norb, int neleca, int nelecb, const double* hdiag_det, 
                      double* hdiag_csf, cudaStream_t stream) {
   CSF_REQUIRE(norb >= 0 && norb <= 63 && blocks != nullptr, "hdiag_csf: bad arguments");
   if (norb <= 16)
-    return run_blocks<XF_HDIAG>(1, hdiag_det, 0, hdiag_csf, 0, csd_mask, blocks, nblock, stream, norb, eri);
+    return run_blocks<XF_HDIAG>(1, hdiag_det, 0, hdiag_csf, 0, csd_mask, blocks, nblock, stream, false, norb, eri);
   // more than 16 orbitals (4 bits no longer name one): a thread per CSF
   int npair_orb = norb * (norb + 1) / 2;
   for (int b = 0; b < nblock; ++b) {

@@ -125,3 +125,22 @@ def test_many_vectors_fill_the_gpu(norb, na, nb, smult):
     d = torch.zeros((256, t.ndet), dtype=torch.float64, device="cuda")
     assert _us(lambda: t.dev_csf2det(x)) < 8 * _us(lambda: t.dev_csf2det(x[:1]))
     assert _us(lambda: t.dev_det2csf(d)) < 8 * _us(lambda: t.dev_det2csf(d[:1]))
+
+
+@pytest.mark.parametrize("norb,na,nb,smult,nvec", [(18, 15, 3, 17, 16), (20, 17, 3, 19, 16), (16, 12, 4, 13, 8)])
+def test_determinants_without_csfs(norb, na, nb, smult, nvec):
+    """Most determinants of a high-spin space are in configurations without
+    CSFs: zeros in the result, at the cost of a few passes over it (by their own
+    tasks 13 to 16)."""
+    import torch
+    from pyscf_forge_b200.csf_fci.csfstring import CSFTransformer
+    t = CSFTransformer(norb, na, nb, smult)
+    x = torch.ones((nvec, t.ncsf), dtype=torch.float64, device="cuda")
+    det = t.dev_csf2det(x)
+    for b in t._blocks:
+        rows = t.csd_mask[b["csd_offset"]:b["csd_offset"] + b["nconf"] * b["ndet"]].long()
+        if b["ncsf"] == 0:
+            assert not det[:, rows].any()
+        else:
+            assert det[:, rows].any()
+    assert _us(lambda: t.dev_csf2det(x)) < 9 * _us(lambda: det.zero_())
