@@ -422,10 +422,15 @@ int csffci_contract_1e(int norb, int neleca, int nelecb, const double* h1a, cons
   CSF_REQUIRE(norb >= 1 && norb <= 63, "contract_1e: bad norb %d", norb);
   unsigned long long Na = host_binom(norb, neleca), Nb = host_binom(norb, nelecb);
   int nla = neleca * (norb - neleca + 1), nlb = nelecb * (norb - nelecb + 1);
-  // rows that fit in shared memory (7000 columns at 16 orbitals)
+  // Rows that fit in shared memory (7000 columns at 16 orbitals), not for
+  // narrow or flat vectors: a block has a thread per column and four rows, so
+  // most of it would be idle (element-wise against by rows, us: 184756 x 1 121
+  // and 644, 38760 x 20 135 and 218, 10626 x 24 65 and 75, 1 x 3432 20 and 23;
+  // but 2024 x 24 25 and 20, 1770 x 60 56 and 30, 20 x 4845 46 and 36).
   const size_t smem = (((size_t)C1_ROWS * Nb * sizeof(double) + 15) & ~(size_t)15) +
                       (size_t)C1_ROWS * nla * sizeof(C1Link) + (size_t)norb * norb * sizeof(double);
-  if (Na > 0 && Nb > 0 && Na < (1ull << 31) && Nb < (1ull << 24) && smem <= 227 * 1024 - 1024) {
+  const bool wide = Nb >= 32 || (Nb >= 24 && Na <= 4096);
+  if (Na >= 14 && wide && Na < (1ull << 31) && Nb < (1ull << 24) && smem <= 227 * 1024 - 1024) {
     if (smem > 48 * 1024)
       CSF_CUDA(cudaFuncSetAttribute(k_contract_1e_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long nx = ((long long)Na + C1_ROWS - 1) / C1_ROWS;

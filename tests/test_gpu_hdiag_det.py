@@ -42,3 +42,38 @@ def test_contract_1e_against_oracle(norb, na, nb):
     got = D.dev_contract_1e(ha, hb, torch.as_tensor(ci, device="cuda"), norb, (na, nb),
                             torch.as_tensor(out, device="cuda")).cpu().numpy()
     assert np.abs(got - out - R.contract_1e_ab(ha, hb, ci, norb, (na, nb)).ravel()).max() < 1e-12
+
+
+def _us(call):
+    """Device time of one call, microseconds (the least of five)."""
+    import torch
+    call()
+    best = float("inf")
+    for _ in range(5):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        torch.cuda.synchronize()
+        e[0].record()
+        for _ in range(10):
+            call()
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]) * 100)
+    return best
+
+
+@pytest.mark.parametrize("norb,nelec", [(20, 10), (24, 9), (30, 5)])
+def test_contract_1e_of_one_column(norb, nelec):
+    """A vector of one beta string costs about what one of one alpha string
+    does (five times as much by rows), and both give the same."""
+    import torch
+    from math import comb
+    from pyscf_forge_b200.fci import direct_spin1 as D
+    rng = np.random.default_rng(norb)
+    h = torch.as_tensor(rng.normal(size=(norb, norb)), device="cuda")
+    ci = torch.as_tensor(rng.normal(size=comb(norb, nelec)), device="cuda")
+    out = [torch.zeros_like(ci) for _ in range(2)]
+    D.dev_contract_1e(h, h, ci, norb, (nelec, 0), out[0])
+    D.dev_contract_1e(h, h, ci, norb, (0, nelec), out[1])
+    assert float((out[0] - out[1]).abs().max()) < 1e-10  # at most 200 products below 30
+    assert _us(lambda: D.dev_contract_1e(h, h, ci, norb, (nelec, 0), out[0])) \
+        < 2.5 * _us(lambda: D.dev_contract_1e(h, h, ci, norb, (0, nelec), out[1]))
