@@ -46,39 +46,53 @@ __global__ void k_absorb_h2e(int norb, int npair, const double* h1e, const doubl
 //   jv[I][q] = sum_{i in I} J_iq          (only for the alpha strings)
 // with J_ij = (ii|jj) = eri[ii][jj], K_ij = (ij|ji) = eri[ij][ij].
 //
-// A warp per string of either spin, its lanes over q: the sums are chains of
-// loads, so what counts is how many run at once (one thread per string left
-// most of the GPU idle: 45 us a spin at 14 orbitals and 7 electrons, now
-// 10 us for both in one launch).
+// LANES 32: a warp per string of either spin, its lanes over q.  The sums are
+// chains of loads, so what counts is how many run at once (one thread per
+// string left most of the GPU idle: 45 us a spin at 14 orbitals and 7 electrons,
+// now 10 us for both in one launch).  LANES 1: a thread per string, for as many
+// strings as fill the GPU that way: 32 lanes then only multiply the work of
+// finding a string and its orbitals (see hdiag_det_run).
+template <int LANES>
 __global__ void __launch_bounds__(128) k_string_energy(int norb, int neleca, int nelecb, int npair,
                                                        unsigned long long na, unsigned long long nb,
                                                        const double* __restrict__ ha, const double* __restrict__ hb,
                                                        const double* __restrict__ eri, double* ea, double* ja,
                                                        double* eb, uint64_t* sb) {
-  const int lane = threadIdx.x & 31;
-  const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-  for (unsigned long long w = blockIdx.x * (unsigned long long)(blockDim.x >> 5) + (threadIdx.x >> 5); w < na + nb;
+  const int lane = threadIdx.x & (LANES - 1);
+  const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x / LANES);
+  for (unsigned long long w = blockIdx.x * (unsigned long long)(blockDim.x / LANES) + threadIdx.x / LANES; w < na + nb;
        w += nw) {
     const bool alpha = w < na;
     const unsigned long long I = alpha ? w : w - na;
     const unsigned long long s = str_unrank(norb, alpha ? neleca : nelecb, I);
     const double* const h = alpha ? ha : hb;
     double e = 0.0;
-    for (int q = lane; q < norb; q += 32) {
+    for (int q = lane; q < norb; q += LANES) {
+      const bool occ = (s >> q) & 1ull;
+      if (LANES == 1 && !alpha && !occ) continue;
       const int qq = pair_index(q, q);
       double j = 0.0, k = 0.0;
-#pragma unroll 4
-      for (int i = 0; i < norb; ++i)
-        if ((s >> i) & 1ull) {
+      if (LANES == 1) {
+        for (unsigned long long b = s; b; b &= b - 1) {
+          const int i = __ffsll((long long)b) - 1;
           const int iq = pair_index(i, q);
           j += eri[(int64_t)pair_index(i, i) * npair + qq];
-          k += eri[(int64_t)iq * npair + iq];
+          if (occ) k += eri[(int64_t)iq * npair + iq];
         }
-      if ((s >> q) & 1ull) e += h[q * norb + q] + 0.5 * (j - k);
+      } else {
+#pragma unroll 4
+        for (int i = 0; i < norb; ++i)
+          if ((s >> i) & 1ull) {
+            const int iq = pair_index(i, q);
+            j += eri[(int64_t)pair_index(i, i) * npair + qq];
+            k += eri[(int64_t)iq * npair + iq];
+          }
+      }
+      if (occ) e += h[q * norb + q] + 0.5 * (j - k);
       if (alpha) ja[I * norb + q] = j;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+    for (int o = LANES / 2; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
     if (lane == 0) {
       if (alpha) {
         ea[I] = e;
@@ -95,6 +109,7 @@ __global__ void __launch_bounds__(128) k_string_energy(int norb, int neleca, int
 // block: two table reads an element at 14 orbitals instead of a loop over 7
 // electrons (110 -> 26 us for 94 MB, which take 15 us to write).
 constexpr int HD_BITS = 7, HD_ROWS = 4;
+constexpr long long HD_WARPS = 20000;
 __global__ void __launch_bounds__(256) k_hdiag_det_table(int norb, unsigned long long Na, unsigned long long Nb,
                                                          const double* __restrict__ ea, const double* __restrict__ eb,
                                                          const double* __restrict__ ja, const uint64_t* __restrict__ sb,
@@ -159,8 +174,13 @@ static int hdiag_det_run(int norb, int neleca, int nelecb, unsigned long long Na
                          const double* h1a, const double* h1b, const double* eri, double* ea, double* ja, double* eb,
                          uint64_t* sb, double* hdiag, cudaStream_t stream) {
   const int npair = norb * (norb + 1) / 2;
-  k_string_energy<<<grid_for((long long)(Na + Nb) * 32, 128), 128, 0, stream>>>(norb, neleca, nelecb, npair, Na, Nb,
-                                                                                h1a, h1b, eri, ea, ja, eb, sb);
+  // a warp per string up to HD_WARPS strings (us, warps against threads: 13 000
+  // strings 40 and 57, 18 600 36 and 40, 26 000 56 and 45, 78 000 155 and 45,
+  // 735 000 1580 and 214)
+  const long long nstr = (long long)(Na + Nb);
+  auto kern = nstr <= HD_WARPS ? k_string_energy<32> : k_string_energy<1>;
+  kern<<<grid_for(nstr <= HD_WARPS ? nstr * 32 : nstr, 128), 128, 0, stream>>>(norb, neleca, nelecb, npair, Na, Nb, h1a,
+                                                                               h1b, eri, ea, ja, eb, sb);
   const int st = check_launch("hdiag_det strings");
   if (st) return st;
   ProfScope ps_("k_hdiag_det", stream);
