@@ -120,7 +120,9 @@ __device__ __forceinline__ unsigned long long xf_somos(const XfOrb& o, int64_t c
   return out;
 }
 
-// B fragment of columns n0 + 8 t + g, k = kb + t + 4 j
+// B fragment of columns n0 + 8 t + g, k = kb + t + 4 j.  umat is indexed in 32
+// bits without sign: at most 2^32 determinants leave a block at most 65535 spin
+// determinants and no more CSFs, but 25 orbitals (20,5) have 2.15e9 entries.
 template <int MODE>
 __device__ __forceinline__ void xf_bfrag(const XfTile& B, const double* u, int n, int N, int kb, int k1, int tq,
                                          double (&b)[4]) {
@@ -128,7 +130,7 @@ __device__ __forceinline__ void xf_bfrag(const XfTile& B, const double* u, int n
   for (int j = 0; j < 4; ++j) {
     const int k = kb + tq + 4 * j;
     double v = 0.0;
-    if (k < k1 && n < N) v = MODE == XF_CSF2DET ? u[n * B.ncsf + k] : u[k * B.ncsf + n];
+    if (k < k1 && n < N) v = u[MODE == XF_CSF2DET ? (uint32_t)n * (uint32_t)B.ncsf + k : (uint32_t)k * (uint32_t)B.ncsf + n];
     b[j] = MODE == XF_HDIAG ? v * v : v;
   }
 }
