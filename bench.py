@@ -29,7 +29,8 @@ C0-C2 end to end, beside the reference solver's timings and energies
 (run_solves).
 
 Reference arm: the reference's own CPU sigma (pyscf/lib/mcscf GAS library
-with one subspace, built into oracle/_ref) on all host cores.
+with one subspace, built into oracle/_ref) on all host cores; where that is
+not built, a line that says so.
 """
 import argparse
 import json
@@ -45,6 +46,7 @@ sys.path.insert(0, ROOT)
 NORB, NELEC, RANK = 16, (8, 8), 32
 WORKLOAD = "CAS(16,16) (8,8) singlet FP64 sigma"
 METRIC = "CAS(16,16) FP64 sigma/s"
+NO_REFERENCE = "the reference's CPU library (oracle/_ref) is not built here"
 # smaller singlet cases of the same kernel, for profiling captures
 WORKLOADS = {"cas16": (16, (8, 8), 32), "cas14": (14, (7, 7), 28), "cas12": (12, (6, 6), 24),
              "cas16_5e5e": (16, (5, 5), 32)}
@@ -202,6 +204,10 @@ def run_reference(args, rank_env):
     if rank != 0:
         return
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import gasref
+    if not gasref.available():
+        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
+        return
     import restate as R
     from math import comb
     h1, eri = seeded_integrals(NORB, RANK)
@@ -346,7 +352,7 @@ def run_ours(args, rank_env):
         import gasref
         if not gasref.available():
             with_ref = False
-            line["cpu_baseline"] = {"unavailable": "the reference's CPU library (oracle/_ref) is not built here"}
+            line["cpu_baseline"] = {"unavailable": NO_REFERENCE}
     if rank == 0 and world == 1 and with_ref:
         # one full reference sigma on the host, on the very vector the timed
         # loop used: the measured CPU baseline, and the check of the timed
