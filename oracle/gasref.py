@@ -24,6 +24,8 @@ import os
 
 import numpy as np
 
+import restate
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 REF_DIR = os.path.join(HERE, "_ref")
 
@@ -267,7 +269,11 @@ def make_rdm12s(bra, ket, norb, nelec):
 
 
 def make_rdm12(bra, ket, norb, nelec):
-    """Spin-free assembly as in pyscf/mcscf/fci_gas.py:724-733."""
+    """Spin-free assembly as in pyscf/mcscf/fci_gas.py:724-733.  Without the
+    library, the dense restatement, which is compared with it where it is built
+    (tests/test_oracle.py)."""
+    if not available():
+        return restate.make_rdm12(np.asarray(bra), np.asarray(ket), norb, nelec)
     (d1a, d1b), (d2aa, d2ab, d2bb) = make_rdm12s(bra, ket, norb, nelec)
     dm2 = d2aa + d2bb + d2ab + d2ab.transpose(2, 3, 0, 1)
     return d1a + d1b, dm2
