@@ -94,6 +94,24 @@ def test_large_spaces(same, norb, na, nb):
     assert float((m2 - d2[0] - d2[2] - d2[1] - d2[1].permute(2, 3, 0, 1)).abs().max()) < 4 * tol
 
 
+@pytest.mark.parametrize("norb,n", [(13, 5), (16, 4)])
+@pytest.mark.parametrize("eta", [1, -1])
+def test_large_symmetric_spaces(norb, n, eta):
+    """c = +-c^T, which forms the strings' lower triangle alone, with 45 and 52
+    links a spin."""
+    import torch
+    from pyscf_forge_b200.fci import direct_spin1 as D
+    gen = torch.Generator(device="cuda").manual_seed(norb)
+    c = torch.randn((comb(norb, n),) * 2, dtype=torch.float64, device="cuda", generator=gen)
+    c = c + eta * c.T
+    c /= torch.linalg.vector_norm(c)
+    tol = 32 * 2.0 ** -53 * c.numel() ** 0.5
+    d1, d2 = _reference(c, c, norb, n, n)
+    m1, m2 = D.dev_rdm12(c.reshape(-1), None, norb, (n, n))
+    assert float((m1 - d1[0] - d1[1]).abs().max()) < 2 * tol
+    assert float((m2 - d2[0] - d2[2] - d2[1] - d2[1].permute(2, 3, 0, 1)).abs().max()) < 4 * tol
+
+
 # the form that is faster by a wide margin at these sizes: (bra is ket, space, fused)
 FORMS = [(False, 16, 8, 0, False), (False, 14, 7, 0, False), (True, 16, 8, 0, False), (False, 16, 2, 2, False),
          (False, 13, 1, 1, False), (False, 12, 4, 3, True), (False, 16, 3, 3, True), (False, 11, 5, 4, True),

@@ -144,3 +144,46 @@ def test_determinants_without_csfs(norb, na, nb, smult, nvec):
         else:
             assert det[:, rows].any()
     assert _us(lambda: t.dev_csf2det(x)) < 9 * _us(lambda: det.zero_())
+
+
+@pytest.mark.parametrize("norb,na,nb,smult", [(10, 5, 5, 1), (12, 6, 6, 3), (12, 7, 4, 4), (14, 7, 7, 3), (16, 4, 4, 1)])
+def test_diagonal_of_large_spaces(norb, na, nb, smult):
+    """Up to 14 open shells, 91 exchange pairs and 1001 CSFs a configuration:
+    sum_x U[x,k]^2 hdiag[x] + sum_ab K(a,b) Z[ab,k] on 40 configurations of every
+    block, the open shells taken from the strings of a determinant.
+
+    Tolerance: both sums have at most 3432 + 91 terms, of weights that add up to
+    1 and 91 at most, of N(0, 1) values (below 8): rounding below
+    4000 * 92 * 8 * 1.1e-16 = 4e-10 in any order, 1e-11 and less in practice."""
+    import torch
+    from pyscf_forge_b200 import _capi
+    from pyscf_forge_b200._runtime import ptr, stream
+    from pyscf_forge_b200.csf_fci.csfstring import CSFTransformer
+    t = CSFTransformer(norb, na, nb, smult)
+    g = torch.Generator(device="cuda").manual_seed(norb)
+    npair = norb * (norb + 1) // 2
+    hd = torch.randn(t.ndet, generator=g, dtype=torch.float64, device="cuda")
+    eri = torch.randn((npair, npair), generator=g, dtype=torch.float64, device="cuda")
+    got = t.dev_hdiag_csf(hd, eri)
+    strs = []
+    for n, count in ((na, t.ndeta), (nb, t.ndetb)):
+        s = torch.empty(count, dtype=torch.int64, device="cuda")
+        _capi.call("csffci_gen_strings", norb, n, ptr(s), stream())
+        strs.append(s)
+    kk = eri.diagonal()
+    for b in t._blocks:
+        if not b["ncsf"]:
+            continue
+        conf = torch.randint(b["nconf"], (min(40, b["nconf"]),), generator=g, device="cuda")
+        rows = conf[:, None] * b["ndet"] + torch.arange(b["ndet"], device="cuda")
+        dets = t.csd_mask[b["csd_offset"] + rows].long()
+        want = hd[dets] @ b["umat"].reshape(b["ndet"], b["ncsf"]) ** 2
+        if b["nspin"] >= 2:
+            open_ = strs[0][dets[:, 0] // t.ndetb] ^ strs[1][dets[:, 0] % t.ndetb]
+            bits = (open_[:, None] >> torch.arange(norb, device="cuda")) & 1
+            somo = bits.nonzero()[:, 1].reshape(len(conf), b["nspin"])
+            ab = [(i, j) for j in range(b["nspin"]) for i in range(j)]
+            lo, hi = (somo[:, [p[q] for p in ab]] for q in (0, 1))
+            want = want + kk[hi * (hi + 1) // 2 + lo] @ b["zmat"]
+        cols = b["csf_offset"] + conf[:, None] * b["ncsf"] + torch.arange(b["ncsf"], device="cuda")
+        assert float((got[cols] - want).abs().max()) < 4e-10
