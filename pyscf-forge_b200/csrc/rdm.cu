@@ -577,8 +577,8 @@ static RdmFusedJob fused_job(int norb, int neleca, int nelecb, const csffci_link
 // Whether the fused kernel takes these Grams (one, or alpha-alpha, beta-beta
 // and alpha-beta), or the slab form does: the shorter of two estimates in
 // microseconds, fitted to both forms at 8 to 16 orbitals and 1 to 260 000
-// determinants (870 calls; the form taken was never more than 1.27 times the
-// other's time).  The fused kernel pays for every pass over the determinants
+// determinants (870 calls; the form taken was at most 1.3 times the other's
+// time).  The fused kernel pays for every pass over the determinants
 // and for whole tiles of 16 columns, the slab form by the element of T and of
 // its 64 x 64 Gram tiles.  Measured, slab form against fused (us), two vectors at 16
 // orbitals: 8960 determinants 106 against 194, 12870 x 1 164 against 1544,

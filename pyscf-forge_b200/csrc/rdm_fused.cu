@@ -1,7 +1,7 @@
 // Fused RDM kernel: the excitation rows of a tile of determinants are built
 // in shared memory and contracted there, so that T(pq, J) = <J|E_pq|c> never
 // goes through global memory (norb 2..16; rdm.cu keeps the slab form for the
-// rest).
+// rest, and for vectors of few columns or few determinants: take_fused).
 //
 // Rows.  For a real vector with bra == ket the ordered rows T_pq are replaced
 // by S_pq = T_pq + T_qp (p > q; S_pp = T_pp) and A_pq = T_pq - T_qp.  By
@@ -400,7 +400,8 @@ __device__ __forceinline__ bool rf_movers(const RFArgs& g, unsigned char* smraw,
 // warps.  The MMA warps wait for a stage one by one (mbarrier), so a warp
 // that is done early starts the next tile while the others finish.  SPLIT:
 // registers re-split between the roles (setmaxnreg): launched with 128 per
-// thread, 512 threads, MMA warps 144, movers 80.
+// thread, 512 threads, MMA warps 8 (BASE + 1) + 40 and at most 184, movers the
+// rest of 256 (144 and 112 at 14 orbitals, 184 and 72 at 16).
 template <int BASE, bool SPLIT, int NS>
 __global__ void __launch_bounds__((RF_NMW + RF_NMOV) * 32, 1) k_rdm_fused(const __grid_constant__ RFArgs g) {
   constexpr int NTH = (RF_NMW + RF_NMOV) * 32;
@@ -492,6 +493,9 @@ __global__ void __launch_bounds__((RF_NMW + RF_NMOV) * 32, 1) k_rdm_fused(const 
       }
   } else {
     if constexpr (SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(REG_MOV));
+    // groups of 16 links a lane holds: five for one row set at 13 to 15 orbitals,
+    // where a spin has up to 49, 56 and 64 links (four would hold them; not
+    // measured), else three, and the plain loops take the links beyond
     if (!rf_movers<(NS == 1 && BASE >= 8 && BASE < 16) ? 5 : 3, NS>(g, smraw, sym, L0, L1, tid - RF_NMW * 32, lane, warp - RF_NMW)) bad_s = 1;
   }
   __syncthreads();  // the partial sums of this CTA are written
@@ -707,22 +711,18 @@ static int rf_dispatch(RFArgs& g, int grid, size_t smem, cudaStream_t stream) {
       RF_CASE(18, 1);  // 16
       default: break;
     }
-  else switch (g.base) {
+  else switch (g.base) {  // those of one, two, three or four passes at 2 to 16 orbitals
       RF_CASE(0, 2);
       RF_CASE(1, 2);
       RF_CASE(2, 2);
       RF_CASE(3, 2);
       RF_CASE(4, 2);
       RF_CASE(5, 2);
-      RF_CASE(6, 2);
-      RF_CASE(7, 2);
       RF_CASE(8, 2);
       RF_CASE(9, 2);
       RF_CASE(10, 2);
       RF_CASE(11, 2);
-      RF_CASE(12, 2);
       RF_CASE(13, 2);
-      RF_CASE(14, 2);
       RF_CASE(15, 2);
       RF_CASE(16, 2);
       RF_CASE(17, 2);
@@ -786,7 +786,7 @@ size_t rdm_fused_workspace(int norb, long long Nb, int nlb) {
 }
 
 bool rdm_fused_fits(const RdmFusedJob& j) {
-  // Na * Nb indexes a vector in 32 bits
+  // 16 orbitals at most: C(16, 8)^2 determinants, which index a vector in 32 bits
   if (j.norb < 2 || j.norb > 16) return false;
   RFArgs g = rf_args(j);
   return rf_layout(g) != 0;

@@ -81,7 +81,9 @@ struct MPLayout {
   // setmaxnreg; the k-steps from KR on are then read from shared memory.  The
   // movers of a job table hold what for one problem is in constant memory or
   // in uniform registers: 56 spilled (20 problems of 12 orbitals 8.28 ms, in an
-  // earlier form), 72 do not (6.83 ms).  At 13 orbitals shared memory has no room for more.
+  // earlier form), 72 do not (6.83 ms).  At 13 orbitals a table has 56 and does
+  // not spill; 12 k-steps in registers there would need 196 KB of shared memory
+  // in place of 181 and have not been measured.
   static constexpr bool SPLIT = NMMA == 12;
   static constexpr int KR = KS <= 14 ? KS : KS > 20 ? 17 : BATCH ? 12 : 17;
   static constexpr int AT = (KS - KR) * (PT + (TAIL ? 1 : 0)) * 64;  // elements of that part of h2e

@@ -77,16 +77,17 @@ int sigma_rr_single_variant(int norb) {
 // singlet 7.6 -> 4.5, 8 (4,4) singlet 12.4 -> 5; call: 11 (6,5) 199 -> 121, 12
 // (6,6) singlet 368 -> 249, 13 (7,6) 2600 -> 1840; tables of 20 large problems,
 // kernel: 8 orbitals 38 -> 26, 10 388 -> 271, 11 1695 -> 1083, 12 7430 ->
-// 5280; of 30 small ones: 8 orbitals 25 -> 17, 10 68 -> 45, 12 198 -> 146.  k_sigma_ws against the best tile shape: 14
-// orbitals singlet 7.61 -> 6.31 ms, 15: 31.1 -> 25.8 ms.  The batched
-// solver's autotuner times every variant on its own job tables.
+// 5280; of 30 small ones: 8 orbitals 25 -> 17, 10 68 -> 45, 12 198 -> 146.
+// k_sigma_ws against the best tile shape: 14 orbitals singlet 7.61 -> 6.31 ms,
+// 15: 31.1 -> 25.8 ms.  The batched solver's autotuner times every variant on
+// its own job tables.
 int rr_default_variant(int norb) {
   const char* env = getenv("CSFFCI_SIGMA_VARIANT");
   if (env) {
     const int v = atoi(env);
     if (batch_variant_valid(norb, v)) return v;
   }
-  return sigma_ws_supported(norb) ? RR_VARIANT_WS : 2;
+  return RR_VARIANT_WS;  // 4 to 16 orbitals, which is all that comes here
 }
 
 // fill the bookkeeping fields of the jobs; returns the largest Nb, nla, nlb
