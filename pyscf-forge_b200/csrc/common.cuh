@@ -96,6 +96,13 @@ __host__ __device__ inline int pair_index(int p, int q) {
   return hi * (hi + 1) / 2 + lo;
 }
 
+// Dynamic shared memory of a block at most (static: up to 256 bytes).  A kernel
+// that needs more than 48 KB is allowed this much whatever the call takes: the
+// limit belongs to the kernel, and one of the call's own size would fail the
+// launch of a larger call that another thread is making, or of a plan made
+// before.
+constexpr int MAX_SMEM = 227 * 1024 - 256;
+
 inline int grid_for(long long n, int block, int cap = 148 * 32) {
   long long g = (n + block - 1) / block;
   if (g > cap) g = cap;

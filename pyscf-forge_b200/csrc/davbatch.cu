@@ -53,6 +53,13 @@ constexpr int DB_NW = DB_NT / 32;
 constexpr int DB_ST = 128;  // threads of the small per-problem kernels
 constexpr int DB_RT = 256;  // threads of the subspace eigenproblem
 
+// shared memory of the subspace eigenproblem, matrices of ld columns; the
+// kernel is allowed the most of any plan (see MAX_SMEM)
+constexpr size_t db_ritz_smem(size_t ld) {
+  return sizeof(double) * (2 * ld * ld + (2 * DB_KMAX + 1) * ld) + sizeof(int) * ld;
+}
+constexpr int DB_RITZ_SMEM = (int)db_ritz_smem(DB_CAPMAX | 1);
+
 struct DBProb {
   int64_t n;
   int32_t k, cap, space, unit0, nunits, pad;
@@ -910,16 +917,6 @@ int enqueue_iteration(csffci_batch_plan_t* P, cudaStream_t s) {
   return P->kb <= 4 ? enqueue_iteration_km<4>(P, s) : enqueue_iteration_km<DB_KMAX>(P, s);
 }
 
-template <int KM>
-int set_stream_smem(int bytes) {
-  CSF_CUDA(cudaFuncSetAttribute(k_db_proj<KM, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  CSF_CUDA(cudaFuncSetAttribute(k_db_proj<KM, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  CSF_CUDA(cudaFuncSetAttribute(k_db_proj<KM, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  CSF_CUDA(cudaFuncSetAttribute(k_db_hv<KM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  CSF_CUDA(cudaFuncSetAttribute(k_db_ritz<KM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  return CSFFCI_OK;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1240,9 +1237,9 @@ int csffci_batch_plan_bind(csffci_batch_plan_t* P, void* arena, size_t arena_byt
   const int km = P->kb <= 4 ? 4 : DB_KMAX;
   P->smem_stream = sizeof(double) * km * (DB_CH + DB_CAPMAX);
   const size_t ldr = P->capb | 1;
-  P->smem_ritz = sizeof(double) * (2 * ldr * ldr + (2 * DB_KMAX + 1) * ldr) + sizeof(int) * ldr;
+  P->smem_ritz = db_ritz_smem(ldr);
   if (P->smem_ritz > 48 * 1024)
-    CSF_CUDA(cudaFuncSetAttribute(k_db_sritz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P->smem_ritz));
+    CSF_CUDA(cudaFuncSetAttribute(k_db_sritz, cudaFuncAttributeMaxDynamicSharedMemorySize, DB_RITZ_SMEM));
   CSF_CUDA(cudaMallocHost(&P->hcount, sizeof(int)));
   CSF_CUDA(cudaStreamSynchronize(stream));
   P->bound = true;

@@ -450,9 +450,9 @@ int csffci_contract_1e(int norb, int neleca, int nelecb, const double* h1a, cons
   const size_t smem = (((size_t)C1_ROWS * Nb * sizeof(double) + 15) & ~(size_t)15) +
                       (size_t)C1_ROWS * nla * sizeof(C1Link) + (size_t)norb * norb * sizeof(double);
   const bool wide = Nb >= 32 || (Nb >= 24 && Na <= 4096);
-  if (Na >= 14 && wide && Na < (1ull << 31) && Nb < (1ull << 24) && smem <= 227 * 1024 - 1024) {
+  if (Na >= 14 && wide && Na < (1ull << 31) && Nb < (1ull << 24) && smem <= MAX_SMEM) {
     if (smem > 48 * 1024)
-      CSF_CUDA(cudaFuncSetAttribute(k_contract_1e_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      CSF_CUDA(cudaFuncSetAttribute(k_contract_1e_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
     const long long nx = ((long long)Na + C1_ROWS - 1) / C1_ROWS;
     // few rows: the columns are split as well
     long long ny = (2 * 148 + nx - 1) / nx, most = ((long long)Nb + 255) / 256;

@@ -489,8 +489,8 @@ static int tslab_tile_launch(int norb, long long Nb, int nla, int nlb, const csf
                              const csffci_link_t* lb, const double* c, long long J0, long long s, int spin,
                              double* T, cudaStream_t stream) {
   const size_t smem = (size_t)norb * norb * TT_LD * sizeof(double);
-  if (smem > 48 * 1024) CSF_CUDA(cudaFuncSetAttribute(k_tslab_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      (int)smem));
+  if (smem > 48 * 1024)
+    CSF_CUDA(cudaFuncSetAttribute(k_tslab_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
   ProfScope ps("k_tslab_tile", stream);
   k_tslab_tile<<<grid_for((s + TT_J - 1) / TT_J, 1, 148 * 4), 256, smem, stream>>>(norb, Nb, nla, nlb, la, lb, c,
                                                                                    J0, s, spin, T);

@@ -646,7 +646,7 @@ static size_t rf_layout(RFArgs& g) {
     g.off_rf = take((size_t)g.rows_e * sizeof(int));
     g.off_tab = take((size_t)(RF_MAXT + RF_NMW) * sizeof(int2));
     g.off_bar = take((2 * RF_XST + RF_LST) * sizeof(unsigned long long));
-    if (off <= 227 * 1024 - 256) return off;
+    if (off <= MAX_SMEM) return off;
   }
   return 0;
 }
@@ -688,7 +688,7 @@ static int rf_launch(const RFArgs& g, int grid, size_t smem, cudaStream_t stream
       return CSFFCI_ERR_INVALID;
     }
   }
-  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
   ProfScope ps("k_rdm_fused", stream);
   kern<<<grid, (RF_NMW + RF_NMOV) * 32, smem, stream>>>(g);
   return check_launch("rdm (fused)");

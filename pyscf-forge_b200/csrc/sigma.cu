@@ -337,13 +337,15 @@ static int pick_stride(int base, int want_mod16a, int want_mod16b) {
   return s;
 }
 
+constexpr size_t K_SIGMA_SMEM = 227 * 1024;  // allowed whatever the call takes (see MAX_SMEM); no static part
+
 static SigmaConfig sigma_config(int norb, int nla) {
   SigmaConfig c;
   int npair = norb * (norb + 1) / 2;
   c.npad = (npair + 7) & ~7;
   c.threads = 4 * c.npad;
   c.hstride = pick_stride(c.npad, 4, 12);
-  const size_t limit = 227 * 1024;
+  const size_t limit = K_SIGMA_SMEM;
   size_t links = (size_t)((c.npad + 1) & ~1) * 4 + (size_t)nla * 8 + 64;
   c.hsmem = false;
   c.nt = 2;
@@ -375,7 +377,7 @@ static SigmaConfig sigma_config(int norb, int nla) {
 template <int NT, bool HS>
 static int launch_sigma(const SigmaConfig& c, SigmaArgs& g, int grid, cudaStream_t stream) {
   auto kern = k_sigma<NT, HS>;
-  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
+  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K_SIGMA_SMEM));
   ProfScope ps("k_sigma", stream);
   kern<<<grid, c.threads, c.smem, stream>>>(g);
   return check_launch("sigma");

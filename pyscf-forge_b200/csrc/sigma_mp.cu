@@ -520,7 +520,7 @@ static int mp_launch_as(int norb, MPArgs& g, long long max_nb, long long max_til
   g.off_al = take((size_t)MP_AL * L::NP * sizeof(uint2));
   g.off_job = take(sizeof(MPJob));
   g.off_bar = take(8 * sizeof(unsigned long long));
-  if (off > 227 * 1024 - 256) {
+  if (off > MAX_SMEM) {
     set_error("sigma: row-pair tiles exceed shared memory (%zu)", off);
     return CSFFCI_ERR_INVALID;
   }
@@ -535,7 +535,7 @@ static int mp_launch_as(int norb, MPArgs& g, long long max_nb, long long max_til
       return CSFFCI_ERR_INVALID;
     }
   }
-  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)off));
+  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
   const int grid = (int)(max_tiles < 148 ? (max_tiles > 0 ? max_tiles : 1) : 148);  // one CTA per SM
   g.rounds = (int)(nelem * 16 / MP_ROUND + 1);
   if (g.rounds > 256) g.rounds = 256;

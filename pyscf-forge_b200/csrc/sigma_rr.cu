@@ -173,7 +173,7 @@ int sigma_rr_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev,
   g.off_pn = take((size_t)2 * npair * sizeof(unsigned));
   g.off_zf = take((size_t)npair * sizeof(int));
   const size_t smem = off;
-  if (smem > 227 * 1024 - 256) {
+  if (smem > MAX_SMEM) {
     set_error("sigma: tile of %zu bytes exceeds shared memory", smem);
     return CSFFCI_ERR_INVALID;
   }

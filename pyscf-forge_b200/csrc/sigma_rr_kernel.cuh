@@ -431,7 +431,7 @@ template <int KS, int MT, int MW, int NT>
 static int launch_rr(RRArgs& g, size_t smem, cudaStream_t stream) {
   constexpr int NW = RRLayout<MT, MW, NT>::NW;
   auto kern = g.jobs ? k_sigma_rr<KS, MT, MW, NT, true> : k_sigma_rr<KS, MT, MW, NT, false>;
-  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
   int dev = 0, nsm = 148, per_sm = 1;
   CSF_CUDA(cudaGetDevice(&dev));
   CSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));

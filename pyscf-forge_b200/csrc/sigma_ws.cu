@@ -280,7 +280,7 @@ static int launch_ws(RRArgs& g, size_t smem, cudaStream_t stream) {
                                                   : k_sigma_ws<KS, MT, MW, true, MINB, ONLY_DET>)
                      : ((MW == 8 && g.det_stride) ? k_sigma_ws<KS, MT, MW, false, MINB, MW == 8>
                                                   : k_sigma_ws<KS, MT, MW, false, MINB, ONLY_DET>);
-  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
   int dev = 0, nsm = 148, per_sm = 0;
   CSF_CUDA(cudaGetDevice(&dev));
   CSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -330,7 +330,7 @@ size_t ws_layout(RRArgs& g, int npair, int rows_multiple, long long max_nb, int 
     const unsigned o = take(extra_bytes);
     if (extra_off) *extra_off = o;
   }
-  return off > 227 * 1024 - 256 ? 0 : off;
+  return off > MAX_SMEM ? 0 : off;
 }
 
 int sigma_ws_launch(int norb, int njobs, const csffci_sigma_job_t* jobs_dev, const csffci_sigma_job_t& job0,

@@ -315,7 +315,7 @@ int sigma_wsr_launch(int norb, const csffci_sigma_job_t& job0, long long total_u
               WSR_REG_LAUNCH);
     return CSFFCI_ERR_INVALID;
   }
-  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CSF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
   int dev = 0, nsm = 148, per_sm = 0;
   CSF_CUDA(cudaGetDevice(&dev));
   CSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
