@@ -9,10 +9,10 @@
 // What bounds it: the random 8-byte accesses through csd_mask (one 32-byte
 // sector each), then latency.  Measured, block by block launches of 64 x 64
 // GEMM tiles and a thread per configuration -> this:
-//   CAS(14,14) triplet, 2 vectors  CSF->det 0.91 -> 0.36 ms, det->CSF 1.01 -> 0.29 ms
-//   CAS(12,12) singlet, 3 vectors  CSF->det 0.38 -> 0.08 ms, det->CSF 0.42 -> 0.05 ms
-//   CAS(16,16) singlet, 1 vector   CSF->det 4.9 -> 3.2 ms, det->CSF 3.4 -> 2.3 ms
-//   CAS(14,14) triplet diagonal    2.75 -> 0.34 ms
+//   CAS(14,14) triplet, 2 vectors  CSF->det 0.91 -> 0.34 ms, det->CSF 1.01 -> 0.25 ms
+//   CAS(12,12) singlet, 3 vectors  CSF->det 0.38 -> 0.04 ms, det->CSF 0.42 -> 0.03 ms
+//   CAS(16,16) singlet, 1 vector   CSF->det 4.9 -> 3.1 ms, det->CSF 3.4 -> 2.15 ms
+//   CAS(14,14) triplet diagonal    2.75 -> 0.33 ms
 #include <string.h>
 
 #include "common.cuh"
