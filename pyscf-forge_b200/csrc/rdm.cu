@@ -497,8 +497,10 @@ static int tslab_tile_launch(int norb, long long Nb, int nla, int nlb, const csf
   return check_launch("rdm T slab");
 }
 
+// pairs: 0 below two electrons (of that spin), whose terms cancel but for
+// rounding, else 1 (NaN stays)
 __global__ void k_rdm_assemble(int norb, const double* __restrict__ G, int ld, const double* __restrict__ d1,
-                               double* dm2) {
+                               double pairs, double* dm2) {
   const int n = norb, n2 = n * n;
   long long tot = (long long)n2 * n2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
@@ -509,14 +511,14 @@ __global__ void k_rdm_assemble(int norb, const double* __restrict__ G, int ld, c
     int s = (int)(t % n);
     double v = G[(long long)(q * n + p) * ld + r * n + s];
     if (q == r) v -= d1[s * n + p];
-    dm2[t] = v;
+    dm2[t] = pairs * v;
   }
 }
 
 // spin-resolved assembly: dm2[p][q][r][s] = G[(qp)][(rs)] - d_qr d1[p][s]
 // (same-spin blocks) or G[(qp)][(rs)] (alpha-beta block, d1 == NULL)
 __global__ void k_rdm_assemble_s(int norb, const double* __restrict__ G, int ld, const double* __restrict__ d1,
-                                 double* dm2) {
+                                 double pairs, double* dm2) {
   const int n = norb, n2 = n * n;
   long long tot = (long long)n2 * n2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
@@ -527,7 +529,8 @@ __global__ void k_rdm_assemble_s(int norb, const double* __restrict__ G, int ld,
     int s = (int)(t % n);
     double v = G[(long long)(q * n + p) * ld + r * n + s];
     if (d1 && q == r) v -= d1[p * n + s];
-    dm2[t] = v;
+    // p+ r+ s q of one spin vanishes for p = r and for q = s
+    dm2[t] = (d1 && (p == r || q == s) ? 0.0 : pairs) * v;
   }
 }
 
@@ -685,7 +688,7 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
     if ((st = check_launch("rdm1 from the Gram"))) return st;
     k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1t, dm1);
     if ((st = check_launch("rdm1 transpose"))) return st;
-    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, ld, dm1, dm2);
+    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, ld, dm1, ne < 2 ? 0.0 : 1.0, dm2);
     return check_launch("rdm2 assemble");
   }
   long long S = ndet < (1ll << 18) ? ndet : (1ll << 18);
@@ -718,7 +721,8 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1t, dm1);
   if ((st = check_launch("rdm1 transpose"))) return st;
   if (dm2) {
-    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, n2, dm1, dm2);
+    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(
+        norb, G, n2, dm1, neleca + nelecb < 2 ? 0.0 : 1.0, dm2);
     return check_launch("rdm2 assemble");
   }
   return CSFFCI_OK;
@@ -793,11 +797,12 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
         if ((st = check_launch("rdm1 from the Gram"))) return st;
         k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1t, s ? dm1b : dm1a);
         if ((st = check_launch("rdm1 transpose"))) return st;
-        k_rdm_assemble_s<<<gs, 256, 0, stream>>>(norb, G, ld, d1t, s ? dm2bb : dm2aa);
+        k_rdm_assemble_s<<<gs, 256, 0, stream>>>(norb, G, ld, d1t, ne < 2 ? 0.0 : 1.0,
+                                                s ? dm2bb : dm2aa);
         if ((st = check_launch("rdm2 assemble"))) return st;
       }
       if ((st = rdm_fused_run(Jab, work, stream))) return st;
-      k_rdm_assemble_s<<<gs, 256, 0, stream>>>(norb, G, ld, nullptr, dm2ab);
+      k_rdm_assemble_s<<<gs, 256, 0, stream>>>(norb, G, ld, nullptr, 1.0, dm2ab);
       return check_launch("rdm2ab assemble");
     }
   }
@@ -847,11 +852,11 @@ int csffci_rdm12s(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
   if (two) {
     const int g = grid_for((long long)n2 * n2, 256, 148 * 8);
     // same-spin: <p+ r+ s q> = <E_pq E_rs> - d_qr <p+ s> = ... - d_qr dm1[s][p]
-    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gaa, n2, d1at, dm2aa);
+    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gaa, n2, d1at, neleca < 2 ? 0.0 : 1.0, dm2aa);
     if ((st = check_launch("rdm2aa assemble"))) return st;
-    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gab, n2, nullptr, dm2ab);
+    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gab, n2, nullptr, 1.0, dm2ab);
     if ((st = check_launch("rdm2ab assemble"))) return st;
-    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gbb, n2, d1bt, dm2bb);
+    k_rdm_assemble_s<<<g, 256, 0, stream>>>(norb, Gbb, n2, d1bt, nelecb < 2 ? 0.0 : 1.0, dm2bb);
     return check_launch("rdm2bb assemble");
   }
   return CSFFCI_OK;

@@ -575,8 +575,11 @@ __device__ __forceinline__ double rf_d1(const double* M, int ld, int n, double h
   return v * half_inv_n * (p == q ? 2.0 : 1.0);
 }
 
-__global__ void k_rdm_assemble_sa(int n, const double* __restrict__ M, int ld, int rows_s, double half_inv_n,
-                                  double* dm1, double* dm2) {
+// one: a block of one spin, whose x+ r+ s y vanishes for x = r and for y = s.
+// pairs: 0 below two electrons of that kind, else 1.  Such terms cancel but for
+// rounding and are set to zero (NaN stays).
+__global__ void k_rdm_assemble_sa(int n, const double* __restrict__ M, int ld, int rows_s, double half_inv_n, bool one,
+                                  double pairs, double* dm1, double* dm2) {
   const int n2 = n * n;
   const long long tot = (long long)n2 * n2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
@@ -591,7 +594,7 @@ __global__ void k_rdm_assemble_sa(int n, const double* __restrict__ M, int ld, i
     v *= 0.25;
     if (y == r) v -= 0.5 * rf_d1(M, ld, n, half_inv_n, x, s);
     if (x == s) v -= 0.5 * rf_d1(M, ld, n, half_inv_n, y, r);
-    dm2[t] = v;
+    dm2[t] = (one && (x == r || y == s) ? 0.0 : pairs) * v;
     if (t < n2) dm1[t] = rf_d1(M, ld, n, half_inv_n, (int)(t / n), (int)(t % n));
   }
 }
@@ -861,7 +864,8 @@ int rdm_assemble_sa(const RdmFusedJob& j, const double* M, int nelec, double* dm
                     cudaStream_t stream) {
   const long long n2 = (long long)j.norb * j.norb;
   k_rdm_assemble_sa<<<grid_for(n2 * n2, 128, 148 * 8), 128, 0, stream>>>(
-      j.norb, M, rdm_fused_ld(j), rdm_fused_rows_s(j), nelec > 0 ? 0.5 / nelec : 0.0, dm1, dm2);
+      j.norb, M, rdm_fused_ld(j), rdm_fused_rows_s(j), nelec > 0 ? 0.5 / nelec : 0.0, j.spin[0] != 3,
+      nelec < 2 ? 0.0 : 1.0, dm1, dm2);
   return check_launch("rdm assemble");
 }
 

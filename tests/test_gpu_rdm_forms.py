@@ -135,3 +135,21 @@ def test_form_taken(same, norb, na, nb, fused):
         finally:
             _capi.profile_enable(False)
         assert ("k_rdm_fused" in ran, "k_tslab_tile" in ran) == (fused, not fused)
+
+
+@pytest.mark.parametrize("norb,na,nb", [(2, 1, 0), (5, 0, 1), (6, 3, 1), (8, 1, 4), (7, 4, 3), (12, 1, 3), (16, 1, 1),
+                                        (17, 1, 1)])
+@pytest.mark.parametrize("same", [True, False])
+def test_what_vanishes_is_zero(norb, na, nb, same):
+    """The two-particle density of fewer than two electrons, and p+ r+ s q of one
+    spin with p = r or q = s, exactly."""
+    import torch
+    from pyscf_forge_b200.fci import direct_spin1 as D
+    gen = torch.Generator(device="cuda").manual_seed(norb)
+    c = [torch.randn(comb(norb, na) * comb(norb, nb), dtype=torch.float64, device="cuda", generator=gen) for _ in range(2)]
+    _, (aa, _, bb) = D.dev_rdm12s(c[0], None if same else c[1], norb, (na, nb))
+    for n, dm2 in ((na, aa), (nb, bb)):
+        assert bool(dm2.any()) == (n > 1)
+        assert not torch.einsum("pqps->pqs", dm2).any() and not torch.einsum("pqrq->pqr", dm2).any()
+    _, dm2 = D.dev_rdm12(c[0], None if same else c[1], norb, (na, nb))
+    assert bool(dm2.any()) == (na + nb > 1)
