@@ -688,7 +688,8 @@ int csffci_rdm12(int norb, int neleca, int nelecb, const csffci_link_t* link_a,
     if ((st = check_launch("rdm1 from the Gram"))) return st;
     k_transpose_small<<<grid_for(n2, 256), 256, 0, stream>>>(norb, d1t, dm1);
     if ((st = check_launch("rdm1 transpose"))) return st;
-    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, ld, dm1, ne < 2 ? 0.0 : 1.0, dm2);
+    k_rdm_assemble<<<grid_for((long long)n2 * n2, 256, 148 * 8), 256, 0, stream>>>(norb, G, ld, dm1,
+                                                                                   ne < 2 ? 0.0 : 1.0, dm2);
     return check_launch("rdm2 assemble");
   }
   long long S = ndet < (1ll << 18) ? ndet : (1ll << 18);
